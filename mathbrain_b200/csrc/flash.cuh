@@ -22,6 +22,7 @@ struct FlashArgs {
     int B, H, T, N, K, nT;
     float v_total;
     int silu, listed_only;
+    const int* level;       // [B, nT] or null: the every-step tensor-core kernels work on the tiles marked smooth::LEVEL_EXACT only
     int test_withhold;      // test hook: see MBEMA_FLAG_TEST_WITHHOLD_ARRIVE
 };
 
@@ -36,7 +37,6 @@ int flash_bwd_simt(FlashArgs a, float* dW, void* ws, cudaStream_t st);
 
 // tensor-core (tcgen05) path
 bool flash_tc_supported(int H, int N, int K);
-size_t flash_fwd_tc_ws();
 int flash_fwd_tc(const FlashArgs& a, void* ws, cudaStream_t st);
 bool flash_bwd_tc_supported(int H, int N, int K);
 size_t flash_bwd_tc_ws(int64_t B, int64_t H, int64_t T, int64_t N);

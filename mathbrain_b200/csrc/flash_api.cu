@@ -1,5 +1,6 @@
 // C entry points of the flash-EMA attention: argument checks and dispatch on the compute mode.
 #include "flash.cuh"
+#include "smooth.cuh"
 
 using namespace mbema;
 
@@ -38,8 +39,11 @@ extern "C" int mbema_flash_tc_supported(int64_t H, int64_t N, int64_t K) {
     return flash_tc_supported((int)H, (int)N, (int)K) ? 1 : 0;
 }
 
-extern "C" size_t mbema_flash_fwd_workspace_bytes(int64_t, int64_t, int64_t, int64_t, int64_t, int64_t, int) {
-    return 256;
+// the first STATUS_BYTES of a tensor-core workspace hold the kernels' status word
+static constexpr size_t STATUS_BYTES = 512;
+
+extern "C" size_t mbema_flash_fwd_workspace_bytes(int64_t B, int64_t H, int64_t T, int64_t, int64_t N, int64_t K, int mode) {
+    return mode == MBEMA_MODE_TC_BF16 ? STATUS_BYTES + smooth::ws_bytes(B, H, T, N, K) : 256;
 }
 
 static int flash_fwd_impl(const void* Q, int q_dtype, const int64_t* x, const void* E_k, const void* E_v,
@@ -64,8 +68,14 @@ static int flash_fwd_impl(const void* Q, int q_dtype, const int64_t* x, const vo
     if (e_row_index) { a.erow = e_row_index; a.e_rows = e_rows; }
     if (mode == MBEMA_MODE_TC_BF16) {
         if (!workspace) return MBEMA_ERR_NULL;
-        if (workspace_bytes < flash_fwd_tc_ws()) return MBEMA_ERR_WORKSPACE;
-        return flash_fwd_tc(a, workspace, (cudaStream_t)stream);
+        if (workspace_bytes < mbema_flash_fwd_workspace_bytes(B, H, T, hd, N, K, mode)) return MBEMA_ERR_WORKSPACE;
+        cudaStream_t st = (cudaStream_t)stream;
+        if (flags & MBEMA_FLAG_EVERY_STEP) return flash_fwd_tc(a, workspace, st);
+        int* status = reinterpret_cast<int*>((reinterpret_cast<uintptr_t>(workspace) + 15) & ~uintptr_t(15));
+        const smooth::Ws w = smooth::carve(static_cast<unsigned char*>(workspace) + STATUS_BYTES, B, H, T, N, K);
+        if ((rc = smooth::prepare(a, w, st)) || (rc = smooth::forward(a, w, status, st))) return rc;
+        a.level = w.level;
+        return flash_fwd_tc(a, workspace, st);
     }
     return flash_fwd_simt(a, (cudaStream_t)stream);
 }

@@ -27,6 +27,7 @@
 #include "flash.cuh"
 #include <cuda_fp16.h>
 #include "sm100_ptx.cuh"
+#include "smooth.cuh"
 
 namespace mbema {
 namespace tc {
@@ -122,6 +123,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_flash_fwd_tc(FlashArgs a, int* s
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int D = a.H * HD;
     const int t0 = tile * TM;
+    if (a.level && a.level[b * a.nT + tile] != smooth::LEVEL_EXACT) return;      // done by the smooth-state kernel
     const int Lb = a.seq_lens ? min(max(a.seq_lens[b], 0), a.T) : a.T;
     const bool is_epi = warp < EPI_WARPS;
     const int row = (warp & 3) * 32 + lane;         // time step within the tile (== TMEM lane for epilogue warps)
@@ -498,8 +500,6 @@ __global__ void __launch_bounds__(THREADS, 1) k_flash_fwd_tc(FlashArgs a, int* s
 bool flash_tc_supported(int H, int N, int K) {
     return (H % tc::HPC) == 0 && (N == 64 || N == 128) && K <= tc::MAX_SLOTS && tc::smem_layout(N, K).total <= 227 * 1024;
 }
-
-size_t flash_fwd_tc_ws() { return 256; }
 
 int flash_fwd_tc(const FlashArgs& a, void* ws, cudaStream_t st) {
     int* status = reinterpret_cast<int*>((reinterpret_cast<uintptr_t>(ws) + 15) & ~uintptr_t(15));

@@ -1,0 +1,88 @@
+// Attention over slot states that vary smoothly inside a time tile ("smooth path"): shared declarations.
+//
+// Between two occurrences of its token a slot's state only decays, M_n(t) = M_n(t0) rho_n^(t - t0), so with half-lives
+// of hundreds of steps the gate SiLU(M(t) W) of a slot is a smooth function of t over a tile of 128 steps.  It is
+// evaluated at the four Chebyshev nodes of the tile instead of at its 128 steps and expanded in the Chebyshev
+// polynomials T_0..T_3 of the step: gate[t,k,d] = sum_j T_j(t) c_j[k,d].  With Q'[t,(j,d)] = T_j(t) Q[t,d] the operator
+// becomes an ordinary attention with head width 4 * 64 over the virtual keys E_k c_j and values E_v c_j, all of it
+// tensor-core products; one gate evaluation serves 32 steps.  An occurrence inside the tile starts a new item with the
+// state (state + 1) rho^-(step), extended backwards to the tile start and valid for the steps after it.
+//
+// Error: the remainder of the cubic interpolant is f''''(x) d^4 / 192 with d the change of the pre-activation over half
+// a tile.  k_items measures d per tile (root mean square over the gate's columns of M . lambda . W * 64) and the decay
+// over half a tile, and picks the number of segments the tile is cut into (1, 2, 4 or 8, each with nodes of its own);
+// what eight segments do not resolve goes to the kernels that evaluate every step (level LEVEL_EXACT).  With
+// half-lives of 1024..4096, states to 600 and W_pe ~ N(0, 0.02^2) the outputs differ from the exact sum by 1e-6 and
+// dW_pe by 1e-4 (norm-wise), against about 1e-3 from the 16-bit operands.
+#pragma once
+#include "flash.cuh"
+
+namespace mbema {
+namespace smooth {
+
+static constexpr int TM = MBEMA_TILE_T;     // steps per tile
+static constexpr int HD = 64;
+static constexpr int NJ = 4;                // nodes = coefficients per item
+static constexpr int IBLK = 128;            // items per block
+static constexpr int NCH = 4;               // a head's 64 columns are walked in chunks of 16: 16 x NJ = one swizzle atom
+static constexpr int ATOM = TM * 128;       // bytes of a 128-row x 64-column 16-bit operand tile
+static constexpr int WPIECE = 64 * 128;     // W' rows (node, 16 columns) x 64 channels
+static constexpr int LEVELS = 4;            // level L cuts the tile into 2^L segments
+static constexpr int LEVEL_EXACT = LEVELS;
+static constexpr int SEG_IMAGES = (1 << LEVELS) - 1;   // W' images: segment s of level L at index 2^L - 1 + s
+// Half a segment's decay exponent and pre-activation change that a cubic still resolves: remainders below
+// 0.16^4 / 192 = 3.4e-6 (of the state sum) and, at 2.5, below 16-bit rounding of the gradients (measured dW_pe: 5e-4).
+static constexpr float MAX_DECAY = 0.16f, MAX_SWING = 2.5f;
+
+// Per-call workspace (after the status block), written by the prep kernels.
+struct Ws {
+    float* gram;            // [N, N] W_pe W_pe^T / D
+    unsigned char* w_img;   // [SEG_IMAGES][H][NCH][N / 64][WPIECE] node-scaled W_pe, fp16, swizzled operand pieces
+    unsigned char* a_img;   // [B * nT][IB][N / 64][ATOM] item states, fp16 of state / 64, swizzled operand tiles
+    int2* meta;             // [B * nT][IB * 128] {row of the E tables, first valid step | last << 8}
+    uint4* mask;            // [B * nT][IB][128] bit i of row t: item i of the block is valid at step t
+    int* n_items;           // [B * nT]
+    int* level;             // [B * nT]
+    int IB;                 // item blocks reserved per tile
+};
+
+inline size_t ws_bytes(int64_t B, int64_t H, int64_t T, int64_t N, int64_t K) {
+    const size_t tiles = (size_t)B * ((T + TM - 1) / TM), IB = (size_t)(K + TM + IBLK - 1) / IBLK, NK = (size_t)N / 64;
+    return align_up((size_t)N * N * 4, 1024) + SEG_IMAGES * (size_t)H * NCH * NK * WPIECE + tiles * IB * NK * ATOM +
+           align_up(tiles * IB * IBLK * sizeof(int2), 1024) + tiles * IB * IBLK * sizeof(uint4) + 2 * align_up(tiles * 4, 1024) + 1024;
+}
+
+inline Ws carve(void* p0, int64_t B, int64_t H, int64_t T, int64_t N, int64_t K) {
+    const size_t tiles = (size_t)B * ((T + TM - 1) / TM), IB = (size_t)(K + TM + IBLK - 1) / IBLK, NK = (size_t)N / 64;
+    unsigned char* p = reinterpret_cast<unsigned char*>(align_up(reinterpret_cast<size_t>(p0), 1024));
+    Ws w;
+    w.IB = (int)IB;
+    w.gram = reinterpret_cast<float*>(p); p += align_up((size_t)N * N * 4, 1024);
+    w.w_img = p; p += SEG_IMAGES * (size_t)H * NCH * NK * WPIECE;
+    w.a_img = p; p += tiles * IB * NK * ATOM;
+    w.meta = reinterpret_cast<int2*>(p); p += align_up(tiles * IB * IBLK * sizeof(int2), 1024);
+    w.mask = reinterpret_cast<uint4*>(p); p += tiles * IB * IBLK * sizeof(uint4);
+    w.n_items = reinterpret_cast<int*>(p); p += align_up(tiles * 4, 1024);
+    w.level = reinterpret_cast<int*>(p);
+    return w;
+}
+
+// Chebyshev basis of a step, scaled so that the coefficients need no factors: beta_j = s_j T_j(u) with
+// s = {1, 2 cos(pi/8), sqrt 2, -2 cos(pi/8)}, the E rows taken times 1/4 and the coefficients formed as
+//   c_0 = (g0 + g3) + (g1 + g2)   c_1 = (g0 - g3) + tan(pi/8) (g1 - g2)   c_2 = (g0 + g3) - (g1 + g2)   c_3 = (g1 - g2) - tan(pi/8) (g0 - g3)
+__device__ __forceinline__ void basis(int row, int level, float (&beta)[NJ]) {
+    const int len = TM >> level;
+    const float u = ((float)(row & (len - 1)) - 0.5f * (float)(len - 1)) * (2.0f / (float)len);
+    const float t2 = fmaf(2.0f * u, u, -1.0f);
+    beta[0] = 1.0f;
+    beta[1] = 1.8477590650f * u;
+    beta[2] = 1.4142135624f * t2;
+    beta[3] = -1.8477590650f * u * fmaf(2.0f, t2, -1.0f);     // T_3 = u (4 u^2 - 3) = u (2 T_2 - 1)
+}
+static constexpr float TAN_PI_8 = 0.41421356237f;
+
+int prepare(const FlashArgs& a, const Ws& w, cudaStream_t st);
+int forward(const FlashArgs& a, const Ws& w, int* status, cudaStream_t st);
+
+}  // namespace smooth
+}  // namespace mbema

@@ -1,0 +1,448 @@
+// Flash-EMA attention forward over smooth slot states (see smooth.cuh): one CTA per (tile, head, sample).
+//
+// Items are walked in blocks of 128, a head's 64 columns in chunks of 16 (16 columns x 4 coefficients = one 64-wide
+// swizzle atom).  Per block, on the tensor cores:
+//     pre_c [128 items x 64]  = A . W'_c            A: item states, W'_c: W_pe scaled to the four nodes
+//     S     [128 steps x 128] += Q'_c . K_c^T       K_c = E_k c_j, written by the gate warps
+//     O'_c  [128 steps x 64]  += P . V_c            P from tensor memory, V_c = E_v c_j
+// Warps: two gate warpgroups (a thread per item; the even and the odd chunks), two softmax warpgroups (a thread per
+// step and half a block's items), one loader (bulk copies of A and W' images), one lane issuing the gate products and
+// one issuing S and P.V, so that neither waits for the other's operands.  All hand-offs are mbarriers with bounded waits.
+//
+// Bound: special functions and issue slots, not the tensor cores.  A block takes 4 * 64 tanh per item and one exponential
+// per item and step (3072 cycles of the special-function pipe at 16 a clock), 2560 cycles of tensor work.
+#include "smooth.cuh"
+#include "sm100_ptx.cuh"
+
+namespace mbema {
+namespace smooth {
+
+using namespace ptx;
+
+namespace fwd {
+
+static constexpr int GATE_WARPS = 8, SM_WARPS = 8;
+static constexpr int W_LOAD = 16, W_GATE = 17, W_ATT = 18;       // warp 19 only fills the warpgroup
+static constexpr int THREADS = 20 * 32;      // launched with 96 registers a thread: 61440 >= 4 * 128 * 104 + 128 * 56
+static constexpr uint32_t T_O = 0, T_S = 256, T_PRE = 384;     // tensor-memory columns
+static constexpr float RESCALE = 8.0f;      // log2 units the softmax reference may lag behind (P <= 2^8 in fp16)
+
+struct Bars {
+    uint64_t a_full[2], a_free[2], w_full[2], w_free[2], pre_full[2], pre_empty[2], kv_full[NCH], k_free[2], v_free[NCH];
+    uint64_t s_full, p_full, mx_full, o_full, drain;
+    uint32_t tmem_base;
+    int abort_flag, drain_flag;
+    unsigned spin_limit;
+};
+
+static constexpr int Q_OFF = 0, A_OFF = Q_OFF + NCH * ATOM, W_OFF = A_OFF + 2 * ATOM, K_OFF = W_OFF + 2 * WPIECE, V_OFF = K_OFF + 2 * ATOM,
+                     MX_OFF = V_OFF + NCH * ATOM, BAR_OFF = MX_OFF + 4 * TM * 4, SMEM = BAR_OFF + 512 + 1024;
+static_assert(sizeof(Bars) <= 512 && SMEM <= 227 * 1024, "shared memory");
+
+// 16 columns of an E row, raw
+template <bool EF32> struct ERow { uint4 v[EF32 ? 4 : 2]; };
+template <bool EF32>
+__device__ __forceinline__ ERow<EF32> load_e(const void* E, size_t off) {
+    ERow<EF32> r;
+    const uint4* p = reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned char*>(E) + off * (EF32 ? 4 : 2));
+#pragma unroll
+    for (int i = 0; i < (EF32 ? 4 : 2); ++i) r.v[i] = __ldg(p + i);
+    return r;
+}
+// columns 2p, 2p + 1 as fp16, times 1/4
+template <bool EF32>
+__device__ __forceinline__ uint32_t e_pair(const ERow<EF32>& r, int p) {
+    const uint32_t* u = reinterpret_cast<const uint32_t*>(r.v);
+    if (EF32) return pack_f16x2_sat(__uint_as_float(u[2 * p]) * 0.25f, __uint_as_float(u[2 * p + 1]) * 0.25f);
+    return pack_f16x2_sat(bf16_lo(u[p]) * 0.25f, bf16_hi(u[p]) * 0.25f);
+}
+
+// a wait whose outcome is the same for the whole warp (the code after it has warp-wide instructions)
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int tag, const unsigned* lim) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, tag, lim));
+}
+
+template <bool SILU, int NK, bool EF32>
+__global__ void __launch_bounds__(THREADS, 1) k_smooth_fwd(FlashArgs a, Ws w, int* status) {
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* sm = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+    Bars* bars = reinterpret_cast<Bars*>(sm + BAR_OFF);
+    float* mx_sh = reinterpret_cast<float*>(sm + MX_OFF);
+    volatile int* abort_flag = &bars->abort_flag;
+    constexpr int NA = NK == 1 ? 2 : 1;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tile = blockIdx.x, h = blockIdx.y, b = a.order ? a.order[blockIdx.z] : (int)blockIdx.z;
+    const int bt = b * a.nT + tile, t0 = tile * TM, D = a.H * HD;
+    const int Lb = a.seq_lens ? min(max(a.seq_lens[b], 0), a.T) : a.T;
+    const int level = w.level[bt];
+    if (level == LEVEL_EXACT) return;
+    const size_t row0 = ((size_t)b * a.H + h) * a.T + t0;
+    if (t0 >= Lb) {          // a tile beyond the valid length
+        for (int i = tid; i < min(TM, a.T - t0) * (HD / 4); i += THREADS)
+            *reinterpret_cast<float4*>(a.O + (row0 + i / (HD / 4)) * HD + (i % (HD / 4)) * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (tid < min(TM, a.T - t0)) a.LSE[row0 + tid] = 0.f;
+        return;
+    }
+    if (tid == 0) {
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&bars->a_full[i], 1); mbar_init(&bars->a_free[i], 1);
+            mbar_init(&bars->w_full[i], 1); mbar_init(&bars->w_free[i], 1);
+            mbar_init(&bars->pre_full[i], 1); mbar_init(&bars->pre_empty[i], 4);
+            mbar_init(&bars->k_free[i], 1);
+        }
+        for (int i = 0; i < NCH; ++i) { mbar_init(&bars->kv_full[i], 4); mbar_init(&bars->v_free[i], 1); }
+        mbar_init(&bars->s_full, 1); mbar_init(&bars->p_full, SM_WARPS); mbar_init(&bars->mx_full, SM_WARPS);
+        mbar_init(&bars->o_full, 1); mbar_init(&bars->drain, 2);
+        bars->abort_flag = *reinterpret_cast<volatile int*>(status);      // an earlier CTA gave up: do nothing
+        bars->drain_flag = 0;
+        bars->spin_limit = a.test_withhold ? 64u : MBEMA_SPIN_LIMIT;
+        fence_barrier_init();
+    }
+    if (warp == W_GATE) {
+        tmem_alloc(&bars->tmem_base, 512);
+        tmem_relinquish();
+    }
+    // Q' tiles: row t, chunk c holds q[16 c + dd] beta_j(t) log2(e) / 8 at column 16 j + dd
+    if (tid < TM * NCH) {
+        const int t = tid & (TM - 1), c = tid >> 7;
+        float beta[NJ], q[16];
+        basis(t, level, beta);
+#pragma unroll
+        for (int i = 0; i < 16; i += 4) {
+            const float4 v = t0 + t < Lb ? ld4_dyn_f32(a.Q, a.q_dt, (row0 + t) * HD + c * 16 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+            q[i] = v.x; q[i + 1] = v.y; q[i + 2] = v.z; q[i + 3] = v.w;
+        }
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) {
+            const float s = beta[j] * (0.125f * 1.4426950409f);
+#pragma unroll
+            for (int g = 0; g < 2; ++g)
+                *reinterpret_cast<uint4*>(sm + Q_OFF + c * ATOM + t * 128 + (((2 * j + g) ^ (t & 7)) << 4)) =
+                    make_uint4(pack_f16x2_sat(q[8 * g] * s, q[8 * g + 1] * s), pack_f16x2_sat(q[8 * g + 2] * s, q[8 * g + 3] * s),
+                               pack_f16x2_sat(q[8 * g + 4] * s, q[8 * g + 5] * s), pack_f16x2_sat(q[8 * g + 6] * s, q[8 * g + 7] * s));
+        }
+    }
+    fence_proxy_async_smem();
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    const uint32_t tmem = bars->tmem_base;
+    const int n_blk = (w.n_items[bt] + IBLK - 1) / IBLK;
+    const int n_it = bars->abort_flag ? 0 : n_blk << level;        // blocks of segment 0, then of segment 1, ...
+    const unsigned* lim = &bars->spin_limit;
+
+    if (warp < GATE_WARPS) {
+        // ======================================================== gate: item r, chunks wg and wg + 2
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
+        const int wg = warp >> 2, r = tid & 127;
+        const uint32_t t_pre = tmem + ((uint32_t)((warp & 3) * 32) << 16) + T_PRE + wg * 64;
+        const int2* meta = w.meta + (size_t)bt * w.IB * IBLK + r;
+        const int x7 = r & 7;
+        int er = n_it > 0 ? __ldg(&meta[0].x) : 0;
+        ERow<EF32> ek, ev;
+        if (n_it > 0) {
+            ek = load_e<EF32>(a.Ek, (size_t)er * D + h * HD + wg * 16);
+            ev = load_e<EF32>(a.Ev, (size_t)er * D + h * HD + wg * 16);
+        }
+        bool alive = true;
+        for (int i = 0; i < n_it && alive; ++i) {
+#pragma unroll 1
+            for (int cc = 0; cc < 2; ++cc) {
+                const int c = wg + 2 * cc;
+                // the next chunk's E columns fly while this chunk is worked on
+                ERow<EF32> nk = ek, nv = ev;
+                if (cc == 1 && i + 1 < n_it) er = __ldg(&meta[(size_t)((i + 1) % n_blk) * IBLK].x);
+                if (cc == 0 || i + 1 < n_it) {
+                    const size_t off = (size_t)er * D + h * HD + (wg + 2 * (cc ^ 1)) * 16;
+                    nk = load_e<EF32>(a.Ek, off);
+                    nv = load_e<EF32>(a.Ev, off);
+                }
+                const int use = 2 * i + cc;
+                if (!(alive = warp_wait(&bars->pre_full[wg], (uint32_t)(use & 1), abort_flag, 1, lim))) break;
+                tc_fence_after_sync();
+                float x[2][NJ][8];
+#pragma unroll
+                for (int j = 0; j < NJ; ++j) tmem_ld_32x32b_x8(t_pre + j * 16, x[0][j]);
+                tmem_wait_ld();
+#pragma unroll
+                for (int j = 0; j < NJ; ++j) tmem_ld_32x32b_x8(t_pre + j * 16 + 8, x[1][j]);
+                unsigned char* kd = sm + K_OFF + wg * ATOM + r * 128;
+                unsigned char* vd = sm + V_OFF + c * ATOM + r * 128;
+#pragma unroll
+                for (int g = 0; g < 2; ++g) {
+                    uint32_t cf[NJ][4];
+#pragma unroll
+                    for (int p = 0; p < 4; ++p) {
+                        f32x2 gt[NJ];
+#pragma unroll
+                        for (int j = 0; j < NJ; ++j) {
+                            const float h0 = x[g][j][2 * p], h1 = x[g][j][2 * p + 1];
+                            const f32x2 hh = pack2(h0, h1);
+                            gt[j] = SILU ? fma2(hh, pack2(tanh_approx(h0), tanh_approx(h1)), hh) : hh;
+                        }
+                        const f32x2 m1 = pack2(-1.f, -1.f), ka = pack2(TAN_PI_8, TAN_PI_8), kn = pack2(-TAN_PI_8, -TAN_PI_8);
+                        const f32x2 s03 = add2(gt[0], gt[3]), s12 = add2(gt[1], gt[2]);
+                        const f32x2 d03 = fma2(gt[3], m1, gt[0]), d12 = fma2(gt[2], m1, gt[1]);
+                        const f32x2 cj[NJ] = {add2(s03, s12), fma2(d12, ka, d03), fma2(s12, m1, s03), fma2(d03, kn, d12)};
+#pragma unroll
+                        for (int j = 0; j < NJ; ++j) {
+                            float lo, hi;
+                            unpack2(cj[j], lo, hi);
+                            cf[j][p] = pack_f16x2_sat(lo, hi);
+                        }
+                    }
+                    if (g == 0) {
+                        tmem_wait_ld();            // the second half's columns are in registers
+                        tc_fence_before_sync();
+                        __syncwarp();
+                        if (lane == 0 && !(a.test_withhold && use == 0)) mbar_arrive(&bars->pre_empty[wg]);
+                        if (use >= 1 && !(alive = warp_wait(&bars->k_free[wg], (uint32_t)((use - 1) & 1), abort_flag, 2, lim))) break;
+                        if (i >= 1 && !(alive = warp_wait(&bars->v_free[c], (uint32_t)((i - 1) & 1), abort_flag, 3, lim))) break;
+                    }
+                    uint32_t e2[4], f2[4];
+#pragma unroll
+                    for (int p = 0; p < 4; ++p) { e2[p] = e_pair<EF32>(ek, 4 * g + p); f2[p] = e_pair<EF32>(ev, 4 * g + p); }
+#pragma unroll
+                    for (int j = 0; j < NJ; ++j) {
+                        const int off = ((2 * j + g) ^ x7) << 4;
+                        st_shared_v4(kd + off, mul_f16x2(cf[j][0], e2[0]), mul_f16x2(cf[j][1], e2[1]), mul_f16x2(cf[j][2], e2[2]), mul_f16x2(cf[j][3], e2[3]));
+                        st_shared_v4(vd + off, mul_f16x2(cf[j][0], f2[0]), mul_f16x2(cf[j][1], f2[1]), mul_f16x2(cf[j][2], f2[2]), mul_f16x2(cf[j][3], f2[3]));
+                    }
+                }
+                if (!alive) break;
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bars->kv_full[c]);
+                ek = nk;
+                ev = nv;
+            }
+        }
+    } else if (warp < GATE_WARPS + SM_WARPS) {
+        // ======================================================== softmax: step `row`, items 64 half .. 64 half + 63
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
+        const int half = (warp >> 2) & 1, row = tid & 127;
+        const uint32_t t_row = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+        const float rest = a.v_total - (float)a.kcount[b];
+        float m, l = 0.f;
+        if (!a.listed_only && rest > 0.f) { m = 0.f; l = half == 0 ? rest : 0.f; } else m = -INFINITY;
+        const uint2* mask = reinterpret_cast<const uint2*>(w.mask + (size_t)bt * w.IB * IBLK + row) + half;
+        const int my_seg = row / (TM >> level);
+        uint2 mk = n_it > 0 ? __ldg(mask) : make_uint2(0u, 0u);
+        bool alive = true;
+        for (int i = 0; i < n_it; ++i) {
+            uint2 mcur = mk;
+            if (i / n_blk != my_seg) mcur = make_uint2(0u, 0u);
+            if (i + 1 < n_it) mk = __ldg(mask + (size_t)((i + 1) % n_blk) * IBLK * 2);
+            if (!(alive = warp_wait(&bars->s_full, (uint32_t)(i & 1), abort_flag, 4, lim))) break;
+            tc_fence_after_sync();
+            float s[64];
+            tmem_ld_32x32b_x32(t_row + T_S + half * 64, s);
+            tmem_ld_32x32b_x32(t_row + T_S + half * 64 + 32, s + 32);
+            tmem_wait_ld();
+            if (!__all_sync(0xffffffffu, (mcur.x & mcur.y) == 0xffffffffu)) {
+#pragma unroll
+                for (int k = 0; k < 32; ++k) {
+                    s[k] = (mcur.x >> k) & 1u ? s[k] : -INFINITY;
+                    s[k + 32] = (mcur.y >> k) & 1u ? s[k + 32] : -INFINITY;
+                }
+            }
+            float b0 = -INFINITY, b1 = -INFINITY;
+#pragma unroll
+            for (int k = 0; k < 64; k += 4) {
+                b0 = fmaxf(b0, fmaxf(s[k], s[k + 1]));
+                b1 = fmaxf(b1, fmaxf(s[k + 2], s[k + 3]));
+            }
+            float* mx = mx_sh + (i & 1) * 2 * TM;
+            mx[half * TM + row] = fmaxf(b0, b1);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars->mx_full);
+            if (!(alive = warp_wait(&bars->mx_full, (uint32_t)(i & 1), abort_flag, 5, lim))) break;
+            const float mb = fmaxf(fmaxf(b0, b1), mx[(half ^ 1) * TM + row]);
+            const bool up = mb > m + RESCALE;
+            if (__any_sync(0xffffffffu, up)) {
+                const float al = up ? ex2_approx(m - mb) : 1.0f;       // m = -inf: 0
+                l *= al;
+                if (up) m = mb;
+                if (i > 0) {       // this half's columns of O' (the products of the earlier blocks completed before S did)
+#pragma unroll 1
+                    for (int k = 0; k < 128; k += 16) {
+                        float o[16];
+                        tmem_ld_32x32b_x16(t_row + T_O + half * 128 + k, o);
+                        tmem_wait_ld();
+#pragma unroll
+                        for (int e = 0; e < 16; ++e) o[e] *= al;
+                        tmem_st_32x32b_x16(t_row + T_O + half * 128 + k, o);
+                    }
+                }
+            }
+            const float mm = m == -INFINITY ? 0.f : m;
+            float l0 = 0.f, l1 = 0.f;
+            // P as fp16 pairs over the half's own score columns (all of them are in registers by now)
+#pragma unroll
+            for (int k = 0; k < 64; k += 32) {
+                uint32_t p2[16];
+#pragma unroll
+                for (int e = 0; e < 16; ++e) {
+                    const float p = ex2_approx(s[k + 2 * e] - mm), q = ex2_approx(s[k + 2 * e + 1] - mm);
+                    l0 += p; l1 += q;
+                    p2[e] = pack_f16x2(p, q);
+                }
+                tmem_st_x16(t_row + T_S + half * 64 + k / 2, p2);
+            }
+            l += l0 + l1;
+            tmem_wait_st();
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars->p_full);
+        }
+        if (alive && n_it > 0) alive = warp_wait(&bars->o_full, 0u, abort_flag, 6, lim);
+        if (alive && __all_sync(0xffffffffu, !*abort_flag)) {
+            tc_fence_after_sync();
+            float* mx = mx_sh + (n_it & 1) * 2 * TM;
+            mx[half * TM + row] = l;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars->mx_full);
+            alive = warp_wait(&bars->mx_full, (uint32_t)(n_it & 1), abort_flag, 7, lim);
+            l += mx[(half ^ 1) * TM + row];
+            const bool ok = t0 + row < Lb && l > 0.f;
+            const float inv = ok ? 1.0f / l : 0.f;
+            float beta[NJ];
+            basis(row, level, beta);
+#pragma unroll 1
+            for (int c = half * 2; c < half * 2 + 2; ++c) {
+                float o[64];
+                if (n_it > 0) {
+                    tmem_ld_32x32b_x32(t_row + T_O + c * 64, o);
+                    tmem_ld_32x32b_x32(t_row + T_O + c * 64 + 32, o + 32);
+                    tmem_wait_ld();
+                } else {
+#pragma unroll
+                    for (int e = 0; e < 64; ++e) o[e] = 0.f;
+                }
+                if (alive && t0 + row < a.T) {
+#pragma unroll
+                    for (int d = 0; d < 16; d += 4) {
+                        float v[4];
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const int k = d + e;
+                            v[e] = ok ? inv * fmaf(beta[3], o[48 + k], fmaf(beta[2], o[32 + k], fmaf(beta[1], o[16 + k], o[k]))) : 0.f;
+                        }
+                        *reinterpret_cast<float4*>(a.O + (row0 + row) * HD + c * 16 + d) = make_float4(v[0], v[1], v[2], v[3]);
+                    }
+                }
+            }
+            if (alive && half == 0 && t0 + row < a.T) a.LSE[row0 + row] = ok ? m * 0.6931471806f + logf(l) : 0.f;
+        }
+    } else {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+        if (warp == W_LOAD && lane == 0) {
+            // ==================================================== loader
+            const unsigned char* img = w.a_img + (size_t)bt * w.IB * NK * ATOM;
+            int np = 0;
+            bool alive = true;
+            for (int i = 0; i < n_it && alive; ++i) {
+                const int seg = i / n_blk, blk = i - seg * n_blk;
+                const unsigned char* wi = w.w_img + (size_t)((((1 << level) - 1 + seg) * a.H + h) * NCH) * NK * WPIECE;
+                const int sa = i % NA, ua = i / NA;
+                if (ua >= 1 && !(alive = mbar_wait(&bars->a_free[sa], (uint32_t)((ua - 1) & 1), abort_flag, 8, lim))) break;
+                mbar_expect_tx(&bars->a_full[sa], NK * ATOM);
+                bulk_load(sm + A_OFF + sa * ATOM, img + (size_t)blk * NK * ATOM, NK * ATOM, &bars->a_full[sa]);
+                for (int p = 0; p < NCH * NK; ++p, ++np) {
+                    const int sw = np & 1, uw = np >> 1;
+                    if (uw >= 1 && !(alive = mbar_wait(&bars->w_free[sw], (uint32_t)((uw - 1) & 1), abort_flag, 9, lim))) break;
+                    mbar_expect_tx(&bars->w_full[sw], WPIECE);
+                    bulk_load(sm + W_OFF + sw * WPIECE, wi + (size_t)p * WPIECE, WPIECE, &bars->w_full[sw]);
+                }
+                if (!alive) mbar_wait<100>(&bars->a_full[sa], (uint32_t)(ua & 1), &bars->drain_flag, 10);
+            }
+            // no copy of this CTA is in flight when it ends (the last A tile landed before its products could be issued)
+            for (int s = 0; s < 2; ++s)
+                if (np > s) mbar_wait<100>(&bars->w_full[s], (uint32_t)(((np - 1 - s) >> 1) & 1), &bars->drain_flag, 10);
+            for (int i = max(0, n_it - NA); i < n_it && alive; ++i)
+                mbar_wait<100>(&bars->a_full[i % NA], (uint32_t)((i / NA) & 1), &bars->drain_flag, 10);
+        } else if (warp == W_GATE && lane == 0) {
+            // ==================================================== gate products
+            const uint32_t idesc = umma_idesc_16(IBLK, 64, 0, 0, 0, 0);
+            int np = 0;
+            bool alive = true;
+            for (int i = 0; i < n_it && alive; ++i) {
+                const int sa = i % NA;
+                if (!(alive = mbar_wait(&bars->a_full[sa], (uint32_t)((i / NA) & 1), abort_flag, 11, lim))) break;
+                for (int c = 0; c < NCH && alive; ++c) {
+                    const int use = 2 * i + (c >> 1);
+                    if (use >= 1 && !(alive = mbar_wait(&bars->pre_empty[c & 1], (uint32_t)((use - 1) & 1), abort_flag, 12, lim))) break;
+                    for (int p = 0; p < NK; ++p, ++np) {
+                        if (!(alive = mbar_wait(&bars->w_full[np & 1], (uint32_t)((np >> 1) & 1), abort_flag, 13, lim))) break;
+                        tc_fence_after_sync();
+                        const uint32_t ab = smem_u32(sm + A_OFF + (sa + p) * ATOM), wb = smem_u32(sm + W_OFF + (np & 1) * WPIECE);
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+                            umma_bf16_ss(tmem + T_PRE + (c & 1) * 64, umma_desc_k_sw128(ab + k * 32), umma_desc_k_sw128(wb + k * 32), idesc, (p | k) != 0);
+                        umma_commit(&bars->w_free[np & 1]);
+                    }
+                    if (alive) umma_commit(&bars->pre_full[c & 1]);
+                }
+                if (alive) umma_commit(&bars->a_free[sa]);
+            }
+            umma_commit(&bars->drain);
+        } else if (warp == W_ATT && lane == 0) {
+            // ==================================================== S and P.V
+            const uint32_t id_s = umma_idesc_16(TM, IBLK, 0, 0, 0, 0), id_o = umma_idesc_16(TM, 64, 0, 1, 0, 0);
+            const uint32_t qb = smem_u32(sm + Q_OFF), kb = smem_u32(sm + K_OFF), vb = smem_u32(sm + V_OFF);
+            bool alive = true;
+            for (int i = 0; i < n_it && alive; ++i) {
+                for (int c = 0; c < NCH; ++c) {
+                    if (!(alive = mbar_wait(&bars->kv_full[c], (uint32_t)(i & 1), abort_flag, 14, lim))) break;
+                    tc_fence_after_sync();
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        umma_bf16_ss(tmem + T_S, umma_desc_k_sw128(qb + c * ATOM + k * 32), umma_desc_k_sw128(kb + (c & 1) * ATOM + k * 32), id_s, (c | k) != 0);
+                    umma_commit(&bars->k_free[c & 1]);
+                }
+                if (!alive) break;
+                umma_commit(&bars->s_full);
+                if (!(alive = mbar_wait(&bars->p_full, (uint32_t)(i & 1), abort_flag, 15, lim))) break;
+                tc_fence_after_sync();
+                for (int c = 0; c < NCH; ++c) {
+#pragma unroll
+                    for (int k = 0; k < 8; ++k)
+                        umma_16_ts(tmem + T_O + c * 64, tmem + T_S + (k < 4 ? k * 8 : 64 + (k - 4) * 8),
+                                   umma_desc_mn_sw128(vb + c * ATOM + k * 2048, ATOM, 1024), id_o, (i | k) != 0);
+                    umma_commit(&bars->v_free[c]);
+                }
+            }
+            umma_commit(&bars->o_full);
+            umma_commit(&bars->drain);
+        }
+    }
+    // ---------------------------------------------------------------- teardown
+    tc_fence_before_sync();
+    __syncthreads();
+    if (warp == W_GATE) {
+        mbar_wait<100>(&bars->drain, 0u, &bars->drain_flag, 16);
+        tc_fence_after_sync();
+        tmem_dealloc(tmem, 512);
+    }
+    if (tid == 0 && (bars->abort_flag | bars->drain_flag)) atomicOr(status, bars->abort_flag | bars->drain_flag);
+}
+
+}  // namespace fwd
+
+int forward(const FlashArgs& a, const Ws& w, int* status, cudaStream_t st) {
+    const dim3 grid(a.nT, a.H, a.B);
+#define MBEMA_SMOOTH(S_, NK_, E_)                                                                                             \
+    do {                                                                                                                       \
+        MBEMA_CUDA_TRY(cudaFuncSetAttribute(fwd::k_smooth_fwd<S_, NK_, E_>, cudaFuncAttributeMaxDynamicSharedMemorySize, fwd::SMEM)); \
+        fwd::k_smooth_fwd<S_, NK_, E_><<<grid, fwd::THREADS, fwd::SMEM, st>>>(a, w, status);                                    \
+    } while (0)
+#define MBEMA_SMOOTH_E(S_, NK_) do { if (a.e_dt == MBEMA_F32) MBEMA_SMOOTH(S_, NK_, true); else MBEMA_SMOOTH(S_, NK_, false); } while (0)
+    if (a.N == 64) { if (a.silu) MBEMA_SMOOTH_E(true, 1); else MBEMA_SMOOTH_E(false, 1); }
+    else { if (a.silu) MBEMA_SMOOTH_E(true, 2); else MBEMA_SMOOTH_E(false, 2); }
+#undef MBEMA_SMOOTH_E
+#undef MBEMA_SMOOTH
+    return check_launch();
+}
+
+}  // namespace smooth
+}  // namespace mbema
