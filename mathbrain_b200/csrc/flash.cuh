@@ -4,6 +4,8 @@
 
 namespace mbema {
 
+namespace smooth { struct Ws; }
+
 struct FlashArgs {
     const void* Q; int q_dt;
     const long long* x;
@@ -40,6 +42,7 @@ bool flash_tc_supported(int H, int N, int K);
 int flash_fwd_tc(const FlashArgs& a, void* ws, cudaStream_t st);
 bool flash_bwd_tc_supported(int H, int N, int K);
 size_t flash_bwd_tc_ws(int64_t B, int64_t H, int64_t T, int64_t N);
-int flash_bwd_tc(FlashArgs a, float* dW, void* ws, cudaStream_t st);
+// smooth_ws: workspace of the smooth-state kernels, which then take the tiles they can (null: every step everywhere)
+int flash_bwd_tc(FlashArgs a, const smooth::Ws* smooth_ws, float* dW, void* ws, cudaStream_t st);
 
 }  // namespace mbema

@@ -43,7 +43,7 @@ extern "C" int mbema_flash_tc_supported(int64_t H, int64_t N, int64_t K) {
 static constexpr size_t STATUS_BYTES = 512;
 
 extern "C" size_t mbema_flash_fwd_workspace_bytes(int64_t B, int64_t H, int64_t T, int64_t, int64_t N, int64_t K, int mode) {
-    return mode == MBEMA_MODE_TC_BF16 ? STATUS_BYTES + smooth::ws_bytes(B, H, T, N, K) : 256;
+    return mode == MBEMA_MODE_TC_BF16 ? STATUS_BYTES + smooth::ws_bytes(B, H, T, N, K, false) : 256;
 }
 
 static int flash_fwd_impl(const void* Q, int q_dtype, const int64_t* x, const void* E_k, const void* E_v,
@@ -109,7 +109,7 @@ extern "C" size_t mbema_flash_bwd_workspace_bytes(int64_t B, int64_t H, int64_t 
     // in tensor-core mode the first 512 bytes hold the kernel status word, whichever kernel ends up running
     size_t need = flash_bwd_simt_ws(B, H, T, N) + (mode == MBEMA_MODE_TC_BF16 ? 512 : 0);
     if (mode == MBEMA_MODE_TC_BF16 && flash_bwd_tc_supported((int)H, (int)N, (int)K)) {
-        const size_t tc = flash_bwd_tc_ws(B, H, T, N);
+        const size_t tc = align_up(flash_bwd_tc_ws(B, H, T, N), 1024) + smooth::ws_bytes(B, H, T, N, K, true);
         if (tc > need) need = tc;
     }
     return need;
@@ -146,8 +146,10 @@ static int flash_bwd_impl(const void* Q, int q_dtype, const int64_t* x, const vo
     if (e_row_index) { a.erow = e_row_index; a.e_rows = e_rows; }
     // tensor-core backward where the shape fits its shared-memory budget (N == 64); otherwise the fp32 kernels
     if (mode == MBEMA_MODE_TC_BF16) {
-        if (!(flags & MBEMA_FLAG_FP32_BACKWARD) && flash_bwd_tc_supported((int)H, (int)N, (int)K))
-            return flash_bwd_tc(a, dW_pe, workspace, st);
+        if (!(flags & MBEMA_FLAG_FP32_BACKWARD) && flash_bwd_tc_supported((int)H, (int)N, (int)K)) {
+            const smooth::Ws w = smooth::carve(static_cast<unsigned char*>(workspace) + flash_bwd_tc_ws(B, H, T, N), B, H, T, N, K);
+            return flash_bwd_tc(a, (flags & MBEMA_FLAG_EVERY_STEP) ? nullptr : &w, dW_pe, workspace, st);
+        }
         // (the first 512 bytes stay reserved for the status word of the tensor-core kernels; the fp32 kernels have no
         // bounded waits and leave it alone)
         return flash_bwd_simt(a, dW_pe, static_cast<unsigned char*>(workspace) + 512, st);

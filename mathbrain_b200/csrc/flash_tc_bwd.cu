@@ -16,6 +16,7 @@
 #include "flash.cuh"
 #include <cuda_fp16.h>
 #include "sm100_ptx.cuh"
+#include "smooth.cuh"
 
 namespace mbema {
 namespace tcb {
@@ -136,6 +137,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_flash_bwd_tc(FlashArgs a, int* s
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int D = a.H * HD;
     const int t0 = tile * TM;
+    if (a.level && a.level[b * a.nT + tile] != smooth::LEVEL_EXACT) return;      // done by the smooth-state kernel
     const int Lb = a.seq_lens ? min(max(a.seq_lens[b], 0), a.T) : a.T;
     const bool is_epi = warp < EPI_WARPS;
     const int row = (warp & 3) * 32 + lane;
@@ -729,12 +731,17 @@ size_t flash_bwd_tc_ws(int64_t B, int64_t H, int64_t T, int64_t N) {
     return 256 + (size_t)(B * (H / tcb::HPC) * nT) * N * tcb::ACC_COLS * sizeof(float) + 256;
 }
 
-int flash_bwd_tc(FlashArgs a, float* dW, void* ws, cudaStream_t st) {
+int flash_bwd_tc(FlashArgs a, const smooth::Ws* smooth_ws, float* dW, void* ws, cudaStream_t st) {
     const int D = a.H * tcb::HD;
     int* status = reinterpret_cast<int*>((reinterpret_cast<uintptr_t>(ws) + 255) & ~uintptr_t(255));
     a.dW_part = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(status) + 256);
     MBEMA_CUDA_TRY(cudaMemsetAsync(a.dEk, 0, (size_t)a.e_rows * D * sizeof(float), st));
     MBEMA_CUDA_TRY(cudaMemsetAsync(a.dEv, 0, (size_t)a.e_rows * D * sizeof(float), st));
+    if (smooth_ws) {
+        int rc;
+        if ((rc = smooth::prepare(a, *smooth_ws, st)) || (rc = smooth::backward(a, *smooth_ws, status, st))) return rc;
+        a.level = smooth_ws->level_bwd;
+    }
     const tcb::Smem L = tcb::smem_layout(a.K, a.N / 64);
     dim3 grid(a.nT, a.H / tcb::HPC, a.B);
 #define MBEMA_LAUNCH_BWD(S_, NK_, R_)                                                                                     \

@@ -32,7 +32,8 @@ static constexpr int LEVEL_EXACT = LEVELS;
 static constexpr int SEG_IMAGES = (1 << LEVELS) - 1;   // W' images: segment s of level L at index 2^L - 1 + s
 // Half a segment's decay exponent and pre-activation change that a cubic still resolves: remainders below
 // 0.16^4 / 192 = 3.4e-6 (of the state sum) and, at 2.5, below 16-bit rounding of the gradients (measured dW_pe: 5e-4).
-static constexpr float MAX_DECAY = 0.16f, MAX_SWING = 2.5f;
+// The backward's two-term node powers (smooth_bwd.cu) want the decay smaller: 0.045^2 / 4 = 5e-4.
+static constexpr float MAX_DECAY = 0.16f, MAX_SWING = 2.5f, MAX_DECAY_BWD = 0.045f;
 
 // Per-call workspace (after the status block), written by the prep kernels.
 struct Ws {
@@ -42,14 +43,17 @@ struct Ws {
     int2* meta;             // [B * nT][IB * 128] {row of the E tables, first valid step | last << 8}
     uint4* mask;            // [B * nT][IB][128] bit i of row t: item i of the block is valid at step t
     int* n_items;           // [B * nT]
-    int* level;             // [B * nT]
+    int* level;             // [B * nT] of the forward
+    int* level_bwd;         // [B * nT] of the backward
+    unsigned char* do_img;  // N = 128, backward: [B * nT][H][NCH][ATOM] dO' operand tiles
     int IB;                 // item blocks reserved per tile
 };
 
-inline size_t ws_bytes(int64_t B, int64_t H, int64_t T, int64_t N, int64_t K) {
+inline size_t ws_bytes(int64_t B, int64_t H, int64_t T, int64_t N, int64_t K, bool backward) {
     const size_t tiles = (size_t)B * ((T + TM - 1) / TM), IB = (size_t)(K + TM + IBLK - 1) / IBLK, NK = (size_t)N / 64;
     return align_up((size_t)N * N * 4, 1024) + SEG_IMAGES * (size_t)H * NCH * NK * WPIECE + tiles * IB * NK * ATOM +
-           align_up(tiles * IB * IBLK * sizeof(int2), 1024) + tiles * IB * IBLK * sizeof(uint4) + 2 * align_up(tiles * 4, 1024) + 1024;
+           align_up(tiles * IB * IBLK * sizeof(int2), 1024) + tiles * IB * IBLK * sizeof(uint4) + 3 * align_up(tiles * 4, 1024) +
+           (backward && NK == 2 ? tiles * H * NCH * ATOM : 0) + 1024;
 }
 
 inline Ws carve(void* p0, int64_t B, int64_t H, int64_t T, int64_t N, int64_t K) {
@@ -63,7 +67,9 @@ inline Ws carve(void* p0, int64_t B, int64_t H, int64_t T, int64_t N, int64_t K)
     w.meta = reinterpret_cast<int2*>(p); p += align_up(tiles * IB * IBLK * sizeof(int2), 1024);
     w.mask = reinterpret_cast<uint4*>(p); p += tiles * IB * IBLK * sizeof(uint4);
     w.n_items = reinterpret_cast<int*>(p); p += align_up(tiles * 4, 1024);
-    w.level = reinterpret_cast<int*>(p);
+    w.level = reinterpret_cast<int*>(p); p += align_up(tiles * 4, 1024);
+    w.level_bwd = reinterpret_cast<int*>(p); p += align_up(tiles * 4, 1024);
+    w.do_img = p;
     return w;
 }
 
@@ -83,6 +89,7 @@ static constexpr float TAN_PI_8 = 0.41421356237f;
 
 int prepare(const FlashArgs& a, const Ws& w, cudaStream_t st);
 int forward(const FlashArgs& a, const Ws& w, int* status, cudaStream_t st);
+int backward(const FlashArgs& a, const Ws& w, int* status, cudaStream_t st);
 
 }  // namespace smooth
 }  // namespace mbema

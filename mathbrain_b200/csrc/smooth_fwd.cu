@@ -12,7 +12,7 @@
 // Bound: special functions and issue slots, not the tensor cores.  A block takes 4 * 64 tanh per item and one exponential
 // per item and step (3072 cycles of the special-function pipe at 16 a clock), 2560 cycles of tensor work.
 #include "smooth.cuh"
-#include "sm100_ptx.cuh"
+#include "smooth_dev.cuh"
 
 namespace mbema {
 namespace smooth {
@@ -38,29 +38,6 @@ struct Bars {
 static constexpr int Q_OFF = 0, A_OFF = Q_OFF + NCH * ATOM, W_OFF = A_OFF + 2 * ATOM, K_OFF = W_OFF + 2 * WPIECE, V_OFF = K_OFF + 2 * ATOM,
                      MX_OFF = V_OFF + NCH * ATOM, BAR_OFF = MX_OFF + 4 * TM * 4, SMEM = BAR_OFF + 512 + 1024;
 static_assert(sizeof(Bars) <= 512 && SMEM <= 227 * 1024, "shared memory");
-
-// 16 columns of an E row, raw
-template <bool EF32> struct ERow { uint4 v[EF32 ? 4 : 2]; };
-template <bool EF32>
-__device__ __forceinline__ ERow<EF32> load_e(const void* E, size_t off) {
-    ERow<EF32> r;
-    const uint4* p = reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned char*>(E) + off * (EF32 ? 4 : 2));
-#pragma unroll
-    for (int i = 0; i < (EF32 ? 4 : 2); ++i) r.v[i] = __ldg(p + i);
-    return r;
-}
-// columns 2p, 2p + 1 as fp16, times 1/4
-template <bool EF32>
-__device__ __forceinline__ uint32_t e_pair(const ERow<EF32>& r, int p) {
-    const uint32_t* u = reinterpret_cast<const uint32_t*>(r.v);
-    if (EF32) return pack_f16x2_sat(__uint_as_float(u[2 * p]) * 0.25f, __uint_as_float(u[2 * p + 1]) * 0.25f);
-    return pack_f16x2_sat(bf16_lo(u[p]) * 0.25f, bf16_hi(u[p]) * 0.25f);
-}
-
-// a wait whose outcome is the same for the whole warp (the code after it has warp-wide instructions)
-__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int tag, const unsigned* lim) {
-    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, tag, lim));
-}
 
 template <bool SILU, int NK, bool EF32>
 __global__ void __launch_bounds__(THREADS, 1) k_smooth_fwd(FlashArgs a, Ws w, int* status) {
@@ -112,15 +89,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_fwd(FlashArgs a, Ws w, in
             const float4 v = t0 + t < Lb ? ld4_dyn_f32(a.Q, a.q_dt, (row0 + t) * HD + c * 16 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
             q[i] = v.x; q[i + 1] = v.y; q[i + 2] = v.z; q[i + 3] = v.w;
         }
-#pragma unroll
-        for (int j = 0; j < NJ; ++j) {
-            const float s = beta[j] * (0.125f * 1.4426950409f);
-#pragma unroll
-            for (int g = 0; g < 2; ++g)
-                *reinterpret_cast<uint4*>(sm + Q_OFF + c * ATOM + t * 128 + (((2 * j + g) ^ (t & 7)) << 4)) =
-                    make_uint4(pack_f16x2_sat(q[8 * g] * s, q[8 * g + 1] * s), pack_f16x2_sat(q[8 * g + 2] * s, q[8 * g + 3] * s),
-                               pack_f16x2_sat(q[8 * g + 4] * s, q[8 * g + 5] * s), pack_f16x2_sat(q[8 * g + 6] * s, q[8 * g + 7] * s));
-        }
+        store_basis_rows(sm + Q_OFF + c * ATOM, t, q, beta, 0.125f * 1.4426950409f);
     }
     fence_proxy_async_smem();
     tc_fence_before_sync();
@@ -171,26 +140,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_fwd(FlashArgs a, Ws w, in
 #pragma unroll
                 for (int g = 0; g < 2; ++g) {
                     uint32_t cf[NJ][4];
-#pragma unroll
-                    for (int p = 0; p < 4; ++p) {
-                        f32x2 gt[NJ];
-#pragma unroll
-                        for (int j = 0; j < NJ; ++j) {
-                            const float h0 = x[g][j][2 * p], h1 = x[g][j][2 * p + 1];
-                            const f32x2 hh = pack2(h0, h1);
-                            gt[j] = SILU ? fma2(hh, pack2(tanh_approx(h0), tanh_approx(h1)), hh) : hh;
-                        }
-                        const f32x2 m1 = pack2(-1.f, -1.f), ka = pack2(TAN_PI_8, TAN_PI_8), kn = pack2(-TAN_PI_8, -TAN_PI_8);
-                        const f32x2 s03 = add2(gt[0], gt[3]), s12 = add2(gt[1], gt[2]);
-                        const f32x2 d03 = fma2(gt[3], m1, gt[0]), d12 = fma2(gt[2], m1, gt[1]);
-                        const f32x2 cj[NJ] = {add2(s03, s12), fma2(d12, ka, d03), fma2(s12, m1, s03), fma2(d03, kn, d12)};
-#pragma unroll
-                        for (int j = 0; j < NJ; ++j) {
-                            float lo, hi;
-                            unpack2(cj[j], lo, hi);
-                            cf[j][p] = pack_f16x2_sat(lo, hi);
-                        }
-                    }
+                    gate_coefficients<SILU, false>(x[g], cf, cf);
                     if (g == 0) {
                         tmem_wait_ld();            // the second half's columns are in registers
                         tc_fence_before_sync();

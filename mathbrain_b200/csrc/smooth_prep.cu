@@ -69,7 +69,7 @@ __global__ void __launch_bounds__(IT_THREADS) k_items(FlashArgs a, Ws w) {
     const int bt = b * a.nT + tile;
     const int Lb = a.seq_lens ? min(max(a.seq_lens[b], 0), a.T) : a.T;
     if (t0 >= Lb) {
-        if (tid == 0) { w.n_items[bt] = 0; w.level[bt] = 0; }
+        if (tid == 0) { w.n_items[bt] = 0; w.level[bt] = w.level_bwd[bt] = 0; }
         return;
     }
     int2* meta = w.meta + (size_t)bt * w.IB * IBLK;
@@ -246,9 +246,13 @@ __global__ void __launch_bounds__(IT_THREADS) k_items(FlashArgs a, Ws w) {
     if (tid == 0) {
         w.n_items[bt] = n_items;
         const float swing = 64.0f * sqrtf(__uint_as_float(swing_sh)), decay = 64.0f * __uint_as_float(decay_sh);
-        int level = 0;
-        while (level < LEVEL_EXACT && !(decay <= MAX_DECAY * (float)(1 << level) && swing <= MAX_SWING * (float)(1 << level))) ++level;
-        w.level[bt] = exact_sh ? LEVEL_EXACT : level;
+        auto pick = [&](float max_decay) {
+            int level = 0;
+            while (level < LEVEL_EXACT && !(decay <= max_decay * (float)(1 << level) && swing <= MAX_SWING * (float)(1 << level))) ++level;
+            return exact_sh ? LEVEL_EXACT : level;
+        };
+        w.level[bt] = pick(MAX_DECAY);
+        w.level_bwd[bt] = pick(MAX_DECAY_BWD);
     }
 }
 
