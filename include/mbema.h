@@ -62,6 +62,7 @@ extern "C" {
 #define MBEMA_FLAG_EVERY_STEP 32       /* MBEMA_MODE_TC_BF16 only: evaluate the gate at every step.  Otherwise the    */
                                        /* kernels evaluate it at four nodes per 128-step tile (or part of it) wherever  */
                                        /* the states decay slowly enough, and at every step where they do not           */
+#define MBEMA_FLAG_TILE_ITEMS 64       /* attention calls: mbema_tile_items has run on this tile_state buffer          */
 /* Test hook of the tensor-core forward and backward: one hand-off between the kernel's warps is withheld and the bounded
  * waits give up after a few polls, so the kernel must end through its give-up path (status word set, products in flight
  * drained, TMEM released, outputs undefined).
@@ -142,6 +143,17 @@ int mbema_tile_states(const int64_t* x, const int64_t* unique, const float* rhos
                       int64_t K, int flags, void* workspace, size_t workspace_bytes, void* stream);
 
 /* ------------------------------------------------------------------------------------------------
+ * What the tensor-core attention kernels read of the snapshots, prepared once for all layers and both directions of a
+ * chunk batch: per (sample, tile) the list of slots and occurrences with their states as operand tiles.  Optional: an
+ * attention call without MBEMA_FLAG_TILE_ITEMS builds them in its own workspace every time.
+ *   tile_state is the buffer mbema_tile_states filled, 1024-byte aligned and mbema_tile_items_bytes(...) long (the snapshots
+ *   and, behind them, the items); 0 bytes: the shape has no tensor-core kernels.  seq_lens as in the attention calls.
+ * ---------------------------------------------------------------------------------------------- */
+size_t mbema_tile_items_bytes(int64_t B, int64_t T, int64_t N, int64_t K);
+int mbema_tile_items(const int64_t* x, const int64_t* unique, const float* rhos, float* tile_state, const float* tok_state,
+                     const int32_t* kcount, const int32_t* seq_lens, int64_t B, int64_t T, int64_t N, int64_t K, void* stream);
+
+/* ------------------------------------------------------------------------------------------------
  * Query gate + LayerNorm, forward and backward.
  * Replaces FusedGatingFunction (mathbrain/triton_fused_gating.py:122-177; kernels :12-57, :61-119).
  *   Y = LayerNorm_eps(x_q * gate(p_pre + bias)) * ln_w + ln_b,  gate = SiLU or identity.
@@ -174,6 +186,7 @@ int mbema_qgate_bwd(const void* dY, int dy_dtype, const void* x_q, int x_dtype, 
  * chooses between its kernels by itself (mathbrain/model.py:78: `if HAS_TRITON and Q_t.is_cuda`); a caller that wants the
  * same behaviour asks here and passes MBEMA_MODE_FP32 otherwise. */
 int mbema_flash_tc_supported(int64_t H, int64_t N, int64_t K);
+/* mode | MBEMA_FLAG_TILE_ITEMS: for calls that pass that flag */
 size_t mbema_flash_fwd_workspace_bytes(int64_t B, int64_t H, int64_t T, int64_t hd, int64_t N, int64_t K, int mode);
 int mbema_flash_fwd(const void* Q, int q_dtype, const int64_t* x, const void* E_k, const void* E_v, int e_dtype,
                     const float* W_pe, const float* rhos, const int64_t* unique, const float* tile_state,

@@ -10,7 +10,7 @@ LIB_PATH = os.path.join(HERE, "libmbema.so")
 
 F32, BF16 = 0, 1
 FLAG_SILU, FLAG_LISTED_ONLY, FLAG_CBASE_EXTRA_DECAY, FLAG_FP32_BACKWARD, FLAG_INDEX_READY = 1, 2, 4, 8, 16
-FLAG_EVERY_STEP = 32
+FLAG_EVERY_STEP, FLAG_TILE_ITEMS = 32, 64
 FLAG_TEST_WITHHOLD_ARRIVE = 1 << 30
 MODE_FP32, MODE_TC_BF16 = 0, 1
 TILE_T = 128
@@ -27,6 +27,8 @@ SIGNATURES = {
     "mbema_query_scan_static": (_i32, [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _i32, _vp]),
     "mbema_tile_states_workspace_bytes": (_sz, [_i64, _i64]),
     "mbema_tile_states": (_i32, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _i32, _vp, _sz, _vp]),
+    "mbema_tile_items_bytes": (_sz, [_i64] * 4),
+    "mbema_tile_items": (_i32, [_vp] * 7 + [_i64] * 4 + [_vp]),
     "mbema_qgate_fwd": (_i32, [_vp, _i32, _vp, _i32, _vp, _vp, _vp, _f32, _vp, _i32, _vp, _vp, _i64, _i64, _i32, _vp]),
     "mbema_qgate_bwd_workspace_bytes": (_sz, [_i64, _i64]),
     "mbema_qgate_bwd": (_i32, [_vp, _i32, _vp, _i32, _vp, _i32, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp,

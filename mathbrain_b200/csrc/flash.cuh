@@ -4,7 +4,7 @@
 
 namespace mbema {
 
-namespace smooth { struct Ws; }
+namespace smooth { struct Items; struct Ws; }
 
 struct FlashArgs {
     const void* Q; int q_dt;
@@ -25,6 +25,8 @@ struct FlashArgs {
     float v_total;
     int silu, listed_only;
     const int* level;       // [B, nT] or null: the every-step tensor-core kernels work on the tiles marked smooth::LEVEL_EXACT only
+    const int* hot;         // with level: [B, nT][smooth::HOT + 1] hot slots of every other tile, which the backward adds to what the
+                            // smooth-state kernel left there
     int test_withhold;      // test hook: see MBEMA_FLAG_TEST_WITHHOLD_ARRIVE
 };
 
@@ -42,7 +44,7 @@ bool flash_tc_supported(int H, int N, int K);
 int flash_fwd_tc(const FlashArgs& a, void* ws, cudaStream_t st);
 bool flash_bwd_tc_supported(int H, int N, int K);
 size_t flash_bwd_tc_ws(int64_t B, int64_t H, int64_t T, int64_t N);
-// smooth_ws: workspace of the smooth-state kernels, which then take the tiles they can (null: every step everywhere)
-int flash_bwd_tc(FlashArgs a, const smooth::Ws* smooth_ws, float* dW, void* ws, cudaStream_t st);
+// it, w: the smooth-state kernels take what they can (null: every step everywhere)
+int flash_bwd_tc(FlashArgs a, const smooth::Items* it, const smooth::Ws* w, float* dW, void* ws, cudaStream_t st);
 
 }  // namespace mbema

@@ -34,6 +34,40 @@ static FlashArgs pack(const void* Q, int q_dtype, const int64_t* x, const void* 
     return a;
 }
 
+// offset of the items block of mbema_tile_items behind the snapshots
+static size_t items_offset(int64_t B, int64_t T, int64_t N, int64_t K) {
+    return align_up((size_t)B * ((T + MBEMA_TILE_T - 1) / MBEMA_TILE_T) * K * N * 6, 1024);
+}
+
+extern "C" size_t mbema_tile_items_bytes(int64_t B, int64_t T, int64_t N, int64_t K) {
+    return (N == 64 || N == 128) && flash_tc_supported(2, (int)N, (int)K) ? items_offset(B, T, N, K) + smooth::items_bytes(B, T, N, K) : 0;
+}
+
+extern "C" int mbema_tile_items(const int64_t* x, const int64_t* unique, const float* rhos, float* tile_state, const float* tok_state,
+                                const int32_t* kcount, const int32_t* seq_lens, int64_t B, int64_t T, int64_t N, int64_t K,
+                                void* stream) {
+    if (B < 0 || T < 1 || N < 1 || K < 1) return MBEMA_ERR_SHAPE;
+    if (T > 8192 || B > 65535 || mbema_tile_items_bytes(B, T, N, K) == 0) return MBEMA_ERR_UNSUPPORTED;
+    if (B == 0) return MBEMA_OK;
+    if (!x || !unique || !rhos || !tile_state || !tok_state || !kcount) return MBEMA_ERR_NULL;
+    if (((uintptr_t)tile_state & 1023) || ((uintptr_t)tok_state & 15)) return MBEMA_ERR_ALIGN;
+    const FlashArgs a = pack(nullptr, 0, x, nullptr, nullptr, 0, nullptr, rhos, unique, tile_state, tok_state, kcount, seq_lens, B, 1, T,
+                             N, K, 0, 0);
+    return smooth::build_items(a, smooth::carve_items(reinterpret_cast<unsigned char*>(tile_state) + items_offset(B, T, N, K), B, T, N, K),
+                               (cudaStream_t)stream);
+}
+
+// the items of an attention call: prepared behind the snapshots, or built now in the workspace
+static int items_of(const FlashArgs& a, int flags, void* ws, smooth::Items& it, cudaStream_t st) {
+    if (flags & MBEMA_FLAG_TILE_ITEMS) {
+        it = smooth::carve_items(const_cast<unsigned char*>(reinterpret_cast<const unsigned char*>(a.tile_state)) + items_offset(a.B, a.T, a.N, a.K),
+                                 a.B, a.T, a.N, a.K);
+        return MBEMA_OK;
+    }
+    it = smooth::carve_items(ws, a.B, a.T, a.N, a.K);
+    return smooth::build_items(a, it, st);
+}
+
 extern "C" int mbema_flash_tc_supported(int64_t H, int64_t N, int64_t K) {
     if (H < 1 || N < 1 || K < 1 || H > 65535 || K > (1 << 20)) return 0;
     return flash_tc_supported((int)H, (int)N, (int)K) ? 1 : 0;
@@ -43,7 +77,8 @@ extern "C" int mbema_flash_tc_supported(int64_t H, int64_t N, int64_t K) {
 static constexpr size_t STATUS_BYTES = 512;
 
 extern "C" size_t mbema_flash_fwd_workspace_bytes(int64_t B, int64_t H, int64_t T, int64_t, int64_t N, int64_t K, int mode) {
-    return mode == MBEMA_MODE_TC_BF16 ? STATUS_BYTES + smooth::ws_bytes(B, H, T, N, K, false) : 256;
+    if (mode == (MBEMA_MODE_TC_BF16 | MBEMA_FLAG_TILE_ITEMS)) return STATUS_BYTES + smooth::ws_bytes(B, H, T, N, false);
+    return mode == MBEMA_MODE_TC_BF16 ? STATUS_BYTES + smooth::ws_bytes(B, H, T, N, false) + smooth::items_bytes(B, T, N, K) : 256;
 }
 
 static int flash_fwd_impl(const void* Q, int q_dtype, const int64_t* x, const void* E_k, const void* E_v,
@@ -68,12 +103,16 @@ static int flash_fwd_impl(const void* Q, int q_dtype, const int64_t* x, const vo
     if (e_row_index) { a.erow = e_row_index; a.e_rows = e_rows; }
     if (mode == MBEMA_MODE_TC_BF16) {
         if (!workspace) return MBEMA_ERR_NULL;
-        if (workspace_bytes < mbema_flash_fwd_workspace_bytes(B, H, T, hd, N, K, mode)) return MBEMA_ERR_WORKSPACE;
+        if (workspace_bytes < mbema_flash_fwd_workspace_bytes(B, H, T, hd, N, K, mode | (flags & MBEMA_FLAG_TILE_ITEMS))) return MBEMA_ERR_WORKSPACE;
         cudaStream_t st = (cudaStream_t)stream;
         if (flags & MBEMA_FLAG_EVERY_STEP) return flash_fwd_tc(a, workspace, st);
         int* status = reinterpret_cast<int*>((reinterpret_cast<uintptr_t>(workspace) + 15) & ~uintptr_t(15));
-        const smooth::Ws w = smooth::carve(static_cast<unsigned char*>(workspace) + STATUS_BYTES, B, H, T, N, K);
-        if ((rc = smooth::prepare(a, w, st)) || (rc = smooth::forward(a, w, status, st))) return rc;
+        unsigned char* p = static_cast<unsigned char*>(workspace) + STATUS_BYTES;
+        const smooth::Ws w = smooth::carve(p, B, H, T, N);
+        smooth::Items it;
+        if ((rc = items_of(a, flags, p + smooth::ws_bytes(B, H, T, N, false), it, st)) || (rc = smooth::prepare(a, it, w, st)) ||
+            (rc = smooth::forward(a, it, w, status, st)))
+            return rc;
         a.level = w.level;
         return flash_fwd_tc(a, workspace, st);
     }
@@ -106,10 +145,12 @@ extern "C" int mbema_flash_fwd_rows(const void* Q, int q_dtype, const int64_t* x
 extern "C" size_t mbema_flash_bwd_workspace_bytes(int64_t B, int64_t H, int64_t T, int64_t hd, int64_t N, int64_t K,
                                                   int mode) {
     (void)hd;
+    const bool items = !(mode & MBEMA_FLAG_TILE_ITEMS);
+    mode &= ~MBEMA_FLAG_TILE_ITEMS;
     // in tensor-core mode the first 512 bytes hold the kernel status word, whichever kernel ends up running
     size_t need = flash_bwd_simt_ws(B, H, T, N) + (mode == MBEMA_MODE_TC_BF16 ? 512 : 0);
     if (mode == MBEMA_MODE_TC_BF16 && flash_bwd_tc_supported((int)H, (int)N, (int)K)) {
-        const size_t tc = align_up(flash_bwd_tc_ws(B, H, T, N), 1024) + smooth::ws_bytes(B, H, T, N, K, true);
+        const size_t tc = flash_bwd_tc_ws(B, H, T, N) + smooth::ws_bytes(B, H, T, N, true) + (items ? smooth::items_bytes(B, T, N, K) : 0);
         if (tc > need) need = tc;
     }
     return need;
@@ -138,7 +179,7 @@ static int flash_bwd_impl(const void* Q, int q_dtype, const int64_t* x, const vo
     if (((uintptr_t)Q | (uintptr_t)E_k | (uintptr_t)E_v | (uintptr_t)O | (uintptr_t)dO | (uintptr_t)dQ | (uintptr_t)W_pe |
          (uintptr_t)tile_state | (uintptr_t)tok_state | (uintptr_t)dE_k | (uintptr_t)dE_v | (uintptr_t)dW_pe) & 15)
         return MBEMA_ERR_ALIGN;
-    if (workspace_bytes < mbema_flash_bwd_workspace_bytes(B, H, T, hd, N, K, mode)) return MBEMA_ERR_WORKSPACE;
+    if (workspace_bytes < mbema_flash_bwd_workspace_bytes(B, H, T, hd, N, K, mode | (flags & MBEMA_FLAG_TILE_ITEMS))) return MBEMA_ERR_WORKSPACE;
     FlashArgs a = pack(Q, q_dtype, x, E_k, E_v, e_dtype, W_pe, rhos, unique, tile_state, tok_state, kcount, seq_lens,
                        B, H, T, N, K, V_total, flags);
     a.O = const_cast<float*>(O); a.LSE = const_cast<float*>(LSE);
@@ -147,8 +188,12 @@ static int flash_bwd_impl(const void* Q, int q_dtype, const int64_t* x, const vo
     // tensor-core backward where the shape fits its shared-memory budget (N == 64); otherwise the fp32 kernels
     if (mode == MBEMA_MODE_TC_BF16) {
         if (!(flags & MBEMA_FLAG_FP32_BACKWARD) && flash_bwd_tc_supported((int)H, (int)N, (int)K)) {
-            const smooth::Ws w = smooth::carve(static_cast<unsigned char*>(workspace) + flash_bwd_tc_ws(B, H, T, N), B, H, T, N, K);
-            return flash_bwd_tc(a, (flags & MBEMA_FLAG_EVERY_STEP) ? nullptr : &w, dW_pe, workspace, st);
+            if (flags & MBEMA_FLAG_EVERY_STEP) return flash_bwd_tc(a, nullptr, nullptr, dW_pe, workspace, st);
+            unsigned char* p = static_cast<unsigned char*>(workspace) + flash_bwd_tc_ws(B, H, T, N);
+            const smooth::Ws w = smooth::carve(p, B, H, T, N);
+            smooth::Items it;
+            if ((rc = items_of(a, flags, p + smooth::ws_bytes(B, H, T, N, true), it, st))) return rc;
+            return flash_bwd_tc(a, &it, &w, dW_pe, workspace, st);
         }
         // (the first 512 bytes stay reserved for the status word of the tensor-core kernels; the fp32 kernels have no
         // bounded waits and leave it alone)

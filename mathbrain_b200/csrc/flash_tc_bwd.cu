@@ -137,7 +137,10 @@ __global__ void __launch_bounds__(THREADS, 1) k_flash_bwd_tc(FlashArgs a, int* s
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int D = a.H * HD;
     const int t0 = tile * TM;
-    if (a.level && a.level[b * a.nT + tile] != smooth::LEVEL_EXACT) return;      // done by the smooth-state kernel
+    // the whole tile, or (the rest being done by the smooth-state kernel) its hot slots, added to what stands there
+    const bool add = a.level && a.level[b * a.nT + tile] != smooth::LEVEL_EXACT;
+    const int* hot = add ? a.hot + (b * a.nT + tile) * (smooth::HOT + 1) : nullptr;
+    if (add && hot[0] == 0) return;
     const int Lb = a.seq_lens ? min(max(a.seq_lens[b], 0), a.T) : a.T;
     const bool is_epi = warp < EPI_WARPS;
     const int row = (warp & 3) * 32 + lane;
@@ -180,7 +183,14 @@ __global__ void __launch_bounds__(THREADS, 1) k_flash_bwd_tc(FlashArgs a, int* s
     }
     if (warp == EPI_WARPS + 1) {
         int n = 0;
-        for (int k0 = 0; k0 < a.K; k0 += 32) {
+        if (add) {
+            n = hot[0];
+            if (lane < n) {
+                slot_sh[lane] = (unsigned short)hot[1 + lane];
+                key_sh[lane] = (int)(a.unique[(size_t)b * a.K + hot[1 + lane]] & 0x7fffffffLL);
+            }
+        }
+        for (int k0 = 0; k0 < a.K && !add; k0 += 32) {
             const int k = k0 + lane;
             const long long kv = (k < a.K) ? a.unique[(size_t)b * a.K + k] : -1;
             const bool ok = kv >= 0;
@@ -677,8 +687,11 @@ __global__ void __launch_bounds__(THREADS, 1) k_flash_bwd_tc(FlashArgs a, int* s
             tmem_wait_ld();
             if (t < a.T && !*abort_flag) {      // after a give-up nothing of this CTA is stored (the status word says so)
 #pragma unroll
-                for (int i = 0; i < 16; i += 4)
-                    *reinterpret_cast<float4*>(a.dQ + qoff + c * 16 + i) = make_float4(dq[i], dq[i + 1], dq[i + 2], dq[i + 3]);
+                for (int i = 0; i < 16; i += 4) {
+                    float4* o = reinterpret_cast<float4*>(a.dQ + qoff + c * 16 + i);
+                    const float4 v = add ? *o : make_float4(0.f, 0.f, 0.f, 0.f);
+                    *o = make_float4(v.x + dq[i], v.y + dq[i + 1], v.z + dq[i + 2], v.w + dq[i + 3]);
+                }
             }
         }
         if (wg == 0) {   // dW^T accumulator: lane = column d of the head pair, TMEM columns = n
@@ -693,7 +706,10 @@ __global__ void __launch_bounds__(THREADS, 1) k_flash_bwd_tc(FlashArgs a, int* s
                     for (int j = 0; j < 32; ++j) acc[j] = 0.f;
                 }
 #pragma unroll
-                for (int j = 0; j < 32; ++j) part_out[(size_t)(c * 32 + j) * ACC_COLS + row] = acc[j] * (STATE_F16_UNSCALE / sigma);
+                for (int j = 0; j < 32; ++j) {
+                    float* o = part_out + (size_t)(c * 32 + j) * ACC_COLS + row;
+                    *o = acc[j] * (STATE_F16_UNSCALE / sigma) + (add ? *o : 0.f);
+                }
             }
         }
     }
@@ -731,16 +747,17 @@ size_t flash_bwd_tc_ws(int64_t B, int64_t H, int64_t T, int64_t N) {
     return 256 + (size_t)(B * (H / tcb::HPC) * nT) * N * tcb::ACC_COLS * sizeof(float) + 256;
 }
 
-int flash_bwd_tc(FlashArgs a, const smooth::Ws* smooth_ws, float* dW, void* ws, cudaStream_t st) {
+int flash_bwd_tc(FlashArgs a, const smooth::Items* it, const smooth::Ws* w, float* dW, void* ws, cudaStream_t st) {
     const int D = a.H * tcb::HD;
     int* status = reinterpret_cast<int*>((reinterpret_cast<uintptr_t>(ws) + 255) & ~uintptr_t(255));
     a.dW_part = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(status) + 256);
     MBEMA_CUDA_TRY(cudaMemsetAsync(a.dEk, 0, (size_t)a.e_rows * D * sizeof(float), st));
     MBEMA_CUDA_TRY(cudaMemsetAsync(a.dEv, 0, (size_t)a.e_rows * D * sizeof(float), st));
-    if (smooth_ws) {
+    if (it) {
         int rc;
-        if ((rc = smooth::prepare(a, *smooth_ws, st)) || (rc = smooth::backward(a, *smooth_ws, status, st))) return rc;
-        a.level = smooth_ws->level_bwd;
+        if ((rc = smooth::prepare(a, *it, *w, st)) || (rc = smooth::backward(a, *it, *w, status, st))) return rc;
+        a.level = w->level_bwd;
+        a.hot = it->hot;
     }
     const tcb::Smem L = tcb::smem_layout(a.K, a.N / 64);
     dim3 grid(a.nT, a.H / tcb::HPC, a.B);

@@ -9,8 +9,8 @@
 // state (state + 1) rho^-(step), extended backwards to the tile start and valid for the steps after it.
 //
 // Error: the remainder of the cubic interpolant is f''''(x) d^4 / 192 with d the change of the pre-activation over half
-// a tile.  k_items measures d per tile (root mean square over the gate's columns of M . lambda . W * 64) and the decay
-// over half a tile, and picks the number of segments the tile is cut into (1, 2, 4 or 8, each with nodes of its own);
+// a tile.  k_levels takes d per tile (root mean square over the gate's columns of M . lambda . W * 64) and the decay over
+// half a tile, and picks the number of segments the tile is cut into (1, 2, 4 or 8, each with nodes of its own);
 // what eight segments do not resolve goes to the kernels that evaluate every step (level LEVEL_EXACT).  With
 // half-lives of 1024..4096, states to 600 and W_pe ~ N(0, 0.02^2) the outputs differ from the exact sum by 1e-6 and
 // dW_pe by 1e-4 (norm-wise), against about 1e-3 from the 16-bit operands.
@@ -35,38 +35,65 @@ static constexpr int SEG_IMAGES = (1 << LEVELS) - 1;   // W' images: segment s o
 // The backward's two-term node powers (smooth_bwd.cu) want the decay smaller: 0.045^2 / 4 = 5e-4.
 static constexpr float MAX_DECAY = 0.16f, MAX_SWING = 2.5f, MAX_DECAY_BWD = 0.045f;
 
-// Per-call workspace (after the status block), written by the prep kernels.
+// Slots with the largest states, per tile.  They stand at the end of the item list, in blocks of their own: the forward walks
+// all blocks, the backward leaves these slots to the every-step kernel.  Their pre-activations move most inside a tile
+// and their gradient rows are the largest of a batch (tens of times the mean), at 1 to 5 % of the work.
+static constexpr int HOT = 16;
+
+// What precompute_boundaries prepares once for all attention calls on a chunk batch: the items of every (sample, tile).
+struct Items {
+    unsigned char* a_img;   // [B * nT][IB][N / 64][ATOM] item states, fp16 of state / 64, swizzled operand tiles
+    uint4* mask;            // [B * nT][IB][128] bit i of row t: item i of the block is valid at step t
+    int2* meta;             // [B * nT][IB * 128] {slot, first valid step | last << 8}
+    int* src;               // [B * nT][IB * 128] where the state comes from: slot k (snapshot) or -1 - step (occurrence); INT_MAX: padding
+    float* q;               // [B * nT][IB * 128] |lambda . state|^2
+    int4* count;            // [B * nT] {items and blocks before the hot ones, items and blocks in all}
+    int* hot;               // [B * nT][HOT + 1] number of hot slots, the slots
+    int IB;                 // blocks reserved per tile
+};
+
+// Per-call workspace (after the status block).
 struct Ws {
     float* gram;            // [N, N] W_pe W_pe^T / D
     unsigned char* w_img;   // [SEG_IMAGES][H][NCH][N / 64][WPIECE] node-scaled W_pe, fp16, swizzled operand pieces
-    unsigned char* a_img;   // [B * nT][IB][N / 64][ATOM] item states, fp16 of state / 64, swizzled operand tiles
-    int2* meta;             // [B * nT][IB * 128] {row of the E tables, first valid step | last << 8}
-    uint4* mask;            // [B * nT][IB][128] bit i of row t: item i of the block is valid at step t
-    int* n_items;           // [B * nT]
     int* level;             // [B * nT] of the forward
     int* level_bwd;         // [B * nT] of the backward
     unsigned char* do_img;  // N = 128, backward: [B * nT][H][NCH][ATOM] dO' operand tiles
-    int IB;                 // item blocks reserved per tile
 };
 
-inline size_t ws_bytes(int64_t B, int64_t H, int64_t T, int64_t N, int64_t K, bool backward) {
-    const size_t tiles = (size_t)B * ((T + TM - 1) / TM), IB = (size_t)(K + TM + IBLK - 1) / IBLK, NK = (size_t)N / 64;
-    return align_up((size_t)N * N * 4, 1024) + SEG_IMAGES * (size_t)H * NCH * NK * WPIECE + tiles * IB * NK * ATOM +
-           align_up(tiles * IB * IBLK * sizeof(int2), 1024) + tiles * IB * IBLK * sizeof(uint4) + 3 * align_up(tiles * 4, 1024) +
+inline size_t items_bytes(int64_t B, int64_t T, int64_t N, int64_t K) {
+    const size_t tiles = (size_t)B * ((T + TM - 1) / TM), IB = (size_t)(K + TM + IBLK - 1) / IBLK + 2, NK = (size_t)N / 64;
+    return tiles * IB * (NK * ATOM + IBLK * (sizeof(uint4) + sizeof(int2) + sizeof(int) + sizeof(float))) + tiles * sizeof(int4) +
+           tiles * (HOT + 1) * 4 + 2048;
+}
+
+inline Items carve_items(void* p0, int64_t B, int64_t T, int64_t N, int64_t K) {
+    const size_t tiles = (size_t)B * ((T + TM - 1) / TM), IB = (size_t)(K + TM + IBLK - 1) / IBLK + 2, NK = (size_t)N / 64;
+    unsigned char* p = reinterpret_cast<unsigned char*>(align_up(reinterpret_cast<size_t>(p0), 1024));
+    Items t;
+    t.IB = (int)IB;
+    t.a_img = p; p += tiles * IB * NK * ATOM;
+    t.mask = reinterpret_cast<uint4*>(p); p += tiles * IB * IBLK * sizeof(uint4);
+    t.meta = reinterpret_cast<int2*>(p); p += tiles * IB * IBLK * sizeof(int2);
+    t.count = reinterpret_cast<int4*>(p); p += tiles * sizeof(int4);
+    t.src = reinterpret_cast<int*>(p); p += tiles * IB * IBLK * sizeof(int);
+    t.q = reinterpret_cast<float*>(p); p += tiles * IB * IBLK * sizeof(float);
+    t.hot = reinterpret_cast<int*>(p);
+    return t;
+}
+
+inline size_t ws_bytes(int64_t B, int64_t H, int64_t T, int64_t N, bool backward) {
+    const size_t tiles = (size_t)B * ((T + TM - 1) / TM), NK = (size_t)N / 64;
+    return align_up((size_t)N * N * 4, 1024) + SEG_IMAGES * (size_t)H * NCH * NK * WPIECE + 2 * align_up(tiles * 4, 1024) +
            (backward && NK == 2 ? tiles * H * NCH * ATOM : 0) + 1024;
 }
 
-inline Ws carve(void* p0, int64_t B, int64_t H, int64_t T, int64_t N, int64_t K) {
-    const size_t tiles = (size_t)B * ((T + TM - 1) / TM), IB = (size_t)(K + TM + IBLK - 1) / IBLK, NK = (size_t)N / 64;
+inline Ws carve(void* p0, int64_t B, int64_t H, int64_t T, int64_t N) {
+    const size_t tiles = (size_t)B * ((T + TM - 1) / TM), NK = (size_t)N / 64;
     unsigned char* p = reinterpret_cast<unsigned char*>(align_up(reinterpret_cast<size_t>(p0), 1024));
     Ws w;
-    w.IB = (int)IB;
     w.gram = reinterpret_cast<float*>(p); p += align_up((size_t)N * N * 4, 1024);
     w.w_img = p; p += SEG_IMAGES * (size_t)H * NCH * NK * WPIECE;
-    w.a_img = p; p += tiles * IB * NK * ATOM;
-    w.meta = reinterpret_cast<int2*>(p); p += align_up(tiles * IB * IBLK * sizeof(int2), 1024);
-    w.mask = reinterpret_cast<uint4*>(p); p += tiles * IB * IBLK * sizeof(uint4);
-    w.n_items = reinterpret_cast<int*>(p); p += align_up(tiles * 4, 1024);
     w.level = reinterpret_cast<int*>(p); p += align_up(tiles * 4, 1024);
     w.level_bwd = reinterpret_cast<int*>(p); p += align_up(tiles * 4, 1024);
     w.do_img = p;
@@ -87,9 +114,12 @@ __device__ __forceinline__ void basis(int row, int level, float (&beta)[NJ]) {
 }
 static constexpr float TAN_PI_8 = 0.41421356237f;
 
-int prepare(const FlashArgs& a, const Ws& w, cudaStream_t st);
-int forward(const FlashArgs& a, const Ws& w, int* status, cudaStream_t st);
-int backward(const FlashArgs& a, const Ws& w, int* status, cudaStream_t st);
+// items of a chunk batch (a: x, unique, rhos, tile_state, tok_state, kcount, seq_lens and the sizes)
+int build_items(const FlashArgs& a, const Items& it, cudaStream_t st);
+// what depends on W_pe: node-scaled images, levels
+int prepare(const FlashArgs& a, const Items& it, const Ws& w, cudaStream_t st);
+int forward(const FlashArgs& a, const Items& it, const Ws& w, int* status, cudaStream_t st);
+int backward(const FlashArgs& a, const Items& it, const Ws& w, int* status, cudaStream_t st);
 
 }  // namespace smooth
 }  // namespace mbema

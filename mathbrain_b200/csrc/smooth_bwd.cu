@@ -55,7 +55,7 @@ __device__ __forceinline__ void red_v4(float* p, float a, float b, float c, floa
 }
 
 template <bool SILU, int NK, bool EF32>
-__global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Ws w, int* status) {
+__global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it, Ws w, int* status) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char* sm = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     using M = L<NK>;
@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Ws w, in
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = bars->tmem_base;
-    const int n_items = w.n_items[bt], n_blk = (n_items + IBLK - 1) / IBLK;
+    const int n_items = it.count[bt].x, n_blk = it.count[bt].y;          // the hot slots are the every-step kernel's
     const int n_it = bars->abort_flag ? 0 : n_blk << level;
     const unsigned* lim = &bars->spin_limit;
     const float unit = exp2f(kappa - 4.0f) * e2 ;         // dS, dK, dc and dpre carry this factor (dS ln 2 more)
@@ -173,11 +173,11 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Ws w, in
         // ======================================================== gate: item r, chunks wg and wg + 2
         const int wg = warp >> 2, r = tid & 127, x7 = r & 7;
         const uint32_t t_lane = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-        const int2* meta = w.meta + (size_t)bt * w.IB * IBLK + r;
+        const int2* meta = it.meta + (size_t)bt * it.IB * IBLK + r;
         unsigned char* kd1 = sm + (wg == 0 ? M::B0 : M::DS) + r * 128;          // first pass: this group's K and V tiles
         unsigned char* vd1 = sm + (wg == 0 ? M::B1 : M::DS + ATOM) + r * 128;
         const float oe = 0.25f / unit, ov = oe * 0.0625f;
-        int er = n_it > 0 ? __ldg(&meta[0].x) : 0, er_next = er;
+        int er = n_it > 0 ? (int)e_row(a, b, __ldg(&meta[0].x)) : 0, er_next = er;
         ERow<EF32> ek, ev;
         if (n_it > 0) {
             ek = load_e<EF32>(a.Ek, (size_t)er * D + h * HD + wg * 16);
@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Ws w, in
                 const bool second = ph >= 2;
                 // the E columns of this thread's next chunk fly while this one is worked on
                 ERow<EF32> nk = ek, nv = ev;
-                if (ph == 2 && i + 1 < n_it) er_next = __ldg(&meta[(size_t)((i + 1) % n_blk) * IBLK].x);
+                if (ph == 2 && i + 1 < n_it) er_next = (int)e_row(a, b, __ldg(&meta[(size_t)((i + 1) % n_blk) * IBLK].x));
                 if (ph < 3 || i + 1 < n_it) {
                     const size_t off = (size_t)(ph == 3 ? er_next : er) * D + h * HD + (wg + 2 * (cc ^ 1)) * 16;
                     nk = load_e<EF32>(a.Ek, off);
@@ -355,7 +355,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Ws w, in
         // ======================================================== softmax (item r, steps 64 half ..), then dQ (step r)
         const int half = (warp >> 2) & 1, r = tid & 127, x7 = r & 7;
         const uint32_t t_lane = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-        const int2* meta = w.meta + (size_t)bt * w.IB * IBLK + r;
+        const int2* meta = it.meta + (size_t)bt * it.IB * IBLK + r;
         float beta[NJ];
         basis(r, level, beta);
         float acc[2][16];
@@ -459,7 +459,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Ws w, in
         asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
         if (warp == W_LOAD && lane == 0) {
             // ==================================================== loader: A per block; W' (and dO') chunks for both passes
-            const unsigned char* img = w.a_img + (size_t)bt * w.IB * NK * ATOM;
+            const unsigned char* img = it.a_img + (size_t)bt * it.IB * NK * ATOM;
             const unsigned char* dimg = NK == 1 ? nullptr : w.do_img + ((size_t)bt * a.H + h) * NCH * ATOM;
             int np = 0, nd = 0;
             bool alive = true;
@@ -613,12 +613,12 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Ws w, in
 
 }  // namespace bwd
 
-int backward(const FlashArgs& a, const Ws& w, int* status, cudaStream_t st) {
+int backward(const FlashArgs& a, const Items& it, const Ws& w, int* status, cudaStream_t st) {
     const dim3 grid(a.nT, a.H, a.B);
 #define MBEMA_SMOOTH(S_, NK_, E_)                                                                                                     \
     do {                                                                                                                               \
         MBEMA_CUDA_TRY(cudaFuncSetAttribute(bwd::k_smooth_bwd<S_, NK_, E_>, cudaFuncAttributeMaxDynamicSharedMemorySize, bwd::L<NK_>::SMEM)); \
-        bwd::k_smooth_bwd<S_, NK_, E_><<<grid, bwd::THREADS, bwd::L<NK_>::SMEM, st>>>(a, w, status);                                    \
+        bwd::k_smooth_bwd<S_, NK_, E_><<<grid, bwd::THREADS, bwd::L<NK_>::SMEM, st>>>(a, it, w, status);                                    \
     } while (0)
 #define MBEMA_SMOOTH_E(S_, NK_) do { if (a.e_dt == MBEMA_F32) MBEMA_SMOOTH(S_, NK_, true); else MBEMA_SMOOTH(S_, NK_, false); } while (0)
     if (a.N == 64) { if (a.silu) MBEMA_SMOOTH_E(true, 1); else MBEMA_SMOOTH_E(false, 1); }

@@ -40,7 +40,7 @@ static constexpr int Q_OFF = 0, A_OFF = Q_OFF + NCH * ATOM, W_OFF = A_OFF + 2 * 
 static_assert(sizeof(Bars) <= 512 && SMEM <= 227 * 1024, "shared memory");
 
 template <bool SILU, int NK, bool EF32>
-__global__ void __launch_bounds__(THREADS, 1) k_smooth_fwd(FlashArgs a, Ws w, int* status) {
+__global__ void __launch_bounds__(THREADS, 1) k_smooth_fwd(FlashArgs a, Items it, Ws w, int* status) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char* sm = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     Bars* bars = reinterpret_cast<Bars*>(sm + BAR_OFF);
@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_fwd(FlashArgs a, Ws w, in
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = bars->tmem_base;
-    const int n_blk = (w.n_items[bt] + IBLK - 1) / IBLK;
+    const int n_blk = it.count[bt].w;
     const int n_it = bars->abort_flag ? 0 : n_blk << level;        // blocks of segment 0, then of segment 1, ...
     const unsigned* lim = &bars->spin_limit;
 
@@ -105,9 +105,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_fwd(FlashArgs a, Ws w, in
         asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
         const int wg = warp >> 2, r = tid & 127;
         const uint32_t t_pre = tmem + ((uint32_t)((warp & 3) * 32) << 16) + T_PRE + wg * 64;
-        const int2* meta = w.meta + (size_t)bt * w.IB * IBLK + r;
+        const int2* meta = it.meta + (size_t)bt * it.IB * IBLK + r;
         const int x7 = r & 7;
-        int er = n_it > 0 ? __ldg(&meta[0].x) : 0;
+        int er = n_it > 0 ? (int)e_row(a, b, __ldg(&meta[0].x)) : 0;
         ERow<EF32> ek, ev;
         if (n_it > 0) {
             ek = load_e<EF32>(a.Ek, (size_t)er * D + h * HD + wg * 16);
@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_fwd(FlashArgs a, Ws w, in
                 const int c = wg + 2 * cc;
                 // the next chunk's E columns fly while this chunk is worked on
                 ERow<EF32> nk = ek, nv = ev;
-                if (cc == 1 && i + 1 < n_it) er = __ldg(&meta[(size_t)((i + 1) % n_blk) * IBLK].x);
+                if (cc == 1 && i + 1 < n_it) er = (int)e_row(a, b, __ldg(&meta[(size_t)((i + 1) % n_blk) * IBLK].x));
                 if (cc == 0 || i + 1 < n_it) {
                     const size_t off = (size_t)er * D + h * HD + (wg + 2 * (cc ^ 1)) * 16;
                     nk = load_e<EF32>(a.Ek, off);
@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_fwd(FlashArgs a, Ws w, in
         const float rest = a.v_total - (float)a.kcount[b];
         float m, l = 0.f;
         if (!a.listed_only && rest > 0.f) { m = 0.f; l = half == 0 ? rest : 0.f; } else m = -INFINITY;
-        const uint2* mask = reinterpret_cast<const uint2*>(w.mask + (size_t)bt * w.IB * IBLK + row) + half;
+        const uint2* mask = reinterpret_cast<const uint2*>(it.mask + (size_t)bt * it.IB * IBLK + row) + half;
         const int my_seg = row / (TM >> level);
         uint2 mk = n_it > 0 ? __ldg(mask) : make_uint2(0u, 0u);
         bool alive = true;
@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_fwd(FlashArgs a, Ws w, in
         asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
         if (warp == W_LOAD && lane == 0) {
             // ==================================================== loader
-            const unsigned char* img = w.a_img + (size_t)bt * w.IB * NK * ATOM;
+            const unsigned char* img = it.a_img + (size_t)bt * it.IB * NK * ATOM;
             int np = 0;
             bool alive = true;
             for (int i = 0; i < n_it && alive; ++i) {
@@ -379,12 +379,12 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_fwd(FlashArgs a, Ws w, in
 
 }  // namespace fwd
 
-int forward(const FlashArgs& a, const Ws& w, int* status, cudaStream_t st) {
+int forward(const FlashArgs& a, const Items& it, const Ws& w, int* status, cudaStream_t st) {
     const dim3 grid(a.nT, a.H, a.B);
 #define MBEMA_SMOOTH(S_, NK_, E_)                                                                                             \
     do {                                                                                                                       \
         MBEMA_CUDA_TRY(cudaFuncSetAttribute(fwd::k_smooth_fwd<S_, NK_, E_>, cudaFuncAttributeMaxDynamicSharedMemorySize, fwd::SMEM)); \
-        fwd::k_smooth_fwd<S_, NK_, E_><<<grid, fwd::THREADS, fwd::SMEM, st>>>(a, w, status);                                    \
+        fwd::k_smooth_fwd<S_, NK_, E_><<<grid, fwd::THREADS, fwd::SMEM, st>>>(a, it, w, status);                                    \
     } while (0)
 #define MBEMA_SMOOTH_E(S_, NK_) do { if (a.e_dt == MBEMA_F32) MBEMA_SMOOTH(S_, NK_, true); else MBEMA_SMOOTH(S_, NK_, false); } while (0)
     if (a.N == 64) { if (a.silu) MBEMA_SMOOTH_E(true, 1); else MBEMA_SMOOTH_E(false, 1); }

@@ -51,126 +51,196 @@ __global__ void __launch_bounds__(256) k_weights(FlashArgs a, Ws w) {
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// one CTA per (tile, sample): items, their operand tiles, validity masks and the tile's level
+// one CTA per (tile, sample): the item list.  A slot is an item from the tile start to its first occurrence; every
+// occurrence is one from the next step to the next occurrence.  Slots in list order, then occurrences in step order; the
+// hot slots and their occurrences the same way in blocks after them.
 // ---------------------------------------------------------------------------------------------------------------
-static constexpr int IT_THREADS = 256;
-static constexpr int MAX_CHECKED = 1024;
+static constexpr int IL_THREADS = 1024;
 
-__global__ void __launch_bounds__(IT_THREADS) k_items(FlashArgs a, Ws w) {
-    __shared__ int tok[TM], head[TM], next[TM], slot_of[TM];
-    __shared__ int hkey[256], hval[256];
-    __shared__ int wsum[8], n_items_sh, exact_sh, n_chk;
-    __shared__ unsigned swing_sh, decay_sh;
-    __shared__ int chk[MAX_CHECKED];
-    __shared__ float rho_sh[128], lam_sh[128];
-    __shared__ int lohi_sh[IBLK];
+struct ListSmem {
+    int tok[TM], head[TM], next[TM], occ[TM], slot_of[TM], hkey[256], hval[256], wsum[2][32], hot[HOT], n_hot, dup, total[2];
+    unsigned long long best[32];
+};
+
+__global__ void __launch_bounds__(IL_THREADS) k_items_list(FlashArgs a, Items it) {
+    extern __shared__ float metric[];          // [K]: size of the slot's state in this tile; negative: not a hot candidate
+    __shared__ ListSmem s;
     const int tile = blockIdx.x, b = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int N = a.N, NK = N >> 6, CH = N / 8, t0 = tile * TM;
-    const int bt = b * a.nT + tile;
+    const int N = a.N, CH = N / 8, t0 = tile * TM, bt = b * a.nT + tile;
     const int Lb = a.seq_lens ? min(max(a.seq_lens[b], 0), a.T) : a.T;
     if (t0 >= Lb) {
-        if (tid == 0) { w.n_items[bt] = 0; w.level[bt] = w.level_bwd[bt] = 0; }
+        if (tid == 0) { it.count[bt] = make_int4(0, 0, 0, 0); it.hot[bt * (HOT + 1)] = 0; }
         return;
     }
-    int2* meta = w.meta + (size_t)bt * w.IB * IBLK;
-    if (tid == 0) { n_items_sh = 0; exact_sh = 0; n_chk = 0; swing_sh = 0u; decay_sh = 0u; }
-    hkey[tid] = -1;
+    int2* meta = it.meta + (size_t)bt * it.IB * IBLK;
+    int* src = it.src + (size_t)bt * it.IB * IBLK;
+    if (tid == 0) { s.n_hot = 0; s.dup = 0; s.total[0] = s.total[1] = 0; }
+    if (tid < 256) s.hkey[tid] = -1;
     if (tid < TM) {
-        tok[tid] = (t0 + tid < Lb) ? (int)(a.x[(size_t)b * a.T + t0 + tid] & 0x7fffffffLL) : -1;
-        slot_of[tid] = -1;
+        s.tok[tid] = (t0 + tid < Lb) ? (int)(a.x[(size_t)b * a.T + t0 + tid] & 0x7fffffffLL) : -1;
+        s.slot_of[tid] = -1;
     }
     __syncthreads();
-    if (tid < N) {
-        const float r = a.rhos[tid];
-        const float lam = fabsf(logf(r));                     // rho = 0: infinite, exact path
-        rho_sh[tid] = log2f(r);
-        lam_sh[tid] = lam;
-        atomicMax(&decay_sh, __float_as_uint(lam == lam ? lam : INFINITY));
-    }
-    if (tid < TM) {            // chains of equal tokens inside the tile: their first step, and the next one after this
-        const int me = tok[tid];
-        int hd = tid, nx = TM - 1;
+    if (tid < TM) {            // equal tokens inside the tile: their first step, their number, the next one after this
+        const int me = s.tok[tid];
+        int hd = tid, nx = TM - 1, n = 0;
         for (int j = TM - 1; j >= 0; --j) {
-            const bool same = tok[j] == me;
+            const bool same = s.tok[j] == me;
+            n += same;
             if (same && j < hd) hd = j;
             if (same && j > tid) nx = j;
         }
-        head[tid] = hd;
-        next[tid] = nx;
+        s.head[tid] = hd;
+        s.next[tid] = nx;
+        s.occ[tid] = n;
         if (me >= 0 && hd == tid) {
             int p = (me * 0x9E3779B1u) >> 24;
-            while (atomicCAS(&hkey[p], -1, me) != -1) p = (p + 1) & 255;
-            hval[p] = tid;
+            while (atomicCAS(&s.hkey[p], -1, me) != -1) p = (p + 1) & 255;
+            s.hval[p] = tid;
         }
     }
     __syncthreads();
-    // slots in list order
-    const int n_valid = a.kcount[b];
-    for (int k0 = 0; k0 < a.K && n_items_sh < n_valid; k0 += IT_THREADS) {
-        const int k = k0 + tid;
-        const long long kv = (k < a.K) ? a.unique[(size_t)b * a.K + k] : -1;
-        const bool ok = kv >= 0;
-        const unsigned m = __ballot_sync(0xffffffffu, ok);
-        if (lane == 0) wsum[warp] = __popc(m);
-        __syncthreads();
-        int pos = n_items_sh + __popc(m & ((1u << lane) - 1u)), total = 0;
+    // sizes: |state at the tile start| + sqrt(N) per occurrence in the tile
+    const __half* snap = reinterpret_cast<const __half*>(a.tile_state + (size_t)a.B * a.nT * a.K * N) + (size_t)bt * a.K * N;
+#pragma unroll 2
+    for (int i0 = 0; i0 < a.K * CH; i0 += IL_THREADS) {
+        const int i = i0 + tid, k = i / CH, c8 = i % CH;
+        const bool in = k < a.K;
+        const uint4 v = in ? __ldg(reinterpret_cast<const uint4*>(snap + (size_t)k * N) + c8) : make_uint4(0u, 0u, 0u, 0u);
+        const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+        float q = 0.f;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) { if (i < warp) pos += wsum[i]; total += wsum[i]; }
-        if (ok) {
-            const int key = (int)(kv & 0x7fffffffLL);
-            int p = (key * 0x9E3779B1u) >> 24, first = -1;
-            while (hkey[p] != -1) {
-                if (hkey[p] == key) { first = hval[p]; break; }
-                p = (p + 1) & 255;
+        for (int e = 0; e < 4; ++e) {
+            const float2 f = unpack_f16x2(u[e]);
+            q = fmaf(f.x, f.x, fmaf(f.y, f.y, q));
+        }
+        for (int o = CH / 2; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+        if (c8 == 0 && in) {
+            const long long kv = a.unique[(size_t)b * a.K + k];
+            float m = -1.f;
+            if (kv >= 0) {
+                m = sqrtf(q) * STATE_F16_UNSCALE;
+                const int key = (int)(kv & 0x7fffffffLL);
+                int p = (key * 0x9E3779B1u) >> 24;
+                while (s.hkey[p] != -1) {
+                    if (s.hkey[p] == key) {
+                        const int f = s.hval[p];
+                        m += (float)s.occ[f] * sqrtf((float)N);
+                        if (atomicExch(&s.slot_of[f], k) >= 0) s.dup = 1;     // a token listed twice: every-step kernels
+                        break;
+                    }
+                    p = (p + 1) & 255;
+                }
             }
-            if (first >= 0 && atomicExch(&slot_of[first], k) >= 0) exact_sh = 1;     // a token listed twice
-            meta[pos] = make_int2(k, (first >= 0 ? first : TM - 1) << 8);
+            metric[k] = m;
+        }
+    }
+    __syncthreads();
+    // the HOT largest, ties by list order
+    for (int r = 0; r < HOT; ++r) {
+        unsigned long long best = 0ull;
+        for (int k = tid; k < a.K; k += IL_THREADS)
+            if (metric[k] >= 0.f) best = max(best, ((unsigned long long)__float_as_uint(metric[k]) << 32) | (unsigned)(0x7fffffff - k));
+        for (int o = 16; o > 0; o >>= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
+        if (lane == 0) s.best[warp] = best;
+        __syncthreads();
+        if (warp == 0) {
+            best = s.best[lane];
+            for (int o = 16; o > 0; o >>= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
+            if (lane == 0 && best != 0ull) {
+                const int k = 0x7fffffff - (int)(best & 0xffffffffull);
+                metric[k] = -2.f;                              // hot
+                s.hot[s.n_hot++] = k;
+            }
         }
         __syncthreads();
-        if (tid == 0) n_items_sh += total;
-        __syncthreads();
     }
-    const int n_slots = n_items_sh;
-    {   // occurrences that have steps after them in the tile
-        const bool ok = tid < TM - 1 && tok[tid & (TM - 1)] >= 0 && slot_of[head[tid & (TM - 1)]] >= 0;
+    if (tid <= HOT) it.hot[bt * (HOT + 1) + tid] = tid == 0 ? s.n_hot : (tid - 1 < s.n_hot ? s.hot[tid - 1] : 0);
+    // ordered compaction, cold items first
+    auto put = [&](bool ok, int cls, int k, int lohi, int from, int base) -> int {     // returns the number of items of class `cls`
         const unsigned m = __ballot_sync(0xffffffffu, ok);
-        if (lane == 0) wsum[warp] = __popc(m);
+        if (lane == 0) s.wsum[0][warp] = __popc(m);
         __syncthreads();
-        int pos = n_slots + __popc(m & ((1u << lane) - 1u)), total = 0;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) { if (i < warp) pos += wsum[i]; total += wsum[i]; }
-        if (ok) meta[pos] = make_int2(-1 - tid, (tid + 1) | (next[tid] << 8));
+        if (warp == 0) {
+            int v = s.wsum[0][lane];
+            for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(0xffffffffu, v, o); if (lane >= o) v += u; }
+            s.wsum[1][lane] = v;
+        }
         __syncthreads();
-        if (tid == 0) n_items_sh += total;
+        if (ok) {
+            const int pos = base + s.total[cls] + (warp ? s.wsum[1][warp - 1] : 0) + __popc(m & ((1u << lane) - 1u));
+            meta[pos] = make_int2(k, lohi);
+            src[pos] = from;
+        }
+        const int n = s.wsum[1][31];
         __syncthreads();
+        if (tid == 0) s.total[cls] += n;
+        __syncthreads();
+        return s.total[cls];
+    };
+    auto first_of = [&](int k) -> int {       // first step of slot k's token in the tile, or the last row
+        const int key = (int)(a.unique[(size_t)b * a.K + k] & 0x7fffffffLL);
+        int p = (key * 0x9E3779B1u) >> 24;
+        while (s.hkey[p] != -1) {
+            if (s.hkey[p] == key) return s.hval[p];
+            p = (p + 1) & 255;
+        }
+        return TM - 1;
+    };
+    for (int k0 = 0; k0 < a.K; k0 += IL_THREADS) {
+        const int k = k0 + tid;
+        const bool ok = k < a.K && metric[k] >= 0.f;
+        put(ok, 0, k, ok ? first_of(k) << 8 : 0, k, 0);
     }
-    const int n_items = n_items_sh, n_blk = (n_items + IBLK - 1) / IBLK;
-    // operand tiles; the items' lambda . M is bounded on the way, and those that could matter are listed for a closer look
-    float trace = 0.f;
-    for (int n = 0; n < N; ++n) trace += w.gram[n * N + n];
-    const float look = (MAX_SWING / 64.0f) * (MAX_SWING / 64.0f) / fmaxf(trace, 1e-30f);     // |v|^2 tr(G) >= v' G v
+    const int own = tid < TM - 1 && s.tok[tid] >= 0 ? s.slot_of[s.head[tid]] : -1;
+    const bool occ = own >= 0, is_hot = occ && metric[own] < 0.f;
+    const int n_cold = put(occ && !is_hot, 0, own, occ ? (tid + 1) | (s.next[tid] << 8) : 0, -1 - tid, 0);
+    const int base = (n_cold + IBLK - 1) / IBLK * IBLK;
+    put(tid < s.n_hot, 1, tid < s.n_hot ? s.hot[tid] : 0, tid < s.n_hot ? first_of(s.hot[tid]) << 8 : 0, tid < s.n_hot ? s.hot[tid] : 0, base);
+    const int n_hot = put(is_hot, 1, own, occ ? (tid + 1) | (s.next[tid] << 8) : 0, -1 - tid, base);
+    const int n_all = base + n_hot, n_blk = (n_all + IBLK - 1) / IBLK;
+    for (int i = n_cold + tid; i < base; i += IL_THREADS) { meta[i] = make_int2(0, 1); src[i] = 0x7fffffff; }      // padding: no valid step
+    for (int i = n_all + tid; i < n_blk * IBLK; i += IL_THREADS) { meta[i] = make_int2(0, 1); src[i] = 0x7fffffff; }
+    if (tid == 0) it.count[bt] = make_int4(s.dup ? -1 - n_cold : n_cold, base / IBLK, n_all, n_blk);
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// one CTA per (block of items, tile, sample): operand tile, validity masks, |lambda . state|^2
+// ---------------------------------------------------------------------------------------------------------------
+__global__ void __launch_bounds__(256) k_items_fill(FlashArgs a, Items it) {
+    __shared__ float rho_sh[128], lam_sh[128];
+    __shared__ int lohi_sh[IBLK], src_sh[IBLK];
+    const int blk = blockIdx.x, bt = blockIdx.z * a.nT + blockIdx.y, tid = threadIdx.x;
+    if (blk >= it.count[bt].w) return;
+    const int N = a.N, NK = N >> 6, CH = N / 8, b = blockIdx.z, t0 = blockIdx.y * TM;
+    const size_t i0 = ((size_t)bt * it.IB + blk) * IBLK;
+    if (tid < N) {
+        const float r = a.rhos[tid];
+        rho_sh[tid] = log2f(r);
+        lam_sh[tid] = fabsf(logf(r)) * STATE_F16_UNSCALE;
+    }
+    if (tid < IBLK) { lohi_sh[tid] = it.meta[i0 + tid].y; src_sh[tid] = it.src[i0 + tid]; }
+    __syncthreads();
     const __half* snap = reinterpret_cast<const __half*>(a.tile_state + (size_t)a.B * a.nT * a.K * N) + (size_t)bt * a.K * N;
     const float* toks = a.tok_state + ((size_t)b * a.T + t0) * N;
-    unsigned char* img = w.a_img + (size_t)bt * w.IB * NK * ATOM;
-    for (int i = tid; i < n_blk * IBLK * CH; i += IT_THREADS) {
-        const int item = i / CH, c8 = i % CH, r = item & (IBLK - 1);
+    unsigned char* img = it.a_img + ((size_t)bt * it.IB + blk) * NK * ATOM;
+#pragma unroll 4
+    for (int i = tid; i < IBLK * CH; i += 256) {
+        const int r = i / CH, c8 = i % CH, from = src_sh[r];
         uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (item < n_items) {
-            const int src = meta[item].x;
-            if (src >= 0) {
-                v = __ldg(reinterpret_cast<const uint4*>(snap + (size_t)src * N) + c8);
-            } else {
-                const int s = -1 - src;
-                const float4* p = reinterpret_cast<const float4*>(toks + (size_t)s * N + c8 * 8);
-                const float4 p0 = __ldg(p), p1 = __ldg(p + 1);
-                const float st[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
-                float o[8];
+        if (from >= 0 && from != 0x7fffffff) {
+            v = __ldg(reinterpret_cast<const uint4*>(snap + (size_t)from * N) + c8);
+        } else if (from < 0) {
+            const int s = -1 - from;
+            const float4* p = reinterpret_cast<const float4*>(toks + (size_t)s * N + c8 * 8);
+            const float4 p0 = __ldg(p), p1 = __ldg(p + 1);
+            const float st[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
+            float o[8];
 #pragma unroll
-                for (int e = 0; e < 8; ++e) o[e] = (st[e] + 1.0f) * STATE_F16_SCALE * exp2f(-(float)s * rho_sh[c8 * 8 + e]);
-                v = make_uint4(pack_f16x2_sat(o[0], o[1]), pack_f16x2_sat(o[2], o[3]), pack_f16x2_sat(o[4], o[5]), pack_f16x2_sat(o[6], o[7]));
-            }
+            for (int e = 0; e < 8; ++e) o[e] = (st[e] + 1.0f) * STATE_F16_SCALE * exp2f(-(float)s * rho_sh[c8 * 8 + e]);
+            v = make_uint4(pack_f16x2_sat(o[0], o[1]), pack_f16x2_sat(o[2], o[3]), pack_f16x2_sat(o[4], o[5]), pack_f16x2_sat(o[6], o[7]));
         }
-        *reinterpret_cast<uint4*>(img + (size_t)(item / IBLK) * NK * ATOM + (c8 >> 3) * ATOM + sw_chunk(r, c8 & 7)) = v;
+        *reinterpret_cast<uint4*>(img + (c8 >> 3) * ATOM + sw_chunk(r, c8 & 7)) = v;
         const uint32_t u[4] = {v.x, v.y, v.z, v.w};
         float q = 0.f;
 #pragma unroll
@@ -180,16 +250,62 @@ __global__ void __launch_bounds__(IT_THREADS) k_items(FlashArgs a, Ws w) {
             q = fmaf(x, x, fmaf(y, y, q));
         }
         for (int o = CH / 2; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
-        q *= STATE_F16_UNSCALE * STATE_F16_UNSCALE;
-        if (c8 == 0 && !(q <= look)) {
-            const int at = atomicAdd(&n_chk, 1);
-            if (at < MAX_CHECKED) chk[at] = item;
-            else atomicMax(&swing_sh, __float_as_uint(q * trace));       // list full: the bound itself
-        }
+        if (c8 == 0) it.q[i0 + r] = q;
+    }
+    const int row = tid & (TM - 1), half = tid >> 7;
+    unsigned m0 = 0u, m1 = 0u;
+#pragma unroll 8
+    for (int i = 0; i < 32; ++i) {
+        const int p = lohi_sh[half * 64 + i], q = lohi_sh[half * 64 + 32 + i];
+        m0 |= (row >= (p & 255) && row <= (p >> 8)) ? (1u << i) : 0u;
+        m1 |= (row >= (q & 255) && row <= (q >> 8)) ? (1u << i) : 0u;
+    }
+    reinterpret_cast<uint2*>(it.mask + i0 + row)[half] = make_uint2(m0, m1);
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// one CTA per (tile, sample): the levels.  |lambda . state|^2 tr(G) bounds v' G v; items whose bound could matter are
+// looked at closely, the others are not.
+// ---------------------------------------------------------------------------------------------------------------
+static constexpr int MAX_CHECKED = 1024;
+
+__global__ void __launch_bounds__(256) k_levels(FlashArgs a, Items it, Ws w) {
+    __shared__ int chk[MAX_CHECKED], n_chk;
+    __shared__ unsigned swing_sh[2], decay_sh;          // [0] items before the hot ones, [1] hot items
+    __shared__ float lam_sh[128], trace_sh;
+    const int bt = blockIdx.y * a.nT + blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int N = a.N, NK = N >> 6;
+    const int4 cnt = it.count[bt];
+    if (cnt.w == 0) {
+        if (tid == 0) w.level[bt] = w.level_bwd[bt] = 0;
+        return;
+    }
+    if (tid == 0) { n_chk = 0; swing_sh[0] = swing_sh[1] = decay_sh = 0u; }
+    __syncthreads();
+    if (tid < N) {
+        const float lam = fabsf(logf(a.rhos[tid]));               // rho = 0: infinite, every step
+        lam_sh[tid] = lam;
+        atomicMax(&decay_sh, __float_as_uint(lam == lam ? lam : INFINITY));
+    }
+    if (warp == 0) {
+        float t = 0.f;
+        for (int n = lane; n < N; n += 32) t += w.gram[n * N + n];
+        t = warp_sum(t);
+        if (lane == 0) trace_sh = t;
     }
     __syncthreads();
-    // v' G v of the listed items: a warp each, a lane per channel
-    for (int j = warp; j < min(n_chk, MAX_CHECKED); j += IT_THREADS / 32) {
+    const float trace = trace_sh;
+    const float look = (MAX_SWING / 64.0f) * (MAX_SWING / 64.0f) / fmaxf(trace, 1e-30f);
+    const float* q = it.q + (size_t)bt * it.IB * IBLK;
+    for (int i = tid; i < cnt.w * IBLK; i += 256)
+        if (!(q[i] <= look)) {
+            const int at = atomicAdd(&n_chk, 1);
+            if (at < MAX_CHECKED) chk[at] = i;
+            else atomicMax(&swing_sh[i >= cnt.y * IBLK], __float_as_uint(q[i] * trace));       // list full: the bound itself
+        }
+    __syncthreads();
+    const unsigned char* img = it.a_img + (size_t)bt * it.IB * NK * ATOM;
+    for (int j = warp; j < min(n_chk, MAX_CHECKED); j += 8) {      // a warp per item, a lane per channel
         const int item = chk[j], r = item & (IBLK - 1);
         float vl[4], y[4];
 #pragma unroll
@@ -211,54 +327,34 @@ __global__ void __launch_bounds__(IT_THREADS) k_items(FlashArgs a, Ws w) {
                     if (32 * e < N) y[e] = fmaf(vm, __ldg(g + lane + 32 * e), y[e]);
             }
         }
-        const float q = warp_sum(vl[0] * y[0] + vl[1] * y[1] + vl[2] * y[2] + vl[3] * y[3]);
-        if (lane == 0) atomicMax(&swing_sh, __float_as_uint(q >= 0.f ? q : (q < 0.f ? 0.f : INFINITY)));
-    }
-    // what the kernels read of an item: its row of the E tables and its steps
-    __syncthreads();
-    for (int i = tid; i < n_blk * IBLK; i += IT_THREADS) {
-        int2 o = make_int2(0, 1);                          // padding: first step after the last
-        if (i < n_items) {
-            const int2 mt = meta[i];
-            const int k = mt.x >= 0 ? mt.x : slot_of[head[-1 - mt.x]];
-            o = make_int2(a.erow ? a.erow[(size_t)b * a.K + k] : b * a.K + k, mt.y);
-        } else if (a.erow == nullptr) {
-            o.x = b * a.K;
-        }
-        meta[i] = o;
+        const float v = warp_sum(vl[0] * y[0] + vl[1] * y[1] + vl[2] * y[2] + vl[3] * y[3]);
+        if (lane == 0) atomicMax(&swing_sh[item >= cnt.y * IBLK], __float_as_uint(v >= 0.f ? v : (v < 0.f ? 0.f : INFINITY)));
     }
     __syncthreads();
-    uint4* mask = w.mask + (size_t)bt * w.IB * IBLK;
-    for (int blk = 0; blk < n_blk; ++blk) {
-        if (tid < IBLK) lohi_sh[tid] = meta[blk * IBLK + tid].y;
-        __syncthreads();
-        const int row = tid & (TM - 1), half = tid >> 7;
-        unsigned m0 = 0u, m1 = 0u;
-#pragma unroll 8
-        for (int i = 0; i < 32; ++i) {
-            const int p = lohi_sh[half * 64 + i], q = lohi_sh[half * 64 + 32 + i];
-            m0 |= (row >= (p & 255) && row <= (p >> 8)) ? (1u << i) : 0u;
-            m1 |= (row >= (q & 255) && row <= (q >> 8)) ? (1u << i) : 0u;
-        }
-        reinterpret_cast<uint2*>(mask + blk * IBLK + row)[half] = make_uint2(m0, m1);
-        __syncthreads();
-    }
     if (tid == 0) {
-        w.n_items[bt] = n_items;
-        const float swing = 64.0f * sqrtf(__uint_as_float(swing_sh)), decay = 64.0f * __uint_as_float(decay_sh);
-        auto pick = [&](float max_decay) {
+        const float decay = 64.0f * __uint_as_float(decay_sh);
+        auto pick = [&](float max_decay, float q2) {
+            const float swing = 64.0f * sqrtf(q2);
             int level = 0;
             while (level < LEVEL_EXACT && !(decay <= max_decay * (float)(1 << level) && swing <= MAX_SWING * (float)(1 << level))) ++level;
-            return exact_sh ? LEVEL_EXACT : level;
+            return cnt.x < 0 ? LEVEL_EXACT : level;
         };
-        w.level[bt] = pick(MAX_DECAY);
-        w.level_bwd[bt] = pick(MAX_DECAY_BWD);
+        const float cold = __uint_as_float(swing_sh[0]), hot = __uint_as_float(swing_sh[1]);
+        w.level[bt] = pick(MAX_DECAY, fmaxf(cold, hot));
+        w.level_bwd[bt] = pick(MAX_DECAY_BWD, cold);
     }
 }
 
-int prepare(const FlashArgs& a, const Ws& w, cudaStream_t st) {
+int build_items(const FlashArgs& a, const Items& it, cudaStream_t st) {
+    const size_t smem = (size_t)a.K * sizeof(float);
+    k_items_list<<<dim3(a.nT, a.B), IL_THREADS, smem, st>>>(a, it);
+    k_items_fill<<<dim3(it.IB, a.nT, a.B), 256, 0, st>>>(a, it);
+    return check_launch();
+}
+
+int prepare(const FlashArgs& a, const Items& it, const Ws& w, cudaStream_t st) {
     k_weights<<<SEG_IMAGES * a.H * NCH + a.N, 256, 0, st>>>(a, w);
-    k_items<<<dim3(a.nT, a.B), IT_THREADS, 0, st>>>(a, w);
+    k_levels<<<dim3(a.nT, a.B), 256, 0, st>>>(a, it, w);
     return check_launch();
 }
 

@@ -292,6 +292,7 @@ class TileStates:
     seq_lens: Optional[torch.Tensor]    # [B] i32 or None
     unique: torch.Tensor                # [B, K] i64, the slot list the snapshots were built for
     shape: tuple                        # (B, T, K, N)
+    flags: int = 0                      # FLAG_TILE_ITEMS: the buffer also holds the items of the tensor-core kernels
 
 
 @_on_tensor_device
@@ -320,7 +321,10 @@ def precompute_boundaries(x, unique_tensor, rhos, Br, c_init=None, doc_ids=None,
             raise _lib.MbemaError("c_init must be [B, K, N] matching unique_tensor [B, K]")
     nT = (L + _lib.TILE_T - 1) // _lib.TILE_T
     n_el = B * nT * K * N
-    tile_buf = torch.empty(n_el * 6 + 16, dtype=torch.uint8, device=x.device)   # fp32 block, then the 16-bit copy
+    # fp32 block, its 16-bit copy and (unless the mode rules the tensor-core kernels out) their items
+    items = lib.mbema_tile_items_bytes(B, L, N, K) if _OPTIONS["mode"] != "fp32" else 0
+    tile_buf = torch.empty(max(n_el * 6 + 16, items) + 1024, dtype=torch.uint8, device=x.device)
+    tile_buf = tile_buf[-tile_buf.data_ptr() % 1024:]
     tile_state = tile_buf[: n_el * 4].view(torch.float32).view(B, nT, K, N)
     tok_state = torch.empty(B, L, N, dtype=torch.float32, device=x.device)
     kcount = torch.empty(2 * B, dtype=torch.int32, device=x.device)   # counts, then samples by decreasing count
@@ -338,7 +342,11 @@ def precompute_boundaries(x, unique_tensor, rhos, Br, c_init=None, doc_ids=None,
     _lib.check(rc, "mbema_tile_states")
     if seq_lens is not None:
         seq_lens = seq_lens.to(torch.int32).contiguous()
-    return TileStates(tile_state, tok_state, kcount, seq_lens, unique, (B, L, K, N))
+    if items:
+        rc = lib.mbema_tile_items(_ptr(x), _ptr(unique), _ptr(rhos), _ptr(tile_state), _ptr(tok_state), _ptr(kcount),
+                                  _ptr(seq_lens), B, L, N, K, _stream())
+        _lib.check(rc, "mbema_tile_items")
+    return TileStates(tile_state, tok_state, kcount, seq_lens, unique, (B, L, K, N), _lib.FLAG_TILE_ITEMS if items else 0)
 
 
 def _build_unique_index(x, device=None):
@@ -423,8 +431,8 @@ class FlashEMAFunction(torch.autograd.Function):
         O = torch.empty(B, H, L, hd, dtype=torch.float32, device=Q.device)
         LSE = torch.empty(B, H, L, dtype=torch.float32, device=Q.device)
         mode = _flash_mode(H, N, K)
-        flags = _flash_flags(use_silu)
-        need = lib.mbema_flash_fwd_workspace_bytes(B, H, L, hd, N, K, mode)
+        flags = _flash_flags(use_silu) | C_bounds.flags
+        need = lib.mbema_flash_fwd_workspace_bytes(B, H, L, hd, N, K, mode | (flags & _lib.FLAG_TILE_ITEMS))
         ws = _tc_workspace(need, Q.device) if mode == _lib.MODE_TC_BF16 else _workspace(need, Q.device)
         _ev = telemetry.begin("mbema_flash_fwd")
         rc = lib.mbema_flash_fwd(_ptr(Qc), _dt(Qc), _ptr(xx), _ptr(Ek), _ptr(Ev), _dt(Ek), _ptr(W), _ptr(rh),
@@ -454,7 +462,7 @@ class FlashEMAFunction(torch.autograd.Function):
         dEk = torch.empty(B, K, D, dtype=torch.float32, device=dO.device)
         dEv = torch.empty(B, K, D, dtype=torch.float32, device=dO.device)
         dW = torch.empty(N, D, dtype=torch.float32, device=dO.device)
-        need = lib.mbema_flash_bwd_workspace_bytes(B, H, L, hd, N, K, mode)
+        need = lib.mbema_flash_bwd_workspace_bytes(B, H, L, hd, N, K, mode | (flags & _lib.FLAG_TILE_ITEMS))
         ws = _tc_workspace(need, dO.device) if mode == _lib.MODE_TC_BF16 else _workspace(need, dO.device)
         _ev = telemetry.begin("mbema_flash_bwd")
         rc = lib.mbema_flash_bwd(_ptr(Qc), _dt(Qc), _ptr(xx), _ptr(Ek), _ptr(Ev), _dt(Ek), _ptr(W), _ptr(rh),
@@ -600,13 +608,13 @@ class FlashEMARowsFunction(torch.autograd.Function):
         O = torch.empty(B, H, L, hd, dtype=torch.float32, device=Q.device)
         LSE = torch.empty(B, H, L, dtype=torch.float32, device=Q.device)
         mode = _flash_mode(H, N, K)
-        flags = _flash_flags(use_silu)
+        flags = _flash_flags(use_silu) | C_bounds.flags
         if mode == _lib.MODE_TC_BF16 and any(ctx.needs_input_grad):
             # Layer-normalised, projected rows give peaked softmaxes, whose gradients are ill-conditioned in 16-bit operands:
             # two correct kernels differ there by more than results may move (dW_pe by tens of per cent), so training over
             # shared rows keeps the kernels that evaluate every step
             flags |= _lib.FLAG_EVERY_STEP
-        need = lib.mbema_flash_fwd_workspace_bytes(B, H, L, hd, N, K, mode)
+        need = lib.mbema_flash_fwd_workspace_bytes(B, H, L, hd, N, K, mode | (flags & _lib.FLAG_TILE_ITEMS))
         ws = _tc_workspace(need, Q.device) if mode == _lib.MODE_TC_BF16 else _workspace(need, Q.device)
         _ev = telemetry.begin("mbema_flash_fwd")
         rc = lib.mbema_flash_fwd_rows(_ptr(Qc), _dt(Qc), _ptr(xx), _ptr(Ek), _ptr(Ev), _dt(Ek), _ptr(ri), U, _ptr(W),
@@ -635,7 +643,7 @@ class FlashEMARowsFunction(torch.autograd.Function):
         dEk = torch.empty(U, D, dtype=torch.float32, device=dO.device)
         dEv = torch.empty(U, D, dtype=torch.float32, device=dO.device)
         dW = torch.empty(N, D, dtype=torch.float32, device=dO.device)
-        need = lib.mbema_flash_bwd_workspace_bytes(B, H, L, hd, N, K, mode)
+        need = lib.mbema_flash_bwd_workspace_bytes(B, H, L, hd, N, K, mode | (flags & _lib.FLAG_TILE_ITEMS))
         ws = _tc_workspace(need, dO.device) if mode == _lib.MODE_TC_BF16 else _workspace(need, dO.device)
         _ev = telemetry.begin("mbema_flash_bwd")
         rc = lib.mbema_flash_bwd_rows(_ptr(Qc), _dt(Qc), _ptr(xx), _ptr(Ek), _ptr(Ev), _dt(Ek), _ptr(ri), U, _ptr(W),
