@@ -59,9 +59,9 @@ extern "C" {
                                        /* x, B and T: the sort is skipped, only the links to the listed keys are      */
                                        /* rebuilt (the model calls the scan and the snapshots on the same chunk,      */
                                        /* mathbrain/model.py:157 and :180)                                            */
-#define MBEMA_FLAG_EVERY_STEP 32       /* MBEMA_MODE_TC_BF16 only: evaluate the gate at every step.  Otherwise the    */
-                                       /* kernels evaluate it at four nodes per 128-step tile (or part of it) wherever  */
-                                       /* the states decay slowly enough, and at every step where they do not           */
+#define MBEMA_FLAG_HOT_EVERY_STEP 32   /* MBEMA_MODE_TC_BF16 forward: evaluate the gate of a tile's sixteen largest     */
+                                       /* slots at every step, as the backward always does; otherwise all gates are     */
+                                       /* evaluated at four nodes per tile (or part of it) where states decay slowly   */
 #define MBEMA_FLAG_TILE_ITEMS 64       /* attention calls: mbema_tile_items has run on this tile_state buffer          */
 /* Test hook of the tensor-core forward and backward: one hand-off between the kernel's warps is withheld and the bounded
  * waits give up after a few polls, so the kernel must end through its give-up path (status word set, products in flight

@@ -25,8 +25,9 @@ struct FlashArgs {
     float v_total;
     int silu, listed_only;
     const int* level;       // [B, nT] or null: the every-step tensor-core kernels work on the tiles marked smooth::LEVEL_EXACT only
-    const int* hot;         // with level: [B, nT][smooth::HOT + 1] hot slots of every other tile, which the backward adds to what the
-                            // smooth-state kernel left there
+    const int* hot;         // with level: [B, nT][smooth::HOT + 1] hot slots, which the every-step kernels take on the other tiles too
+                            // (the backward adds to what the smooth-state kernel left; the forward comes first and is merged
+                            // there; null in the forward: the smooth-state kernel has all slots)
     int test_withhold;      // test hook: see MBEMA_FLAG_TEST_WITHHOLD_ARRIVE
 };
 
@@ -44,7 +45,6 @@ bool flash_tc_supported(int H, int N, int K);
 int flash_fwd_tc(const FlashArgs& a, void* ws, cudaStream_t st);
 bool flash_bwd_tc_supported(int H, int N, int K);
 size_t flash_bwd_tc_ws(int64_t B, int64_t H, int64_t T, int64_t N);
-// it, w: the smooth-state kernels take what they can (null: every step everywhere)
-int flash_bwd_tc(FlashArgs a, const smooth::Items* it, const smooth::Ws* w, float* dW, void* ws, cudaStream_t st);
+int flash_bwd_tc(FlashArgs a, const smooth::Items& it, const smooth::Ws& w, float* dW, void* ws, cudaStream_t st);
 
 }  // namespace mbema

@@ -105,14 +105,18 @@ static int flash_fwd_impl(const void* Q, int q_dtype, const int64_t* x, const vo
         if (!workspace) return MBEMA_ERR_NULL;
         if (workspace_bytes < mbema_flash_fwd_workspace_bytes(B, H, T, hd, N, K, mode | (flags & MBEMA_FLAG_TILE_ITEMS))) return MBEMA_ERR_WORKSPACE;
         cudaStream_t st = (cudaStream_t)stream;
-        if (flags & MBEMA_FLAG_EVERY_STEP) return flash_fwd_tc(a, workspace, st);
         int* status = reinterpret_cast<int*>((reinterpret_cast<uintptr_t>(workspace) + 15) & ~uintptr_t(15));
         unsigned char* p = static_cast<unsigned char*>(workspace) + STATUS_BYTES;
         const smooth::Ws w = smooth::carve(p, B, H, T, N);
         smooth::Items it;
-        if ((rc = items_of(a, flags, p + smooth::ws_bytes(B, H, T, N, false), it, st)) || (rc = smooth::prepare(a, it, w, st)) ||
-            (rc = smooth::forward(a, it, w, status, st)))
-            return rc;
+        if ((rc = items_of(a, flags, p + smooth::ws_bytes(B, H, T, N, false), it, st)) || (rc = smooth::prepare(a, it, w, st))) return rc;
+        if (flags & MBEMA_FLAG_HOT_EVERY_STEP) {
+            a.level = w.level;
+            a.hot = it.hot;
+            if ((rc = flash_fwd_tc(a, workspace, st))) return rc;
+            return smooth::forward(a, it, w, status, st);
+        }
+        if ((rc = smooth::forward(a, it, w, status, st))) return rc;
         a.level = w.level;
         return flash_fwd_tc(a, workspace, st);
     }
@@ -188,12 +192,11 @@ static int flash_bwd_impl(const void* Q, int q_dtype, const int64_t* x, const vo
     // tensor-core backward where the shape fits its shared-memory budget (N == 64); otherwise the fp32 kernels
     if (mode == MBEMA_MODE_TC_BF16) {
         if (!(flags & MBEMA_FLAG_FP32_BACKWARD) && flash_bwd_tc_supported((int)H, (int)N, (int)K)) {
-            if (flags & MBEMA_FLAG_EVERY_STEP) return flash_bwd_tc(a, nullptr, nullptr, dW_pe, workspace, st);
             unsigned char* p = static_cast<unsigned char*>(workspace) + flash_bwd_tc_ws(B, H, T, N);
             const smooth::Ws w = smooth::carve(p, B, H, T, N);
             smooth::Items it;
             if ((rc = items_of(a, flags, p + smooth::ws_bytes(B, H, T, N, true), it, st))) return rc;
-            return flash_bwd_tc(a, &it, &w, dW_pe, workspace, st);
+            return flash_bwd_tc(a, it, w, dW_pe, workspace, st);
         }
         // (the first 512 bytes stay reserved for the status word of the tensor-core kernels; the fp32 kernels have no
         // bounded waits and leave it alone)

@@ -123,7 +123,10 @@ __global__ void __launch_bounds__(THREADS, 1) k_flash_fwd_tc(FlashArgs a, int* s
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int D = a.H * HD;
     const int t0 = tile * TM;
-    if (a.level && a.level[b * a.nT + tile] != smooth::LEVEL_EXACT) return;      // done by the smooth-state kernel
+    // the whole tile; or its hot slots alone, whose result the smooth-state kernel merges with the rest; or nothing
+    const bool part = a.level[b * a.nT + tile] != smooth::LEVEL_EXACT;
+    if (part && !a.hot) return;
+    const int* hot = part ? a.hot + (b * a.nT + tile) * (smooth::HOT + 1) : nullptr;
     const int Lb = a.seq_lens ? min(max(a.seq_lens[b], 0), a.T) : a.T;
     const bool is_epi = warp < EPI_WARPS;
     const int row = (warp & 3) * 32 + lane;         // time step within the tile (== TMEM lane for epilogue warps)
@@ -158,7 +161,14 @@ __global__ void __launch_bounds__(THREADS, 1) k_flash_fwd_tc(FlashArgs a, int* s
     }
     if (warp == EPI_WARPS + 1) {   // ordered compaction of the valid slots (index and key)
         int n = 0;
-        for (int k0 = 0; k0 < a.K; k0 += 32) {
+        if (part) {
+            n = hot[0];
+            if (lane < n) {
+                slot_sh[lane] = (unsigned short)hot[1 + lane];
+                key_sh[lane] = (int)(a.unique[(size_t)b * a.K + hot[1 + lane]] & 0x7fffffffLL);
+            }
+        }
+        for (int k0 = 0; k0 < a.K && !part; k0 += 32) {
             const int k = k0 + lane;
             const long long kv = (k < a.K) ? a.unique[(size_t)b * a.K + k] : -1;
             const bool ok = kv >= 0;
@@ -383,7 +393,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_flash_fwd_tc(FlashArgs a, int* s
         }
         const float rest = a.v_total - (float)a.kcount[b];
         float m, l;
-        if (!a.listed_only && rest > 0.f) { m = 0.f; l = rest; } else { m = -INFINITY; l = 0.f; }
+        if (!part && !a.listed_only && rest > 0.f) { m = 0.f; l = rest; } else { m = -INFINITY; l = 0.f; }
         const uint32_t t_lane = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(wg * HD);
         // In iteration i a thread
         //   (1) starts the TMEM load of slot i's accumulators,
@@ -481,7 +491,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_flash_fwd_tc(FlashArgs a, int* s
 #pragma unroll
             for (int i = 0; i < HD; i += 4)
                 *reinterpret_cast<float4*>(a.O + qoff + i) = make_float4(o[i] * inv, o[i + 1] * inv, o[i + 2] * inv, o[i + 3] * inv);
-            a.LSE[((size_t)b * a.H + h) * a.T + t] = (row_ok && l > 0.f) ? m + logf(l) : 0.f;
+            a.LSE[((size_t)b * a.H + h) * a.T + t] = (row_ok && l > 0.f) ? m + logf(l) : (part ? -INFINITY : 0.f);
         }
     }
     // ---------------------------------------------------------------- teardown

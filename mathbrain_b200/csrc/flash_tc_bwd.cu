@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_flash_bwd_tc(FlashArgs a, int* s
     const int D = a.H * HD;
     const int t0 = tile * TM;
     // the whole tile, or (the rest being done by the smooth-state kernel) its hot slots, added to what stands there
-    const bool add = a.level && a.level[b * a.nT + tile] != smooth::LEVEL_EXACT;
+    const bool add = a.level[b * a.nT + tile] != smooth::LEVEL_EXACT;
     const int* hot = add ? a.hot + (b * a.nT + tile) * (smooth::HOT + 1) : nullptr;
     if (add && hot[0] == 0) return;
     const int Lb = a.seq_lens ? min(max(a.seq_lens[b], 0), a.T) : a.T;
@@ -747,18 +747,17 @@ size_t flash_bwd_tc_ws(int64_t B, int64_t H, int64_t T, int64_t N) {
     return 256 + (size_t)(B * (H / tcb::HPC) * nT) * N * tcb::ACC_COLS * sizeof(float) + 256;
 }
 
-int flash_bwd_tc(FlashArgs a, const smooth::Items* it, const smooth::Ws* w, float* dW, void* ws, cudaStream_t st) {
+int flash_bwd_tc(FlashArgs a, const smooth::Items& it, const smooth::Ws& w, float* dW, void* ws, cudaStream_t st) {
     const int D = a.H * tcb::HD;
     int* status = reinterpret_cast<int*>((reinterpret_cast<uintptr_t>(ws) + 255) & ~uintptr_t(255));
     a.dW_part = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(status) + 256);
     MBEMA_CUDA_TRY(cudaMemsetAsync(a.dEk, 0, (size_t)a.e_rows * D * sizeof(float), st));
     MBEMA_CUDA_TRY(cudaMemsetAsync(a.dEv, 0, (size_t)a.e_rows * D * sizeof(float), st));
-    if (it) {
-        int rc;
-        if ((rc = smooth::prepare(a, *it, *w, st)) || (rc = smooth::backward(a, *it, *w, status, st))) return rc;
-        a.level = w->level_bwd;
-        a.hot = it->hot;
-    }
+    // every tile and slot but the hot ones over smooth states, then the hot slots and the tiles that need every step
+    int rc;
+    if ((rc = smooth::prepare(a, it, w, st)) || (rc = smooth::backward(a, it, w, status, st))) return rc;
+    a.level = w.level_bwd;
+    a.hot = it.hot;
     const tcb::Smem L = tcb::smem_layout(a.K, a.N / 64);
     dim3 grid(a.nT, a.H / tcb::HPC, a.B);
 #define MBEMA_LAUNCH_BWD(S_, NK_, R_)                                                                                     \
@@ -775,7 +774,7 @@ int flash_bwd_tc(FlashArgs a, const smooth::Items* it, const smooth::Ws* w, floa
     if (rows) MBEMA_PICK(true); else MBEMA_PICK(false);
 #undef MBEMA_PICK
 #undef MBEMA_LAUNCH_BWD
-    int rc = check_launch();
+    rc = check_launch();
     if (rc) return rc;
     const int total = a.N * D;
     tcb::k_flash_dw_reduce_tc<<<(total + 255) / 256, 256, 0, st>>>(a.dW_part, dW, a.B, a.H / tcb::HPC, a.nT, D, a.N);

@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_fwd(FlashArgs a, Items it
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem = bars->tmem_base;
-    const int n_blk = it.count[bt].w;
+    const int n_blk = a.hot ? it.count[bt].y : it.count[bt].w;        // the hot slots' blocks are the last ones
     const int n_it = bars->abort_flag ? 0 : n_blk << level;        // blocks of segment 0, then of segment 1, ...
     const unsigned* lim = &bars->spin_limit;
 
@@ -250,12 +250,17 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_fwd(FlashArgs a, Items it
             tc_fence_after_sync();
             float* mx = mx_sh + (n_it & 1) * 2 * TM;
             mx[half * TM + row] = l;
+            // the hot slots' share, from the every-step kernel
+            const bool merge = a.hot && a.hot[bt * (HOT + 1)] > 0 && t0 + row < Lb;
+            const float mh = merge ? a.LSE[row0 + row] * 1.4426950409f : -INFINITY;
             __syncwarp();
             if (lane == 0) mbar_arrive(&bars->mx_full);
             alive = warp_wait(&bars->mx_full, (uint32_t)(n_it & 1), abort_flag, 7, lim);
             l += mx[(half ^ 1) * TM + row];
+            const float mm = fmaxf(m, mh), wc = m == -INFINITY ? 0.f : exp2f(m - mm), wh = merge ? exp2f(mh - mm) : 0.f;
+            l = fmaf(l, wc, wh);
             const bool ok = t0 + row < Lb && l > 0.f;
-            const float inv = ok ? 1.0f / l : 0.f;
+            const float inv = ok ? wc / l : 0.f, inv_h = ok ? wh / l : 0.f;
             float beta[NJ];
             basis(row, level, beta);
 #pragma unroll 1
@@ -273,16 +278,18 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_fwd(FlashArgs a, Items it
 #pragma unroll
                     for (int d = 0; d < 16; d += 4) {
                         float v[4];
+                        float4* out = reinterpret_cast<float4*>(a.O + (row0 + row) * HD + c * 16 + d);
+                        const float4 oh = merge ? *out : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
                         for (int e = 0; e < 4; ++e) {
                             const int k = d + e;
                             v[e] = ok ? inv * fmaf(beta[3], o[48 + k], fmaf(beta[2], o[32 + k], fmaf(beta[1], o[16 + k], o[k]))) : 0.f;
                         }
-                        *reinterpret_cast<float4*>(a.O + (row0 + row) * HD + c * 16 + d) = make_float4(v[0], v[1], v[2], v[3]);
+                        *out = make_float4(fmaf(inv_h, oh.x, v[0]), fmaf(inv_h, oh.y, v[1]), fmaf(inv_h, oh.z, v[2]), fmaf(inv_h, oh.w, v[3]));
                     }
                 }
             }
-            if (alive && half == 0 && t0 + row < a.T) a.LSE[row0 + row] = ok ? m * 0.6931471806f + logf(l) : 0.f;
+            if (alive && half == 0 && t0 + row < a.T) a.LSE[row0 + row] = ok ? mm * 0.6931471806f + logf(l) : 0.f;
         }
     } else {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");

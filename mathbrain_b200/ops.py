@@ -610,10 +610,9 @@ class FlashEMARowsFunction(torch.autograd.Function):
         mode = _flash_mode(H, N, K)
         flags = _flash_flags(use_silu) | C_bounds.flags
         if mode == _lib.MODE_TC_BF16 and any(ctx.needs_input_grad):
-            # Layer-normalised, projected rows give peaked softmaxes, whose gradients are ill-conditioned in 16-bit operands:
-            # two correct kernels differ there by more than results may move (dW_pe by tens of per cent), so training over
-            # shared rows keeps the kernels that evaluate every step
-            flags |= _lib.FLAG_EVERY_STEP
+            # layer-normalised, projected rows give peaked softmaxes, whose gradients are ill-conditioned in 16-bit operands:
+            # the slots that carry them get the same arithmetic in both directions
+            flags |= _lib.FLAG_HOT_EVERY_STEP
         need = lib.mbema_flash_fwd_workspace_bytes(B, H, L, hd, N, K, mode | (flags & _lib.FLAG_TILE_ITEMS))
         ws = _tc_workspace(need, Q.device) if mode == _lib.MODE_TC_BF16 else _workspace(need, Q.device)
         _ev = telemetry.begin("mbema_flash_fwd")
