@@ -268,6 +268,26 @@ int mbema_slot_state_gather(const float* state, const int32_t* last_t, const int
                             const float* rhos, float* c_base, int64_t B, int64_t K, int64_t V, int64_t N, void* stream);
 
 /* ------------------------------------------------------------------------------------------------
+ * Feeding chunks of documents whose slot state is resident (state [B,V,N] f32 after the last update, last_t [B,V] i32 step of
+ * that update or -1, seen [B,cap] i64 tokens in the order they joined, n_seen [B] i64, t0 [B] i32 step of the next chunk):
+ * the wire format that mathbrain/data.py:95-148 and :211-235 build in Python.  x [B,T] i64, fill [B] i32 valid lengths.
+ *   mbema_feed_lists    lists [B,T+cap] i32: the chunk's distinct tokens in order, then the other seen ones in order;
+ *                       counts [B+1] i32: list lengths, and the longest
+ *   mbema_feed_batch    unique [B,K] i64 (0 behind the list), pad_mask [B,K] u8, c_base [B,K,N] f32
+ *   mbema_feed_advance  moves the documents past the chunk (C_seq [B,T,N] from mbema_query_scan on it).  check = 1: changes
+ *                       nothing and raises status[0] (i32) to the longest seen list that would result; tokens beyond `cap`
+ *                       entries are not recorded
+ * ---------------------------------------------------------------------------------------------- */
+int mbema_feed_lists(const int64_t* x, const int32_t* fill, const int64_t* seen, const int64_t* n_seen, int32_t* lists,
+                     int32_t* counts, int64_t B, int64_t T, int64_t V, int64_t cap, void* stream);
+int mbema_feed_batch(const int32_t* lists, const int32_t* counts, const float* state, const int32_t* last_t, const int32_t* t0,
+                     const float* rhos, int64_t* unique, uint8_t* pad_mask, float* c_base, int64_t B, int64_t K, int64_t T,
+                     int64_t V, int64_t N, int64_t cap, void* stream);
+int mbema_feed_advance(const int64_t* x, const int32_t* fill, const float* C_seq, float* state, int32_t* last_t, int64_t* seen,
+                       int64_t* n_seen, int32_t* t0, int32_t* status, int64_t B, int64_t T, int64_t V, int64_t N, int64_t cap,
+                       int check, void* stream);
+
+/* ------------------------------------------------------------------------------------------------
  * Softmax cross-entropy over a chunk of logits rows, forward and backward in one launch, IN PLACE:
  *   loss_rows[r] = logsumexp(logits[r, 0:V]) - logits[r, targets[r]]
  *   logits[r, c] <- (softmax(logits[r, 0:V])[c] - [c == targets[r]]) * scale     (columns [V, ld) <- 0)

@@ -55,6 +55,9 @@ SIGNATURES = {
     "mbema_slot_ln_fwd": (_i32, [_vp, _i32, _vp, _vp, _vp, _f32, _vp, _i32, _vp, _vp, _i64, _i64, _i64, _vp]),
     "mbema_slot_ln_bwd": (_i32, [_vp, _i32, _vp, _i32, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _vp]),
     "mbema_slot_state_gather": (_i32, [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _i64, _i64, _vp]),
+    "mbema_feed_lists": (_i32, [_vp] * 6 + [_i64] * 4 + [_vp]),
+    "mbema_feed_batch": (_i32, [_vp] * 9 + [_i64] * 6 + [_vp]),
+    "mbema_feed_advance": (_i32, [_vp] * 9 + [_i64] * 5 + [_i32, _vp]),
     "mbema_ce_rows": (_i32, [_vp, _i32, _vp, _f32, _vp, _i64, _i64, _i64, _vp]),
     "mbema_slot_grad_scatter": (_i32, [_vp, _vp, _i32, _vp, _vp, _i64, _i64, _i64, _vp]),
 }
