@@ -36,8 +36,10 @@ __device__ __forceinline__ size_t e_row(const FlashArgs& a, int b, int k) {
     return a.erow ? (size_t)a.erow[(size_t)b * a.K + k] : (size_t)b * a.K + k;
 }
 
-int flash_fwd_simt(const FlashArgs& a, cudaStream_t st);
-size_t flash_bwd_simt_ws(int64_t B, int64_t H, int64_t T, int64_t N);
+// workspace sizes depend on B, H, T, N, K of the arguments only
+size_t flash_fwd_simt_ws(const FlashArgs& a);
+int flash_fwd_simt(const FlashArgs& a, void* ws, cudaStream_t st);
+size_t flash_bwd_simt_ws(const FlashArgs& a);
 int flash_bwd_simt(FlashArgs a, float* dW, void* ws, cudaStream_t st);
 
 // tensor-core (tcgen05) path

@@ -22,7 +22,7 @@ static FlashArgs pack(const void* Q, int q_dtype, const int64_t* x, const void* 
     a.Q = Q; a.q_dt = q_dtype; a.x = (const long long*)x; a.Ek = E_k; a.Ev = E_v; a.e_dt = e_dtype;
     a.W = W_pe; a.rhos = rhos; a.unique = (const long long*)unique; a.tile_state = tile_state;
     a.tok_state = tok_state; a.kcount = kcount; a.seq_lens = seq_lens;
-    a.order = kcount + B;
+    a.order = kcount ? kcount + B : nullptr;
     a.B = (int)B; a.H = (int)H; a.T = (int)T; a.N = (int)N; a.K = (int)K;
     a.nT = (int)((T + MBEMA_TILE_T - 1) / MBEMA_TILE_T);
     a.v_total = (float)V_total;
@@ -73,12 +73,17 @@ extern "C" int mbema_flash_tc_supported(int64_t H, int64_t N, int64_t K) {
     return flash_tc_supported((int)H, (int)N, (int)K) ? 1 : 0;
 }
 
+static FlashArgs sizes(int64_t B, int64_t H, int64_t T, int64_t N, int64_t K) {
+    return pack(nullptr, 0, nullptr, nullptr, nullptr, 0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, B, H, T, N, K, 0, 0);
+}
+
 // the first STATUS_BYTES of a tensor-core workspace hold the kernels' status word
 static constexpr size_t STATUS_BYTES = 512;
 
 extern "C" size_t mbema_flash_fwd_workspace_bytes(int64_t B, int64_t H, int64_t T, int64_t, int64_t N, int64_t K, int mode) {
-    if (mode == (MBEMA_MODE_TC_BF16 | MBEMA_FLAG_TILE_ITEMS)) return STATUS_BYTES + smooth::ws_bytes(B, H, T, N, false);
-    return mode == MBEMA_MODE_TC_BF16 ? STATUS_BYTES + smooth::ws_bytes(B, H, T, N, false) + smooth::items_bytes(B, T, N, K) : 256;
+    const bool items = !(mode & MBEMA_FLAG_TILE_ITEMS);
+    if ((mode & ~MBEMA_FLAG_TILE_ITEMS) == MBEMA_MODE_FP32) return flash_fwd_simt_ws(sizes(B, H, T, N, K));
+    return STATUS_BYTES + smooth::ws_bytes(B, H, T, N, false) + (items ? smooth::items_bytes(B, T, N, K) : 0);
 }
 
 static int flash_fwd_impl(const void* Q, int q_dtype, const int64_t* x, const void* E_k, const void* E_v,
@@ -120,7 +125,8 @@ static int flash_fwd_impl(const void* Q, int q_dtype, const int64_t* x, const vo
         a.level = w.level;
         return flash_fwd_tc(a, workspace, st);
     }
-    return flash_fwd_simt(a, (cudaStream_t)stream);
+    // a caller without the workspace gets the kernel that needs none
+    return flash_fwd_simt(a, workspace_bytes >= flash_fwd_simt_ws(a) ? workspace : nullptr, (cudaStream_t)stream);
 }
 
 extern "C" int mbema_flash_fwd(const void* Q, int q_dtype, const int64_t* x, const void* E_k, const void* E_v,
@@ -152,7 +158,7 @@ extern "C" size_t mbema_flash_bwd_workspace_bytes(int64_t B, int64_t H, int64_t 
     const bool items = !(mode & MBEMA_FLAG_TILE_ITEMS);
     mode &= ~MBEMA_FLAG_TILE_ITEMS;
     // in tensor-core mode the first 512 bytes hold the kernel status word, whichever kernel ends up running
-    size_t need = flash_bwd_simt_ws(B, H, T, N) + (mode == MBEMA_MODE_TC_BF16 ? 512 : 0);
+    size_t need = flash_bwd_simt_ws(sizes(B, H, T, N, K)) + (mode == MBEMA_MODE_TC_BF16 ? 512 : 0);
     if (mode == MBEMA_MODE_TC_BF16 && flash_bwd_tc_supported((int)H, (int)N, (int)K)) {
         const size_t tc = flash_bwd_tc_ws(B, H, T, N) + smooth::ws_bytes(B, H, T, N, true) + (items ? smooth::items_bytes(B, T, N, K) : 0);
         if (tc > need) need = tc;
