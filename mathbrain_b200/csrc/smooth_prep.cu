@@ -199,8 +199,9 @@ __global__ void __launch_bounds__(IL_THREADS) k_items_list(FlashArgs a, Items it
     put(tid < s.n_hot, 1, tid < s.n_hot ? s.hot[tid] : 0, tid < s.n_hot ? first_of(s.hot[tid]) << 8 : 0, tid < s.n_hot ? s.hot[tid] : 0, base);
     const int n_hot = put(is_hot, 1, own, occ ? (tid + 1) | (s.next[tid] << 8) : 0, -1 - tid, base);
     const int n_all = base + n_hot, n_blk = (n_all + IBLK - 1) / IBLK;
-    for (int i = n_cold + tid; i < base; i += IL_THREADS) { meta[i] = make_int2(0, 1); src[i] = 0x7fffffff; }      // padding: no valid step
-    for (int i = n_all + tid; i < n_blk * IBLK; i += IL_THREADS) { meta[i] = make_int2(0, 1); src[i] = 0x7fffffff; }
+    // padding: no valid step, state zero; it names a listed slot, since E rows of unlisted ones may hold anything
+    for (int i = n_cold + tid; i < base; i += IL_THREADS) { meta[i] = make_int2(meta[0].x, 1); src[i] = 0x7fffffff; }
+    for (int i = n_all + tid; i < n_blk * IBLK; i += IL_THREADS) { meta[i] = make_int2(s.hot[0], 1); src[i] = 0x7fffffff; }
     if (tid == 0) it.count[bt] = make_int4(s.dup ? -1 - n_cold : n_cold, base / IBLK, n_all, n_blk);
 }
 

@@ -32,8 +32,7 @@ class ChunkFeeder:
         self.seen = torch.zeros(self.B, self.cap, dtype=torch.int64, device=dev)             # tokens seen so far, per document
         self.n_seen = torch.zeros(self.B, dtype=torch.int64, device=dev)
         self.t0 = torch.zeros(self.B, dtype=torch.int32, device=dev)                         # step of the next chunk's first token
-        self._longest = 0          # no list of seen tokens is longer: below `capacity` no overflow check is due
-        self._lists = None         # workspace of next_batch: [B, T + capacity] lists and their lengths
+        self._widest = None        # widest slot list of a next_batch that no advance has followed yet
 
     def reset(self, docs):
         """Start new documents in the given rows (a tensor or list of row numbers)."""
@@ -52,19 +51,23 @@ class ChunkFeeder:
         with torch.cuda.device(self.state.device):
             return self._next_batch(x, fill)
 
+    def _chunk(self, x, fill):
+        if x.dim() != 2 or x.shape[0] != self.B:
+            raise _lib.MbemaError("ChunkFeeder: chunk of shape %s for %d documents" % (tuple(x.shape), self.B))
+        return x.long().contiguous(), fill.to(torch.int32).expand(self.B).contiguous()
+
     def _next_batch(self, x, fill):
         B, T = x.shape
         dev = x.device
         lib = _lib.load()
-        x, fill = x.long().contiguous(), fill.to(torch.int32)
-        n = B * (T + self.cap)
-        if self._lists is None or self._lists.numel() < n + B + 1:
-            self._lists = torch.empty(n + B + 1, dtype=torch.int32, device=dev)
-        lists, counts = self._lists, self._lists[n:n + B + 1]
+        x, fill = self._chunk(x, fill)
+        lists = torch.empty(B, T + self.cap, dtype=torch.int32, device=dev)
+        counts = torch.empty(B + 1, dtype=torch.int32, device=dev)
         rc = lib.mbema_feed_lists(_ptr(x), _ptr(fill), _ptr(self.seen), _ptr(self.n_seen), _ptr(lists), _ptr(counts), B, T, self.V,
                                   self.cap, _stream())
         _lib.check(rc, "mbema_feed_lists")
-        K = max(16, int(counts[B]))                                              # the one host synchronisation
+        self._widest = int(counts[B])                                            # the one host synchronisation
+        K = max(16, self._widest)
         unique = torch.empty(B, K, dtype=torch.int64, device=dev)
         pad_mask = torch.empty(B, K, dtype=torch.bool, device=dev)
         c_base = torch.empty(B, K, self.N, dtype=torch.float32, device=dev)
@@ -85,7 +88,10 @@ class ChunkFeeder:
 
     def _advance(self, x, fill, C_seq):
         B, T = x.shape
-        x, fill, C_seq = x.long().contiguous(), fill.to(torch.int32), C_seq.float().contiguous()
+        x, fill = self._chunk(x, fill)
+        C_seq = C_seq[:B, :T].float().contiguous()
+        if C_seq.shape != (B, T, self.N):
+            raise _lib.MbemaError("ChunkFeeder: C_seq must be [%d, %d, %d]" % (B, T, self.N))
 
         def call(status, check):
             rc = _lib.load().mbema_feed_advance(_ptr(x), _ptr(fill), _ptr(C_seq), _ptr(self.state), _ptr(self.last_t), _ptr(self.seen),
@@ -93,12 +99,12 @@ class ChunkFeeder:
                                                 _stream())
             _lib.check(rc, "mbema_feed_advance")
 
-        self._longest = min(self._longest + T, self.V)
-        if self._longest > self.cap:           # the bound kept here no longer rules an overflow out: ask before anything changes
+        # The lists of the next_batch before this call hold every token seen so far, so no list grows past their width plus T.
+        # Where that rules an overflow out, nothing is asked of the device (a read back costs as much as the three kernels).
+        bound, self._widest = (self.cap + 1 if self._widest is None else min(self._widest + T, self.V)), None
+        if bound > self.cap:
             status = torch.zeros(1, dtype=torch.int32, device=x.device)
             call(status, 1)
-            longest = int(status)
-            if longest > self.cap:
+            if int(status) > self.cap:
                 raise _lib.MbemaError("ChunkFeeder: the list of seen tokens is full (capacity %d)" % self.cap)
-            self._longest = longest
         call(None, 0)

@@ -69,3 +69,40 @@ def test_feeder_refuses_a_full_list():
     C_seq = mb.compute_query_ema_history(x, rhos, 50, batch["c_base"], batch["unique_slots"])
     with pytest.raises(mb._lib.MbemaError):
         feeder.advance(x, fill, C_seq)
+
+
+def test_feeder_vocabulary_of_several_segments_and_strided_lengths():
+    """More tokens than one bitmap segment holds (393216), a strided `fill`, and what is refused: chunks for another number
+    of documents, a state sequence of the wrong shape, a list filled up behind the feeder's back."""
+    import mathbrain_b200 as mb
+    from mathbrain_b200.feeder import ChunkFeeder
+    B, V, N, T = 2, 800_001, 4, 64
+    rng = np.random.Generator(np.random.PCG64(8))
+    rhos = torch.tensor([0.9, 0.99, 0.999, 0.5]).cuda()
+    feeder = ChunkFeeder(B, V, rhos, capacity=256)
+    history = [np.zeros(0, np.int64)] * B
+    edge = np.array([0, 31, 393215, 393216, 786431, 786432, V - 1])
+    for step in range(3):
+        x = rng.integers(0, V, (B, T))
+        x[:, :7] = edge
+        fill = torch.tensor([T, 99, 33, 99]).cuda()[::2]
+        xd = torch.from_numpy(x).cuda()
+        batch = feeder.next_batch(xd, fill)
+        C_seq = mb.compute_query_ema_history(xd, rhos, V, batch["c_base"], batch["unique_slots"])
+        for b, n in enumerate((T, 33)):
+            cu = np.unique(x[b, :n])
+            keys = np.concatenate([cu, np.setdiff1d(history[b], cu)])
+            assert batch["unique_slots"][b, :len(keys)].cpu().numpy().tolist() == keys.tolist()
+            assert int(batch["pad_mask"][b].sum()) == len(keys)
+            history[b] = np.concatenate([history[b], x[b, :n]])
+        with pytest.raises(mb._lib.MbemaError):
+            feeder.advance(xd[:1], fill, C_seq)
+        with pytest.raises(mb._lib.MbemaError):
+            feeder.advance(xd, fill, C_seq[..., :2])
+        feeder.advance(xd, fill, C_seq)
+        assert feeder.n_seen.cpu().tolist() == [len(np.unique(h)) for h in history]
+    before = feeder.state.clone()
+    feeder.n_seen.fill_(250)                # set by the program, as when it restores a saved state
+    with pytest.raises(mb._lib.MbemaError):
+        feeder.advance(torch.arange(B * T).view(B, T).cuda() + 1000, fill, C_seq)
+    assert torch.equal(feeder.state, before)
