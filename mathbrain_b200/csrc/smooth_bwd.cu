@@ -8,7 +8,7 @@
 // W_pe's gradient takes the node powers rho^tau_i as a0 + a1 theta_i (two products instead of four): the part left out is
 // (lambda * half tile)^2 / 4 <= 5e-4 of the fastest channel (MAX_DECAY_BWD), a rounding of the fp16 operand.
 //
-// Two gate warpgroups (a thread per item, even and odd chunks), two step warpgroups (softmax: a thread per item and half
+// Two gate warpgroups (a thread per item, half of a chunk's columns each), two step warpgroups (softmax: a thread per item and half
 // the steps; then a thread per step for dQ), a loader lane and two issuing lanes.  Registers and tensor memory hold all
 // that shared memory (224 KB: Q' 64, dO' 64, states 16, dS 32, W' 16, two operand tiles 32) has no room for; for 128
 // channels dO' is streamed through two stages from a copy in the workspace instead.
@@ -26,7 +26,7 @@ namespace bwd {
 
 static constexpr int GATE_WARPS = 8, SM_WARPS = 8;
 static constexpr int W_LOAD = 16, W_GATE = 17, W_ATT = 18;       // warp 19 only fills the warpgroup
-static constexpr int THREADS = 20 * 32;      // launched with 96 registers a thread: 61440 = 256 * 112 + 256 * 104 + 128 * 48
+static constexpr int THREADS = 20 * 32;      // launched with 96 registers a thread: 61440 = 512 * 104 + 128 * 64
 static constexpr uint32_t T_S = 0, T_DP = 128, T_DQ = 256, T_PRE = 320, T_DW = 384;
 static constexpr float LN2 = 0.6931471806f;
 
@@ -84,13 +84,13 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
         for (int i = 0; i < 2; ++i) {
             mbar_init(&bars->w_full[i], 1); mbar_init(&bars->w_free[i], 1);
             mbar_init(&bars->do_full[i], 1); mbar_init(&bars->do_free[i], 1);
-            mbar_init(&bars->pre1_full[i], 1); mbar_init(&bars->pre2_full[i], 1); mbar_init(&bars->pre_empty[i], 4);
-            mbar_init(&bars->kv_full[i], 4); mbar_init(&bars->kv_free[i], 1);
-            mbar_init(&bars->dkv_full[i], 1); mbar_init(&bars->kg_full[i], 4); mbar_init(&bars->kg_free[i], 1);
-            mbar_init(&bars->dq_full[i], 1); mbar_init(&bars->dpre_full[i], 4); mbar_init(&bars->dp_free[i], 1);
+            mbar_init(&bars->pre1_full[i], 1); mbar_init(&bars->pre2_full[i], 1); mbar_init(&bars->pre_empty[i], GATE_WARPS);
+            mbar_init(&bars->kv_full[i], GATE_WARPS); mbar_init(&bars->kv_free[i], 1);
+            mbar_init(&bars->dkv_full[i], 1); mbar_init(&bars->kg_full[i], GATE_WARPS); mbar_init(&bars->kg_free[i], 1);
+            mbar_init(&bars->dq_full[i], 1); mbar_init(&bars->dpre_full[i], GATE_WARPS); mbar_init(&bars->dp_free[i], 1);
         }
         mbar_init(&bars->sdp_full, 1); mbar_init(&bars->s_read, SM_WARPS); mbar_init(&bars->pds_full, SM_WARPS);
-        mbar_init(&bars->dkv_empty, 4); mbar_init(&bars->dq_empty, 4);
+        mbar_init(&bars->dkv_empty, GATE_WARPS); mbar_init(&bars->dq_empty, 4);
         mbar_init(&bars->blk_done, 1); mbar_init(&bars->flushed, GATE_WARPS); mbar_init(&bars->drain, 2);
         bars->abort_flag = *reinterpret_cast<volatile int*>(status);
         bars->drain_flag = 0;
@@ -169,150 +169,168 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
     const float unit = exp2f(kappa - 4.0f) * e2 ;         // dS, dK, dc and dpre carry this factor (dS ln 2 more)
 
     if (warp < GATE_WARPS) {
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
-        // ======================================================== gate: item r, chunks wg and wg + 2
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
+        // ======================================================== gate: item r, columns 8 wg .. 8 wg + 7 of every chunk
         const int wg = warp >> 2, r = tid & 127, x7 = r & 7;
         const uint32_t t_lane = tmem + ((uint32_t)((warp & 3) * 32) << 16);
         const int2* meta = it.meta + (size_t)bt * it.IB * IBLK + r;
-        unsigned char* kd1 = sm + (wg == 0 ? M::B0 : M::DS) + r * 128;          // first pass: this group's K and V tiles
-        unsigned char* vd1 = sm + (wg == 0 ? M::B1 : M::DS + ATOM) + r * 128;
         const float oe = 0.25f / unit, ov = oe * 0.0625f;
-        int er = n_it > 0 ? (int)e_row(a, b, __ldg(&meta[0].x)) : 0, er_next = er;
+        size_t eo = 0;          // this item's E columns of chunk 0
         ERow<EF32> ek, ev;
         if (n_it > 0) {
-            ek = load_e<EF32>(a.Ek, (size_t)er * D + h * HD + wg * 16);
-            ev = load_e<EF32>(a.Ev, (size_t)er * D + h * HD + wg * 16);
+            eo = e_row(a, b, __ldg(&meta[0].x)) * D + h * HD + wg * 8;
+            ek = load_e<EF32>(a.Ek, eo);
+            ev = load_e<EF32>(a.Ev, eo);
         }
         bool alive = true;
         for (int i = 0; i < n_it && alive; ++i) {
             const int blk = i % n_blk;
+            // ---------------------------------------------------- first pass: K_c and V_c
 #pragma unroll 1
-            for (int ph = 0; ph < 4 && alive; ++ph) {
-                const int cc = ph & 1, c = wg + 2 * cc;
-                const bool second = ph >= 2;
-                // the E columns of this thread's next chunk fly while this one is worked on
-                ERow<EF32> nk = ek, nv = ev;
-                if (ph == 2 && i + 1 < n_it) er_next = (int)e_row(a, b, __ldg(&meta[(size_t)((i + 1) % n_blk) * IBLK].x));
-                if (ph < 3 || i + 1 < n_it) {
-                    const size_t off = (size_t)(ph == 3 ? er_next : er) * D + h * HD + (wg + 2 * (cc ^ 1)) * 16;
-                    nk = load_e<EF32>(a.Ek, off);
-                    nv = load_e<EF32>(a.Ev, off);
-                }
-                const int use = 2 * i + cc;
-                if (!(alive = warp_wait(second ? &bars->pre2_full[wg] : &bars->pre1_full[wg], (uint32_t)(use & 1), abort_flag, 1, lim))) break;
+            for (int c = 0; c < NCH; ++c) {
+                // the E columns of the next chunk fly while this one is worked on
+                const size_t off = eo + ((c + 1) & (NCH - 1)) * 16;
+                const ERow<EF32> nk = load_e<EF32>(a.Ek, off), nv = load_e<EF32>(a.Ev, off);
+                const int st = c & 1;
+                if (!(alive = warp_wait(&bars->pre1_full[st], (uint32_t)((2 * i + (c >> 1)) & 1), abort_flag, 1, lim))) break;
                 tc_fence_after_sync();
-                const uint32_t t_pre = t_lane + ((second || wg == 0) ? T_PRE : T_DQ);
-                uint32_t cf[2][NJ][4], sp[2][NJ][4];
+                uint32_t cf[NJ][4], none[1][4];
                 {
-                    float x[2][NJ][8];
+                    float x[NJ][8];
 #pragma unroll
-                    for (int j = 0; j < NJ; ++j) tmem_ld_32x32b_x8(t_pre + j * 16, x[0][j]);
-                    tmem_wait_ld();
-#pragma unroll
-                    for (int j = 0; j < NJ; ++j) tmem_ld_32x32b_x8(t_pre + j * 16 + 8, x[1][j]);
-                    gate_coefficients<SILU, true>(x[0], cf[0], sp[0]);
+                    for (int j = 0; j < NJ; ++j) tmem_ld_32x32b_x8(t_lane + (st ? T_DQ : T_PRE) + j * 16 + wg * 8, x[j]);
                     tmem_wait_ld();
                     tc_fence_before_sync();
                     __syncwarp();
-                    if (lane == 0 && !(a.test_withhold && i == 0 && ph == 0)) mbar_arrive(&bars->pre_empty[second ? 0 : wg]);
-                    gate_coefficients<SILU, true>(x[1], cf[1], sp[1]);
+                    if (lane == 0 && !(a.test_withhold && i == 0 && c == 0)) mbar_arrive(&bars->pre_empty[st]);
+                    gate_coefficients<SILU, false>(x, cf, none);
                 }
                 // where the operand tiles go: free once the products that read them last have completed
-                if (!second) {
-                    if (cc == 0) { if (i >= 1) alive = warp_wait(&bars->blk_done, (uint32_t)((i - 1) & 1), abort_flag, 2, lim); }
-                    else alive = warp_wait(&bars->kv_free[wg], (uint32_t)(i & 1), abort_flag, 3, lim);
-                } else {
-                    if (c == 0) alive = warp_wait(&bars->sdp_full, (uint32_t)(i & 1), abort_flag, 4, lim);
-                    else alive = warp_wait(&bars->kg_free[(c - 1) & 1], (uint32_t)((2 * i + ((c - 1) >> 1)) & 1), abort_flag, 5, lim);
-                }
+                if (c == 0) { if (i >= 1) alive = warp_wait(&bars->blk_done, (uint32_t)((i - 1) & 1), abort_flag, 2, lim); }
+                else if (c >= 2) alive = warp_wait(&bars->kv_free[st], (uint32_t)(i & 1), abort_flag, 3, lim);
                 if (!alive) break;
-                unsigned char* kd = second ? sm + M::B0 + r * 128 : kd1;
+                unsigned char* kd = sm + (st ? M::DS : M::B0) + r * 128;
 #pragma unroll
-                for (int g = 0; g < 2; ++g) {
-                    uint32_t e4[4], f4[4];
+                for (int t = 0; t < 2; ++t) {      // K to the first tile, V to the one behind it
+                    uint32_t e4[4];
 #pragma unroll
-                    for (int p = 0; p < 4; ++p) { e4[p] = e_pair<EF32>(ek, 4 * g + p); f4[p] = e_pair<EF32>(ev, 4 * g + p); }
+                    for (int p = 0; p < 4; ++p) e4[p] = e_pair<EF32>(t == 0 ? ek : ev, p);
 #pragma unroll
-                    for (int j = 0; j < NJ; ++j) {
-                        const int off = ((2 * j + g) ^ x7) << 4;
-                        st_shared_v4(kd + off, mul_f16x2(cf[g][j][0], e4[0]), mul_f16x2(cf[g][j][1], e4[1]), mul_f16x2(cf[g][j][2], e4[2]), mul_f16x2(cf[g][j][3], e4[3]));
-                        if (!second)
-                            st_shared_v4(vd1 + off, mul_f16x2(cf[g][j][0], f4[0]), mul_f16x2(cf[g][j][1], f4[1]), mul_f16x2(cf[g][j][2], f4[2]), mul_f16x2(cf[g][j][3], f4[3]));
-                    }
+                    for (int j = 0; j < NJ; ++j)
+                        st_shared_v4(kd + t * ATOM + (((2 * j + wg) ^ x7) << 4), mul_f16x2(cf[j][0], e4[0]), mul_f16x2(cf[j][1], e4[1]), mul_f16x2(cf[j][2], e4[2]), mul_f16x2(cf[j][3], e4[3]));
                 }
                 fence_proxy_async_smem();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(second ? &bars->kg_full[wg] : &bars->kv_full[wg]);
-                if (second) {
-                    if (!(alive = warp_wait(&bars->dkv_full[wg], (uint32_t)(use & 1), abort_flag, 6, lim))) break;
-                    tc_fence_after_sync();
-                    if (c >= 1 && !(alive = warp_wait(&bars->dp_free[(c - 1) & 1], (uint32_t)((2 * i + ((c - 1) >> 1)) & 1), abort_flag, 7, lim))) break;
-                    float* gk = a.dEk + (size_t)er * D + h * HD + c * 16;
-                    float* gv = a.dEv + (size_t)er * D + h * HD + c * 16;
-                    const bool live = blk * IBLK + r < n_items;
-#pragma unroll
-                    for (int g = 0; g < 2; ++g) {
-                        uint32_t m0[4], m1[4];
-#pragma unroll
-                        for (int q = 0; q < 2; ++q) {      // four columns at a time
-                            float dk[NJ][4], dv[NJ][4];
-#pragma unroll
-                            for (int j = 0; j < NJ; ++j) {
-                                tmem_ld_x4(t_lane + T_DP + j * 16 + g * 8 + q * 4, dk[j]);
-                                tmem_ld_x4(t_lane + T_DP + 64 + j * 16 + g * 8 + q * 4, dv[j]);
-                            }
-                            tmem_wait_ld();
-                            float ok[4], ovv[4];
-#pragma unroll
-                            for (int p = 0; p < 2; ++p) {
-                                const int pp = 2 * q + p;
-                                const f32x2 e = unpack_h2(e_pair<EF32>(ek, 4 * g + pp)), f0 = unpack_h2(e_pair<EF32>(ev, 4 * g + pp));
-                                const f32x2 f = mul2(f0, pack2(0.0625f, 0.0625f));
-                                f32x2 dc[NJ], sk = 0ull, sv = 0ull;
-#pragma unroll
-                                for (int j = 0; j < NJ; ++j) {
-                                    const f32x2 k2 = pack2(dk[j][2 * p], dk[j][2 * p + 1]), v2 = pack2(dv[j][2 * p], dv[j][2 * p + 1]);
-                                    const f32x2 cj = unpack_h2(cf[g][j][pp]);
-                                    sk = j == 0 ? mul2(cj, k2) : fma2(cj, k2, sk);
-                                    sv = j == 0 ? mul2(cj, v2) : fma2(cj, v2, sv);
-                                    dc[j] = fma2(f, v2, mul2(e, k2));
-                                }
-                                const f32x2 m = pack2(-1.f, -1.f), ka = pack2(TAN_PI_8, TAN_PI_8), kn = pack2(-TAN_PI_8, -TAN_PI_8);
-                                const f32x2 u0 = add2(dc[0], dc[2]), u1 = fma2(dc[2], m, dc[0]), v0 = fma2(dc[3], kn, dc[1]), v1 = fma2(dc[1], ka, dc[3]);
-                                f32x2 d0 = add2(u0, v0), d3 = fma2(v0, m, u0), d1 = add2(u1, v1), d2 = fma2(v1, m, u1);
-                                if (SILU) {
-                                    d0 = mul2(d0, unpack_h2(sp[g][0][pp])); d1 = mul2(d1, unpack_h2(sp[g][1][pp]));
-                                    d2 = mul2(d2, unpack_h2(sp[g][2][pp])); d3 = mul2(d3, unpack_h2(sp[g][3][pp]));
-                                }
-                                // moments over the nodes, an eighth of the unit
-                                const f32x2 c8 = pack2(0.125f, 0.125f), ta = pack2(0.125f * 0.9238795325f, 0.125f * 0.9238795325f),
-                                            tb = pack2(0.125f * 0.3826834324f, 0.125f * 0.3826834324f);
-                                const f32x2 s = mul2(add2(add2(d0, d3), add2(d1, d2)), c8);
-                                const f32x2 x = fma2(fma2(d2, m, d1), tb, mul2(fma2(d3, m, d0), ta));
-                                float lo, hi;
-                                unpack2(s, lo, hi); m0[pp] = pack_f16x2_sat(lo, hi);
-                                unpack2(x, lo, hi); m1[pp] = pack_f16x2_sat(lo, hi);
-                                unpack2(sk, ok[2 * p], ok[2 * p + 1]);
-                                unpack2(sv, ovv[2 * p], ovv[2 * p + 1]);
-                            }
-                            if (live) {
-                                red_v4(gk + g * 8 + q * 4, ok[0] * oe, ok[1] * oe, ok[2] * oe, ok[3] * oe);
-                                red_v4(gv + g * 8 + q * 4, ovv[0] * ov, ovv[1] * ov, ovv[2] * ov, ovv[3] * ov);
-                            }
-                        }
-                        unsigned char* zd = sm + M::B1 + r * 128;
-                        st_shared_v4(zd + ((g ^ x7) << 4), m0[0], m0[1], m0[2], m0[3]);
-                        st_shared_v4(zd + (((2 + g) ^ x7) << 4), m1[0], m1[1], m1[2], m1[3]);
-                    }
-                    tc_fence_before_sync();
-                    fence_proxy_async_smem();
-                    __syncwarp();
-                    if (lane == 0) { mbar_arrive(&bars->dkv_empty); mbar_arrive(&bars->dpre_full[wg]); }
-                }
+                if (lane == 0) mbar_arrive(&bars->kv_full[st]);
                 ek = nk;
                 ev = nv;
             }
-            er = er_next;
+            if (!alive) break;
+            // ---------------------------------------------------- second pass: K_c again; dE rows, node gradients
+            size_t eo_next = eo;
+#pragma unroll 1
+            for (int c = 0; c < NCH; ++c) {
+                if (c == NCH - 1 && i + 1 < n_it) eo_next = e_row(a, b, __ldg(&meta[(size_t)((i + 1) % n_blk) * IBLK].x)) * D + h * HD + wg * 8;
+                const size_t off = eo_next + ((c + 1) & (NCH - 1)) * 16;
+                const ERow<EF32> nk = load_e<EF32>(a.Ek, off), nv = load_e<EF32>(a.Ev, off);
+                const int st = c & 1, use = 2 * i + (c >> 1);
+                if (!(alive = warp_wait(&bars->pre2_full[st], (uint32_t)(use & 1), abort_flag, 1, lim))) break;
+                tc_fence_after_sync();
+                uint32_t cf[NJ][4], sp[NJ][4];
+                {
+                    float x[NJ][8];
+#pragma unroll
+                    for (int j = 0; j < NJ; ++j) tmem_ld_32x32b_x8(t_lane + T_PRE + j * 16 + wg * 8, x[j]);
+                    tmem_wait_ld();
+                    tc_fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&bars->pre_empty[0]);
+                    gate_coefficients<SILU, true>(x, cf, sp);
+                }
+                if (c == 0) alive = warp_wait(&bars->sdp_full, (uint32_t)(i & 1), abort_flag, 4, lim);
+                else alive = warp_wait(&bars->kg_free[(c - 1) & 1], (uint32_t)((2 * i + ((c - 1) >> 1)) & 1), abort_flag, 5, lim);
+                if (!alive) break;
+                {
+                    uint32_t e4[4];
+#pragma unroll
+                    for (int p = 0; p < 4; ++p) e4[p] = e_pair<EF32>(ek, p);
+#pragma unroll
+                    for (int j = 0; j < NJ; ++j)
+                        st_shared_v4(sm + M::B0 + r * 128 + (((2 * j + wg) ^ x7) << 4), mul_f16x2(cf[j][0], e4[0]), mul_f16x2(cf[j][1], e4[1]), mul_f16x2(cf[j][2], e4[2]), mul_f16x2(cf[j][3], e4[3]));
+                }
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bars->kg_full[st]);
+                if (!(alive = warp_wait(&bars->dkv_full[st], (uint32_t)(use & 1), abort_flag, 6, lim))) break;
+                tc_fence_after_sync();
+                float* gk = a.dEk + eo + c * 16;
+                float* gv = a.dEv + eo + c * 16;
+                const bool live = blk * IBLK + r < n_items;
+                uint32_t m0[4], m1[4];
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {      // four columns at a time
+                    float dk[NJ][4], dv[NJ][4];
+#pragma unroll
+                    for (int j = 0; j < NJ; ++j) {
+                        tmem_ld_x4(t_lane + T_DP + j * 16 + wg * 8 + q * 4, dk[j]);
+                        tmem_ld_x4(t_lane + T_DP + 64 + j * 16 + wg * 8 + q * 4, dv[j]);
+                    }
+                    tmem_wait_ld();
+                    if (q == 1) {          // all columns are in registers
+                        tc_fence_before_sync();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&bars->dkv_empty);
+                    }
+                    float ok[4], ovv[4];
+#pragma unroll
+                    for (int p = 0; p < 2; ++p) {
+                        const int pp = 2 * q + p;
+                        const f32x2 e = unpack_h2(e_pair<EF32>(ek, pp)), f0 = unpack_h2(e_pair<EF32>(ev, pp));
+                        const f32x2 f = mul2(f0, pack2(0.0625f, 0.0625f));
+                        f32x2 dc[NJ], sk = 0ull, sv = 0ull;
+#pragma unroll
+                        for (int j = 0; j < NJ; ++j) {
+                            const f32x2 k2 = pack2(dk[j][2 * p], dk[j][2 * p + 1]), v2 = pack2(dv[j][2 * p], dv[j][2 * p + 1]);
+                            const f32x2 cj = unpack_h2(cf[j][pp]);
+                            sk = j == 0 ? mul2(cj, k2) : fma2(cj, k2, sk);
+                            sv = j == 0 ? mul2(cj, v2) : fma2(cj, v2, sv);
+                            dc[j] = fma2(f, v2, mul2(e, k2));
+                        }
+                        const f32x2 m = pack2(-1.f, -1.f), ka = pack2(TAN_PI_8, TAN_PI_8), kn = pack2(-TAN_PI_8, -TAN_PI_8);
+                        const f32x2 u0 = add2(dc[0], dc[2]), u1 = fma2(dc[2], m, dc[0]), v0 = fma2(dc[3], kn, dc[1]), v1 = fma2(dc[1], ka, dc[3]);
+                        f32x2 d0 = add2(u0, v0), d3 = fma2(v0, m, u0), d1 = add2(u1, v1), d2 = fma2(v1, m, u1);
+                        if (SILU) {
+                            d0 = mul2(d0, unpack_h2(sp[0][pp])); d1 = mul2(d1, unpack_h2(sp[1][pp]));
+                            d2 = mul2(d2, unpack_h2(sp[2][pp])); d3 = mul2(d3, unpack_h2(sp[3][pp]));
+                        }
+                        // moments over the nodes, an eighth of the unit
+                        const f32x2 c8 = pack2(0.125f, 0.125f), ta = pack2(0.125f * 0.9238795325f, 0.125f * 0.9238795325f),
+                                    tb = pack2(0.125f * 0.3826834324f, 0.125f * 0.3826834324f);
+                        const f32x2 s = mul2(add2(add2(d0, d3), add2(d1, d2)), c8);
+                        const f32x2 x = fma2(fma2(d2, m, d1), tb, mul2(fma2(d3, m, d0), ta));
+                        float lo, hi;
+                        unpack2(s, lo, hi); m0[pp] = pack_f16x2_sat(lo, hi);
+                        unpack2(x, lo, hi); m1[pp] = pack_f16x2_sat(lo, hi);
+                        unpack2(sk, ok[2 * p], ok[2 * p + 1]);
+                        unpack2(sv, ovv[2 * p], ovv[2 * p + 1]);
+                    }
+                    if (live) {
+                        red_v4(gk + q * 4, ok[0] * oe, ok[1] * oe, ok[2] * oe, ok[3] * oe);
+                        red_v4(gv + q * 4, ovv[0] * ov, ovv[1] * ov, ovv[2] * ov, ovv[3] * ov);
+                    }
+                }
+                // the tile of the moments: free once the dW product before has read it
+                if (c >= 1 && !(alive = warp_wait(&bars->dp_free[(c - 1) & 1], (uint32_t)((2 * i + ((c - 1) >> 1)) & 1), abort_flag, 7, lim))) break;
+                unsigned char* zd = sm + M::B1 + r * 128;
+                st_shared_v4(zd + ((wg ^ x7) << 4), m0[0], m0[1], m0[2], m0[3]);
+                st_shared_v4(zd + (((2 + wg) ^ x7) << 4), m1[0], m1[1], m1[2], m1[3]);
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bars->dpre_full[st]);
+                ek = nk;
+                ev = nv;
+            }
+            eo = eo_next;
             if (alive && blk == n_blk - 1) {
                 // the segment's dW: lane n, chunks 2 wg and 2 wg + 1
                 if (!(alive = warp_wait(&bars->blk_done, (uint32_t)(i & 1), abort_flag, 8, lim))) break;
@@ -372,28 +390,25 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
             tc_fence_after_sync();
             uint32_t p2[32];
 #pragma unroll
-            for (int k = 0; k < 2; ++k) {
-                const int tb = half * 64 + k * 32;
-                float s[32];
-                tmem_ld_32x32b_x32(t_lane + T_S + tb, s);
+            for (int k = 0; k < 4; ++k) {
+                const int tb = half * 64 + k * 16;
+                float s[16];
+                tmem_ld_32x32b_x16(t_lane + T_S + tb, s);
                 tmem_wait_ld();
-                const bool full = __all_sync(0xffffffffu, lo <= tb && hi >= tb + 31);
-                unsigned mask = 0xffffffffu;
-                if (!full) {
-                    const int l0 = max(lo - tb, 0), h0 = min(hi - tb, 31);
-                    mask = l0 > h0 ? 0u : ((0xffffffffu >> (31 - h0)) & (0xffffffffu << l0));
-                }
+                const bool full = __all_sync(0xffffffffu, lo <= tb && hi >= tb + 15);
 #pragma unroll
-                for (int e = 0; e < 32; e += 4) {
+                for (int e = 0; e < 16; e += 4) {
                     const float4 ls = *reinterpret_cast<const float4*>(lse_sh + tb + e);
                     s[e] -= ls.x; s[e + 1] -= ls.y; s[e + 2] -= ls.z; s[e + 3] -= ls.w;
                 }
                 if (!full) {
+                    const int l0 = max(lo - tb, 0), h0 = min(hi - tb, 15);
+                    const unsigned mask = l0 > h0 ? 0u : ((0xffffffffu >> (31 - h0)) & (0xffffffffu << l0));
 #pragma unroll
-                    for (int e = 0; e < 32; ++e) s[e] = (mask >> e) & 1u ? s[e] : -INFINITY;
+                    for (int e = 0; e < 16; ++e) s[e] = (mask >> e) & 1u ? s[e] : -INFINITY;
                 }
 #pragma unroll
-                for (int e = 0; e < 32; e += 2) p2[k * 16 + e / 2] = pack_f16x2_sat(ex2_approx(s[e]), ex2_approx(s[e + 1]));
+                for (int e = 0; e < 16; e += 2) p2[k * 8 + e / 2] = pack_f16x2_sat(ex2_approx(s[e]), ex2_approx(s[e + 1]));
             }
             tc_fence_before_sync();
             __syncwarp();
@@ -431,18 +446,21 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
             for (int cc = 0; cc < 2; ++cc) {
                 if (!(alive = warp_wait(&bars->dq_full[half], (uint32_t)((2 * i + cc) & 1), abort_flag, 11, lim))) break;
                 tc_fence_after_sync();
-                float v[2][32];
-                tmem_ld_32x32b_x32(t_lane + T_DQ, v[0]);
-                tmem_wait_ld();
+                float v[2][16];        // a coefficient's columns at a time, the next ones in flight
+                tmem_ld_32x32b_x16(t_lane + T_DQ, v[0]);
 #pragma unroll
-                for (int e = 0; e < 16; ++e) acc[cc][e] = fmaf(beta[1], v[0][16 + e], acc[cc][e] + v[0][e]);
-                tmem_ld_32x32b_x32(t_lane + T_DQ + 32, v[1]);
-                tmem_wait_ld();
-                tc_fence_before_sync();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&bars->dq_empty);
+                for (int j = 0; j < NJ; ++j) {
+                    tmem_wait_ld();
+                    if (j + 1 < NJ) {
+                        tmem_ld_32x32b_x16(t_lane + T_DQ + (j + 1) * 16, v[(j + 1) & 1]);
+                    } else {
+                        tc_fence_before_sync();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&bars->dq_empty);
+                    }
 #pragma unroll
-                for (int e = 0; e < 16; ++e) acc[cc][e] = fmaf(beta[3], v[1][16 + e], fmaf(beta[2], v[1][e], acc[cc][e]));
+                    for (int e = 0; e < 16; ++e) acc[cc][e] = j == 0 ? acc[cc][e] + v[0][e] : fmaf(beta[j], v[j & 1][e], acc[cc][e]);
+                }
             }
             if (!alive) break;
         }
@@ -456,7 +474,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
                         make_float4(acc[cc][e] * sc, acc[cc][e + 1] * sc, acc[cc][e + 2] * sc, acc[cc][e + 3] * sc);
         }
     } else {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
         if (warp == W_LOAD && lane == 0) {
             // ==================================================== loader: A per block; W' (and dO') chunks for both passes
             const unsigned char* img = it.a_img + (size_t)bt * it.IB * NK * ATOM;

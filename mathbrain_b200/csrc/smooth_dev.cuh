@@ -6,21 +6,21 @@
 namespace mbema {
 namespace smooth {
 
-// 16 columns of an E row as stored
-template <bool EF32> struct ERow { uint4 v[EF32 ? 4 : 2]; };
+// eight columns of an E row as stored
+template <bool EF32> struct ERow { uint4 v[EF32 ? 2 : 1]; };
 template <bool EF32>
 __device__ __forceinline__ ERow<EF32> load_e(const void* E, size_t off) {
     ERow<EF32> r;
     const uint4* p = reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned char*>(E) + off * (EF32 ? 4 : 2));
 #pragma unroll
-    for (int i = 0; i < (EF32 ? 4 : 2); ++i) r.v[i] = __ldg(p + i);
+    for (int i = 0; i < (EF32 ? 2 : 1); ++i) r.v[i] = __ldg(p + i);
     return r;
 }
 // columns 2p, 2p + 1 as fp16, times 1/4 (see basis())
 template <bool EF32>
 __device__ __forceinline__ uint32_t e_pair(const ERow<EF32>& r, int p) {
     const uint32_t* u = reinterpret_cast<const uint32_t*>(r.v);
-    if (EF32) return ptx::pack_f16x2_sat(__uint_as_float(u[2 * p]) * 0.25f, __uint_as_float(u[2 * p + 1]) * 0.25f);
+    if (EF32) return ptx::pack_f16x2_sat(__uint_as_float(u[(2 * p) & 7]) * 0.25f, __uint_as_float(u[(2 * p + 1) & 7]) * 0.25f);
     return ptx::pack_f16x2_sat(ptx::bf16_lo(u[p]) * 0.25f, ptx::bf16_hi(u[p]) * 0.25f);
 }
 
@@ -32,7 +32,7 @@ __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volati
 // Gate of eight columns at the four nodes (x: half the pre-activation for SiLU) -> Chebyshev coefficients as fp16 pairs
 // and, with DERIV, SiLU' at the nodes as fp16 pairs.
 template <bool SILU, bool DERIV>
-__device__ __forceinline__ void gate_coefficients(const float (&x)[NJ][8], uint32_t (&cf)[NJ][4], uint32_t (&sp)[NJ][4]) {
+__device__ __forceinline__ void gate_coefficients(const float (&x)[NJ][8], uint32_t (&cf)[NJ][4], uint32_t (&sp)[DERIV ? NJ : 1][4]) {
     using namespace ptx;
 #pragma unroll
     for (int p = 0; p < 4; ++p) {
@@ -51,7 +51,7 @@ __device__ __forceinline__ void gate_coefficients(const float (&x)[NJ][8], uint3
                     const f32x2 d = fma2(fma2(hh, u, th), pack2(0.5f, 0.5f), pack2(0.5f, 0.5f));
                     float lo, hi;
                     unpack2(d, lo, hi);
-                    sp[j][p] = pack_f16x2(lo, hi);
+                    sp[DERIV ? j : 0][p] = pack_f16x2(lo, hi);
                 }
             }
         }

@@ -5,7 +5,7 @@
 //     pre_c [128 items x 64]  = A . W'_c            A: item states, W'_c: W_pe scaled to the four nodes
 //     S     [128 steps x 128] += Q'_c . K_c^T       K_c = E_k c_j, written by the gate warps
 //     O'_c  [128 steps x 64]  += P . V_c            P from tensor memory, V_c = E_v c_j
-// Warps: two gate warpgroups (a thread per item; the even and the odd chunks), two softmax warpgroups (a thread per
+// Warps: two gate warpgroups (a thread per item; half of a chunk's columns each), two softmax warpgroups (a thread per
 // step and half a block's items), one loader (bulk copies of A and W' images), one lane issuing the gate products and
 // one issuing S and P.V, so that neither waits for the other's operands.  All hand-offs are mbarriers with bounded waits.
 //
@@ -23,7 +23,7 @@ namespace fwd {
 
 static constexpr int GATE_WARPS = 8, SM_WARPS = 8;
 static constexpr int W_LOAD = 16, W_GATE = 17, W_ATT = 18;       // warp 19 only fills the warpgroup
-static constexpr int THREADS = 20 * 32;      // launched with 96 registers a thread: 61440 >= 4 * 128 * 104 + 128 * 56
+static constexpr int THREADS = 20 * 32;      // launched with 96 registers a thread: 61440 = 4 * 128 * 104 + 128 * 64
 static constexpr uint32_t T_O = 0, T_S = 256, T_PRE = 384;     // tensor-memory columns
 static constexpr float RESCALE = 8.0f;      // log2 units the softmax reference may lag behind (P <= 2^8 in fp16)
 
@@ -64,10 +64,10 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_fwd(FlashArgs a, Items it
         for (int i = 0; i < 2; ++i) {
             mbar_init(&bars->a_full[i], 1); mbar_init(&bars->a_free[i], 1);
             mbar_init(&bars->w_full[i], 1); mbar_init(&bars->w_free[i], 1);
-            mbar_init(&bars->pre_full[i], 1); mbar_init(&bars->pre_empty[i], 4);
+            mbar_init(&bars->pre_full[i], 1); mbar_init(&bars->pre_empty[i], GATE_WARPS);
             mbar_init(&bars->k_free[i], 1);
         }
-        for (int i = 0; i < NCH; ++i) { mbar_init(&bars->kv_full[i], 4); mbar_init(&bars->v_free[i], 1); }
+        for (int i = 0; i < NCH; ++i) { mbar_init(&bars->kv_full[i], GATE_WARPS); mbar_init(&bars->v_free[i], 1); }
         mbar_init(&bars->s_full, 1); mbar_init(&bars->p_full, SM_WARPS); mbar_init(&bars->mx_full, SM_WARPS);
         mbar_init(&bars->o_full, 1); mbar_init(&bars->drain, 2);
         bars->abort_flag = *reinterpret_cast<volatile int*>(status);      // an earlier CTA gave up: do nothing
@@ -101,65 +101,56 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_fwd(FlashArgs a, Items it
     const unsigned* lim = &bars->spin_limit;
 
     if (warp < GATE_WARPS) {
-        // ======================================================== gate: item r, chunks wg and wg + 2
+        // ======================================================== gate: item r, columns 8 wg .. 8 wg + 7 of every chunk
         asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
         const int wg = warp >> 2, r = tid & 127;
-        const uint32_t t_pre = tmem + ((uint32_t)((warp & 3) * 32) << 16) + T_PRE + wg * 64;
+        const uint32_t t_pre = tmem + ((uint32_t)((warp & 3) * 32) << 16) + T_PRE + wg * 8;
         const int2* meta = it.meta + (size_t)bt * it.IB * IBLK + r;
         const int x7 = r & 7;
-        int er = n_it > 0 ? (int)e_row(a, b, __ldg(&meta[0].x)) : 0;
+        size_t eo = 0;          // this item's E columns of chunk 0
         ERow<EF32> ek, ev;
         if (n_it > 0) {
-            ek = load_e<EF32>(a.Ek, (size_t)er * D + h * HD + wg * 16);
-            ev = load_e<EF32>(a.Ev, (size_t)er * D + h * HD + wg * 16);
+            eo = e_row(a, b, __ldg(&meta[0].x)) * D + h * HD + wg * 8;
+            ek = load_e<EF32>(a.Ek, eo);
+            ev = load_e<EF32>(a.Ev, eo);
         }
         bool alive = true;
         for (int i = 0; i < n_it && alive; ++i) {
 #pragma unroll 1
-            for (int cc = 0; cc < 2; ++cc) {
-                const int c = wg + 2 * cc;
+            for (int c = 0; c < NCH; ++c) {
                 // the next chunk's E columns fly while this chunk is worked on
                 ERow<EF32> nk = ek, nv = ev;
-                if (cc == 1 && i + 1 < n_it) er = (int)e_row(a, b, __ldg(&meta[(size_t)((i + 1) % n_blk) * IBLK].x));
-                if (cc == 0 || i + 1 < n_it) {
-                    const size_t off = (size_t)er * D + h * HD + (wg + 2 * (cc ^ 1)) * 16;
+                if (c == NCH - 1 && i + 1 < n_it) eo = e_row(a, b, __ldg(&meta[(size_t)((i + 1) % n_blk) * IBLK].x)) * D + h * HD + wg * 8;
+                if (c < NCH - 1 || i + 1 < n_it) {
+                    const size_t off = eo + ((c + 1) & (NCH - 1)) * 16;
                     nk = load_e<EF32>(a.Ek, off);
                     nv = load_e<EF32>(a.Ev, off);
                 }
-                const int use = 2 * i + cc;
-                if (!(alive = warp_wait(&bars->pre_full[wg], (uint32_t)(use & 1), abort_flag, 1, lim))) break;
+                const int st = c & 1, use = 2 * i + (c >> 1);
+                if (!(alive = warp_wait(&bars->pre_full[st], (uint32_t)(use & 1), abort_flag, 1, lim))) break;
                 tc_fence_after_sync();
-                float x[2][NJ][8];
+                float x[NJ][8];
 #pragma unroll
-                for (int j = 0; j < NJ; ++j) tmem_ld_32x32b_x8(t_pre + j * 16, x[0][j]);
+                for (int j = 0; j < NJ; ++j) tmem_ld_32x32b_x8(t_pre + st * 64 + j * 16, x[j]);
                 tmem_wait_ld();
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0 && !(a.test_withhold && use == 0)) mbar_arrive(&bars->pre_empty[st]);
+                uint32_t cf[NJ][4], none[1][4];
+                gate_coefficients<SILU, false>(x, cf, none);
+                if (use >= 1 && !(alive = warp_wait(&bars->k_free[st], (uint32_t)((use - 1) & 1), abort_flag, 2, lim))) break;
+                unsigned char* kd = sm + K_OFF + st * ATOM + r * 128;
+                uint32_t e2[4], f2[4];
 #pragma unroll
-                for (int j = 0; j < NJ; ++j) tmem_ld_32x32b_x8(t_pre + j * 16 + 8, x[1][j]);
-                unsigned char* kd = sm + K_OFF + wg * ATOM + r * 128;
+                for (int p = 0; p < 4; ++p) { e2[p] = e_pair<EF32>(ek, p); f2[p] = e_pair<EF32>(ev, p); }
+#pragma unroll
+                for (int j = 0; j < NJ; ++j)
+                    st_shared_v4(kd + (((2 * j + wg) ^ x7) << 4), mul_f16x2(cf[j][0], e2[0]), mul_f16x2(cf[j][1], e2[1]), mul_f16x2(cf[j][2], e2[2]), mul_f16x2(cf[j][3], e2[3]));
+                if (i >= 1 && !(alive = warp_wait(&bars->v_free[c], (uint32_t)((i - 1) & 1), abort_flag, 3, lim))) break;
                 unsigned char* vd = sm + V_OFF + c * ATOM + r * 128;
 #pragma unroll
-                for (int g = 0; g < 2; ++g) {
-                    uint32_t cf[NJ][4];
-                    gate_coefficients<SILU, false>(x[g], cf, cf);
-                    if (g == 0) {
-                        tmem_wait_ld();            // the second half's columns are in registers
-                        tc_fence_before_sync();
-                        __syncwarp();
-                        if (lane == 0 && !(a.test_withhold && use == 0)) mbar_arrive(&bars->pre_empty[wg]);
-                        if (use >= 1 && !(alive = warp_wait(&bars->k_free[wg], (uint32_t)((use - 1) & 1), abort_flag, 2, lim))) break;
-                        if (i >= 1 && !(alive = warp_wait(&bars->v_free[c], (uint32_t)((i - 1) & 1), abort_flag, 3, lim))) break;
-                    }
-                    uint32_t e2[4], f2[4];
-#pragma unroll
-                    for (int p = 0; p < 4; ++p) { e2[p] = e_pair<EF32>(ek, 4 * g + p); f2[p] = e_pair<EF32>(ev, 4 * g + p); }
-#pragma unroll
-                    for (int j = 0; j < NJ; ++j) {
-                        const int off = ((2 * j + g) ^ x7) << 4;
-                        st_shared_v4(kd + off, mul_f16x2(cf[j][0], e2[0]), mul_f16x2(cf[j][1], e2[1]), mul_f16x2(cf[j][2], e2[2]), mul_f16x2(cf[j][3], e2[3]));
-                        st_shared_v4(vd + off, mul_f16x2(cf[j][0], f2[0]), mul_f16x2(cf[j][1], f2[1]), mul_f16x2(cf[j][2], f2[2]), mul_f16x2(cf[j][3], f2[3]));
-                    }
-                }
-                if (!alive) break;
+                for (int j = 0; j < NJ; ++j)
+                    st_shared_v4(vd + (((2 * j + wg) ^ x7) << 4), mul_f16x2(cf[j][0], f2[0]), mul_f16x2(cf[j][1], f2[1]), mul_f16x2(cf[j][2], f2[2]), mul_f16x2(cf[j][3], f2[3]));
                 fence_proxy_async_smem();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&bars->kv_full[c]);
@@ -229,15 +220,15 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_fwd(FlashArgs a, Items it
             float l0 = 0.f, l1 = 0.f;
             // P as fp16 pairs over the half's own score columns (all of them are in registers by now)
 #pragma unroll
-            for (int k = 0; k < 64; k += 32) {
-                uint32_t p2[16];
+            for (int k = 0; k < 64; k += 16) {
+                uint32_t p2[8];
 #pragma unroll
-                for (int e = 0; e < 16; ++e) {
+                for (int e = 0; e < 8; ++e) {
                     const float p = ex2_approx(s[k + 2 * e] - mm), q = ex2_approx(s[k + 2 * e + 1] - mm);
                     l0 += p; l1 += q;
                     p2[e] = pack_f16x2(p, q);
                 }
-                tmem_st_x16(t_row + T_S + half * 64 + k / 2, p2);
+                tmem_st_x8(t_row + T_S + half * 64 + k / 2, p2);
             }
             l += l0 + l1;
             tmem_wait_st();
@@ -292,7 +283,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_fwd(FlashArgs a, Items it
             if (alive && half == 0 && t0 + row < a.T) a.LSE[row0 + row] = ok ? mm * 0.6931471806f + logf(l) : 0.f;
         }
     } else {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
         if (warp == W_LOAD && lane == 0) {
             // ==================================================== loader
             const unsigned char* img = it.a_img + (size_t)bt * it.IB * NK * ATOM;
