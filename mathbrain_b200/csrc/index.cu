@@ -175,22 +175,23 @@ __global__ void __launch_bounds__(256) k_relink(const int64_t* __restrict__ keys
 // one warp per chain; lanes hold channels lane, lane+32, lane+64, lane+96
 // ----------------------------------------------------------------------------------------------
 static constexpr int CHAIN_WARPS = 8;
+static constexpr int AHEAD = 4;            // steps of a walked chain whose powers are evaluated together
 static constexpr int LONG_CHAIN = 64;      // occurrences from which a chain is scanned with warp shuffles instead of walked
-static constexpr int COOP_BLOCKS = 2;      // CTAs per sample, at the end of the grid, that scan the long chains
 
 // Long chains (the padding token, the most frequent tokens) are not walked but scanned: with U the carried value
 // (state + 1 after the previous occurrence; the seed before the first), occurrence j reads v_j = A_j U_j and hands on
 // U_{j+1} = A_j U_j + 1, A_j = keep_j rho^(t_j - t_{j-1}): an affine map per occurrence.  32 occurrences sit on the
 // lanes and the maps are composed with warp shuffles (a segmented prefix product over time, five steps per block of
-// 32); the N channels are split over the eight warps of the CTA, so a chain of L occurrences costs L/32 * N/8 short
-// scans instead of L dependent steps.  Results go through shared memory so that a row's channels leave together.
+// 32).  The work is dealt out by (chain, 32 channels): a warp takes four channels, whose scans and double-precision powers
+// run side by side, so a chain of L occurrences costs L/32 scans instead of L dependent steps; 4096-step chunks have some ten
+// long chains a sample, so the number of CTAs that share them grows with T.
+__host__ __device__ inline int long_chain_blocks(int T) { return T < 512 ? 2 : T < 4096 ? T / 128 : 32; }
+
 __device__ void scan_long_chains(const IndexWs& w, const float* __restrict__ rhos, const float* __restrict__ c_init,
                                  const int32_t* __restrict__ doc_ids, float* __restrict__ out, int T, int N, int K,
-                                 int extra_decay, int b, int q) {
-    __shared__ int lst[8192 / LONG_CHAIN];
+                                 int extra_decay, int b, int q, int n_blocks) {
+    __shared__ int found[8192 / LONG_CHAIN], lst[8192 / LONG_CHAIN];
     __shared__ int n_long;
-    __shared__ float tile[CHAIN_WARPS][32][17];
-    __shared__ int tile_t[CHAIN_WARPS][32];
     const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
     const int nch = w.n_chain[b];
     const int32_t* ch_off = w.ch_off + (size_t)b * T;
@@ -199,33 +200,44 @@ __device__ void scan_long_chains(const IndexWs& w, const float* __restrict__ rho
     __syncthreads();
     for (int c = tid; c < nch; c += blockDim.x) {
         const int len = ((c + 1 < nch) ? ch_off[c + 1] : T) - ch_off[c];
-        if (len >= LONG_CHAIN) lst[atomicAdd(&n_long, 1)] = c;
+        if (len >= LONG_CHAIN) found[atomicAdd(&n_long, 1)] = c;
     }
     __syncthreads();
-    const int nk = (N + CHAIN_WARPS - 1) / CHAIN_WARPS;          // channels of this warp: [wp * nk, wp * nk + nk)
-    const int n_mine = wp * nk + lane;                           // lane k < nk keeps rho, its log and the carry of channel k
-    const bool mine = lane < nk && n_mine < N;
-    const float rho_k = mine ? rhos[n_mine] : 1.0f;
-    const double l2r_k = mine ? log2((double)rho_k) : 0.0;
-    int kmax = min(nk, N - wp * nk);
-    if (kmax < 0) kmax = 0;
-    for (int li = q; li < n_long; li += COOP_BLOCKS) {
-        const int c = lst[li];
+    for (int i = tid; i < n_long; i += blockDim.x) {        // in chain order: every CTA of the sample deals the same list
+        int rank = 0;
+        for (int j = 0; j < n_long; ++j) rank += found[j] < found[i];
+        lst[rank] = found[i];
+    }
+    __syncthreads();
+    const int groups = (N + 31) / 32;
+    for (int unit = q; unit < n_long * groups; unit += n_blocks) {
+        const int c = lst[unit / groups], n0 = (unit % groups) * 32 + wp * 4;
+        if (n0 >= N) continue;
         const int j0 = ch_off[c];
         const int j1 = (c + 1 < nch) ? ch_off[c + 1] : T;
         const int sd = w.seed[(size_t)b * T + j0];
-        float car = 0.0f;
-        if (sd != NO_SEED && mine && c_init != nullptr) {
-            car = c_init[((size_t)b * K + sd) * N + n_mine];
-            if (extra_decay) car *= rho_k;
+        float rho[4], car[4];
+        double l2r[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const bool in = n0 + k < N;
+            rho[k] = in ? rhos[n0 + k] : 1.0f;
+            l2r[k] = log2((double)rho[k]);
+            car[k] = 0.0f;
+            if (sd != NO_SEED && in && c_init != nullptr) {
+                car[k] = c_init[((size_t)b * K + sd) * N + n0 + k];
+                if (extra_decay) car[k] *= rho[k];
+            }
         }
         bool has = (sd != NO_SEED);
         int s_ref = 0;
         int last_doc = (doc_ids != nullptr) ? doc_ids[(size_t)b * T] : 0;
+        int t_next = j0 + lane < j1 ? s_pos[j0 + lane] : 0;
         for (int jb = j0; jb < j1; jb += 32) {
             const int cnt = min(32, j1 - jb);
             const bool live = lane < cnt;
-            const int t_l = live ? s_pos[jb + lane] : 0;
+            const int t_l = t_next;
+            t_next = jb + 32 + lane < j1 ? s_pos[jb + 32 + lane] : 0;
             int t_prev = __shfl_up_sync(0xffffffffu, t_l, 1);
             if (lane == 0) t_prev = s_ref;
             bool keep = (lane == 0) ? has : true;
@@ -238,49 +250,56 @@ __device__ void scan_long_chains(const IndexWs& w, const float* __restrict__ rho
             }
             const int di = t_l - t_prev;
             const double dt = (double)di;
-            tile_t[wp][lane] = t_l;
-            for (int k = 0; k < kmax; ++k) {
-                const float rn = __shfl_sync(0xffffffffu, rho_k, k);
-                const double l2 = __shfl_sync(0xffffffffu, l2r_k, k);
-                // one step since the last occurrence: the decay is rho itself; longer gaps take the power in double
-                float A = 0.f;
-                if (live && keep) A = (di == 1) ? rn : (float)exp2(dt * l2);
-                const float A_own = A;
-                float Bv = live ? 1.0f : 0.0f;       // dead lanes carry the identity map: lane 31 ends with the last live result
-                if (!live) A = 1.0f;
+            float A[4], Bv[4], own[4], v[4];
 #pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {    // inclusive composition with the maps of the earlier lanes
-                    const float Ap = __shfl_up_sync(0xffffffffu, A, o), Bp = __shfl_up_sync(0xffffffffu, Bv, o);
-                    if (lane >= o) { Bv = fmaf(A, Bp, Bv); A *= Ap; }
+            for (int k = 0; k < 4; ++k) {
+                // one step since the last occurrence: the decay is rho itself; longer gaps take the power in double
+                const float p = (float)exp2(dt * l2r[k]);
+                own[k] = live && keep ? (di == 1 ? rho[k] : p) : 0.0f;
+                A[k] = live ? own[k] : 1.0f;         // dead lanes carry the identity map: lane 31 ends with the last live result
+                Bv[k] = live ? 1.0f : 0.0f;
+            }
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {       // inclusive composition with the maps of the earlier lanes
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const float Ap = __shfl_up_sync(0xffffffffu, A[k], o), Bp = __shfl_up_sync(0xffffffffu, Bv[k], o);
+                    if (lane >= o) { Bv[k] = fmaf(A[k], Bp, Bv[k]); A[k] *= Ap; }
                 }
-                const float U_in = __shfl_sync(0xffffffffu, car, k);
-                float Ae = __shfl_up_sync(0xffffffffu, A, 1), Be = __shfl_up_sync(0xffffffffu, Bv, 1);
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                float Ae = __shfl_up_sync(0xffffffffu, A[k], 1), Be = __shfl_up_sync(0xffffffffu, Bv[k], 1);
                 if (lane == 0) { Ae = 1.0f; Be = 0.0f; }
-                tile[wp][lane][k] = A_own * fmaf(Ae, U_in, Be);                       // v_j = A_j U_j
-                const float U_out = __shfl_sync(0xffffffffu, fmaf(A, U_in, Bv), 31);  // carried past the block
-                if (lane == k) car = U_out;
+                v[k] = own[k] * fmaf(Ae, car[k], Be);                                    // v_j = A_j U_j
+                car[k] = __shfl_sync(0xffffffffu, fmaf(A[k], car[k], Bv[k]), 31);        // carried past the block
             }
-            __syncwarp();
-            for (int idx = lane; idx < cnt * kmax; idx += 32) {
-                const int r = idx / kmax, k = idx - r * kmax;
-                out[((size_t)b * T + tile_t[wp][r]) * N + wp * nk + k] = tile[wp][r][k];
+            if (live) {
+                float* o = out + ((size_t)b * T + t_l) * N + n0;
+                if ((N & 3) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0) {
+                    *reinterpret_cast<float4*>(o) = make_float4(v[0], v[1], v[2], v[3]);
+                } else {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        if (n0 + k < N) o[k] = v[k];
+                }
             }
-            __syncwarp();
             s_ref = __shfl_sync(0xffffffffu, t_l, cnt - 1);
             has = true;
         }
     }
 }
 
-__global__ void __launch_bounds__(CHAIN_WARPS * 32)
+__global__ void __launch_bounds__(CHAIN_WARPS * 32, 4)
 k_chain_scan(IndexWs w, const float* __restrict__ rhos, const float* __restrict__ c_init,
              const int32_t* __restrict__ doc_ids, float* __restrict__ out, int T, int N, int K, int extra_decay) {
     const int b = blockIdx.y;
-    if ((int)blockIdx.x >= (int)gridDim.x - COOP_BLOCKS) {
-        scan_long_chains(w, rhos, c_init, doc_ids, out, T, N, K, extra_decay, b, (int)blockIdx.x - ((int)gridDim.x - COOP_BLOCKS));
+    const int n_long_blocks = long_chain_blocks(T);      // the first of the grid: they take longest
+    if ((int)blockIdx.x < n_long_blocks) {
+        scan_long_chains(w, rhos, c_init, doc_ids, out, T, N, K, extra_decay, b, blockIdx.x, n_long_blocks);
         return;
     }
-    const int c = blockIdx.x * CHAIN_WARPS + (threadIdx.x >> 5);
+    const int c = (blockIdx.x - n_long_blocks) * CHAIN_WARPS + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     const int nch = w.n_chain[b];
     if (c >= nch) return;
@@ -288,6 +307,7 @@ k_chain_scan(IndexWs w, const float* __restrict__ rhos, const float* __restrict_
     const int32_t* s_pos = w.s_pos + (size_t)b * T;
     const int j0 = ch_off[c];
     const int j1 = (c + 1 < nch) ? ch_off[c + 1] : T;
+    if (j1 - j0 >= LONG_CHAIN) return;      // scanned by the first blocks of the grid
     const int sd = w.seed[(size_t)b * T + j0];
 
     double l2r[4];
@@ -307,7 +327,6 @@ k_chain_scan(IndexWs w, const float* __restrict__ rhos, const float* __restrict_
     bool has = (sd != NO_SEED);
     int s_ref = 0;
     int last_doc = (doc_ids != nullptr) ? doc_ids[(size_t)b * T] : 0;
-    if (j1 - j0 >= LONG_CHAIN) return;      // scanned by the cooperative blocks at the end of the grid
     // The chain is walked 32 occurrences at a time: every lane fetches one position (and document id), the steps then
     // take them from registers with shuffles, so a long chain pays the load latency once per 32 steps, not per step.
     for (int jb = j0; jb < j1; jb += 32) {
@@ -315,120 +334,181 @@ k_chain_scan(IndexWs w, const float* __restrict__ rhos, const float* __restrict_
         const int t_l = (jj < j1) ? s_pos[jj] : 0;
         const int d_l = (doc_ids != nullptr && jj < j1) ? doc_ids[(size_t)b * T + t_l] : 0;
         const int cnt = min(32, j1 - jb);
-        for (int q = 0; q < cnt; ++q) {
-            const int t = __shfl_sync(0xffffffffu, t_l, q);
-            bool keep = has;
-            if (doc_ids != nullptr) {
-                const int d = __shfl_sync(0xffffffffu, d_l, q);
-                if (has && d != last_doc) keep = false;
-                last_doc = d;
-            }
-            const int di = t - s_ref;
-            const double dt = (double)di;
+        // the powers of AHEAD steps do not wait for one another, only the states do
+        for (int q0 = 0; q0 < cnt; q0 += AHEAD) {
+            int t[AHEAD];
+            bool keep[AHEAD];
+            float pw[AHEAD][4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                if (32 * i < N) {   // channel groups beyond N do nothing
-                    int n = lane + 32 * i;
-                    // one step since the last occurrence (runs of a repeated token, e.g. the padding): the decay is
-                    // rho itself; longer gaps take the power in double precision (its error is amplified by
-                    // 1 / (1 - rho))
-                    const float pw = (di == 1) ? rho[i] : (float)exp2(dt * l2r[i]);
-                    float cval = keep ? u[i] * pw : 0.0f;
-                    if (n < N) out[((size_t)b * T + t) * N + n] = cval;
-                    u[i] = cval + 1.0f;
+            for (int e = 0; e < AHEAD; ++e) {
+                t[e] = __shfl_sync(0xffffffffu, t_l, (q0 + e) & 31);
+                keep[e] = e > 0 || has;
+                if (doc_ids != nullptr) {
+                    const int d = __shfl_sync(0xffffffffu, d_l, (q0 + e) & 31);
+                    if (d != last_doc) keep[e] = false;
+                    last_doc = d;
+                }
+                // one step since the last occurrence (runs of a repeated token, e.g. the padding): the decay is
+                // rho itself; longer gaps take the power in double precision (its error is amplified by
+                // 1 / (1 - rho))
+                const int di = t[e] - (e > 0 ? t[e - 1] : s_ref);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    if (32 * i < N) {   // channel groups beyond N do nothing
+                        const float p = (float)exp2((double)di * l2r[i]);
+                        pw[e][i] = (di == 1) ? rho[i] : p;
+                    }
                 }
             }
-            s_ref = t;
+#pragma unroll
+            for (int e = 0; e < AHEAD; ++e) {
+                if (q0 + e >= cnt) break;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    if (32 * i < N) {
+                        const int n = lane + 32 * i;
+                        const float cval = keep[e] ? u[i] * pw[e][i] : 0.0f;
+                        if (n < N) out[((size_t)b * T + t[e]) * N + n] = cval;
+                        u[i] = cval + 1.0f;
+                    }
+                }
+            }
+            s_ref = t[AHEAD - 1];        // only read when another group of the same 32 follows
             has = true;
         }
+        s_ref = __shfl_sync(0xffffffffu, t_l, cnt - 1);
+        if (doc_ids != nullptr) last_doc = __shfl_sync(0xffffffffu, d_l, cnt - 1);
     }
 }
 
 // ----------------------------------------------------------------------------------------------
-// one warp per listed slot: state at the start of every time tile
+// one warp per listed slot (`per` of them in turn): state at the start of every time tile.  V > 0: N = 32 V, a lane holds V
+// neighbouring channels and stores them together; V = 0: any N up to 128, a lane holds channels lane, lane + 32, ...
+// dynamic smem: log2(rho) [N] in double | rho_n^(tile * 128) [nT][N] | (staged) the sorted tokens [T]
+// Bound by the bytes written (6 N a slot and tile) where slots share the table of powers, which a CTA builds once for its
+// 8 * per slots; the search for the slot's first occurrence runs over the staged tokens.  The state after an occurrence is
+// what the chain scan left for it: walking the most frequent tokens' hundreds of occurrences here took most of the time.
 // ----------------------------------------------------------------------------------------------
+static constexpr int STAGE_BYTES = 48 * 1024;
+template <int V>
 __global__ void __launch_bounds__(CHAIN_WARPS * 32)
 k_tile_states(IndexWs w, const int64_t* __restrict__ unique, const float* __restrict__ rhos,
-              const float* __restrict__ c_base, float* __restrict__ tile_state, int T, int N, int K, int nT,
-              int extra_decay) {
-    extern __shared__ float pw_sh[];            // [nT][N]: rho_n^(tile * 128), evaluated in double precision
-    for (int i = threadIdx.x; i < nT * N; i += blockDim.x)
-        pw_sh[i] = (float)exp2((double)((i / N) * MBEMA_TILE_T) * log2((double)rhos[i % N]));
+              const float* __restrict__ c_base, const float* __restrict__ tok_state, float* __restrict__ tile_state, int T,
+              int N, int K, int nT, int extra_decay, int per, int staged) {
+    constexpr int NI = V > 0 ? V : 4;
+    extern __shared__ __align__(16) double l2_sh[];
+    float* pw_sh = reinterpret_cast<float*>(l2_sh + N);        // evaluated in double precision
+    int32_t* tok_sh = reinterpret_cast<int32_t*>(pw_sh + nT * N);
+    const int b = blockIdx.y, lane = threadIdx.x & 31;
+    for (int n = threadIdx.x; n < N; n += blockDim.x) l2_sh[n] = log2((double)rhos[n]);
+    if (staged)
+        for (int i = threadIdx.x; i < T; i += blockDim.x) tok_sh[i] = w.s_tok[(size_t)b * T + i];
     __syncthreads();
-    const int b = blockIdx.y;
-    const int k = blockIdx.x * CHAIN_WARPS + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (k >= K) return;
-    const long long kv = unique[(size_t)b * K + k];
-    const int32_t* s_tok = w.s_tok + (size_t)b * T;
+    for (int i = threadIdx.x; i < nT * N; i += blockDim.x) pw_sh[i] = (float)exp2((double)((i / N) * MBEMA_TILE_T) * l2_sh[i % N]);
+    __syncthreads();
+    const int32_t* s_tok = staged ? tok_sh : w.s_tok + (size_t)b * T;
     const int32_t* s_pos = w.s_pos + (size_t)b * T;
-    float* out = tile_state + ((size_t)b * nT * K + k) * N;  // + tile * K * N
-    // the same snapshots in 16 bits follow the fp32 block (operand format of the tensor-core attention kernels:
-    // fp16 of state / 64)
-    __nv_bfloat16* out16 = reinterpret_cast<__nv_bfloat16*>(tile_state + (size_t)gridDim.y * nT * K * N) +
-                           ((size_t)b * nT * K + k) * N;
-    if (kv < 0) {
-        for (int i = 0; i < nT; ++i)
-            for (int n = lane; n < N; n += 32) {
-                out[(size_t)i * K * N + n] = 0.0f;
-                out16[(size_t)i * K * N + n] = __float2bfloat16(0.0f);   // +0 in fp16 as well
+    auto chan = [&](int i) { return V > 0 ? lane * V + i : lane + 32 * i; };
+    double l2r[NI];
+#pragma unroll
+    for (int i = 0; i < NI; ++i) l2r[i] = chan(i) < N ? l2_sh[chan(i)] : 0.0;
+    for (int p = 0; p < per; ++p) {
+        const int k = (blockIdx.x * per + p) * CHAIN_WARPS + (threadIdx.x >> 5);
+        if (k >= K) return;
+        const long long kv = unique[(size_t)b * K + k];
+        float* out = tile_state + ((size_t)b * nT * K + k) * N;  // + tile * K * N
+        // the same snapshots in 16 bits follow the fp32 block (operand format of the tensor-core attention kernels:
+        // fp16 of state / 64, saturated)
+        __half* out16 = reinterpret_cast<__half*>(tile_state + (size_t)gridDim.y * nT * K * N) + ((size_t)b * nT * K + k) * N;
+        auto put = [&](int tile, const float (&v)[NI]) {
+            __half hv[NI];
+#pragma unroll
+            for (int i = 0; i < NI; ++i) hv[i] = __float2half_rn(fminf(v[i] * (1.0f / 64.0f), 65504.0f));
+            float* o = out + (size_t)tile * K * N;
+            __half* o16 = out16 + (size_t)tile * K * N;
+            if (V == 2) {
+                *reinterpret_cast<float2*>(o + lane * 2) = make_float2(v[0], v[1]);
+                *reinterpret_cast<__half2*>(o16 + lane * 2) = __halves2half2(hv[0], hv[1]);
+            } else if (V == 4) {
+                *reinterpret_cast<float4*>(o + lane * 4) = make_float4(v[0], v[1], v[NI - 2], v[NI - 1]);
+                const __half2 lo = __halves2half2(hv[0], hv[1]), hi = __halves2half2(hv[NI - 2], hv[NI - 1]);
+                *reinterpret_cast<uint2*>(o16 + lane * 4) = make_uint2(*reinterpret_cast<const unsigned*>(&lo), *reinterpret_cast<const unsigned*>(&hi));
+            } else {
+#pragma unroll
+                for (int i = 0; i < NI; ++i)
+                    if (chan(i) < N) { o[chan(i)] = v[i]; o16[chan(i)] = hv[i]; }
             }
-        return;
-    }
-    const int key = (int)(kv & 0x7fffffff);
-    int l = 0, r = T;
-    while (l < r) {
-        int m = (l + r) >> 1;
-        if (s_tok[m] < key) l = m + 1; else r = m;
-    }
-    int j = l;
-    double l2r[4];
-    float u[4];
+        };
+        float u[NI];
+        if (kv < 0) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        int n = lane + 32 * i;
-        float rr = (n < N) ? rhos[n] : 1.0f;
-        l2r[i] = (32 * i < N) ? log2((double)rr) : 0.0;
-        u[i] = 0.0f;
-        if (c_base != nullptr && n < N) {
-            u[i] = c_base[((size_t)b * K + k) * N + n];
-            if (extra_decay) u[i] *= rr;
+            for (int i = 0; i < NI; ++i) u[i] = 0.0f;
+            for (int i = 0; i < nT; ++i) put(i, u);
+            continue;
         }
-    }
-    int s_ref = 0;
-    // occurrences are read 32 at a time (one per lane) and handed out with shuffles: `blk` is the first index of the
-    // block in registers; positions of other tokens or beyond T read as "no more occurrences"
-    int blk = -64, pos_l = 0x7fffffff;
-    auto occurrence = [&](int jx) -> int {       // step of the jx-th sorted entry if it is an occurrence of `key`, else INT_MAX
-        if (jx - blk >= 32) {
-            blk = jx;
-            const int jj = jx + lane;
-            pos_l = (jj < T && s_tok[jj] == key) ? s_pos[jj] : 0x7fffffff;
-        }
-        return __shfl_sync(0xffffffffu, pos_l, jx - blk);
-    };
-    for (int tile = 0; tile < nT; ++tile) {
-        const int t0 = tile * MBEMA_TILE_T;
-        for (int s = occurrence(j); s < t0; s = occurrence(j)) {
-            const double dt = (double)(s - s_ref);
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-                if (32 * i < N) u[i] = u[i] * (float)exp2(dt * l2r[i]) + 1.0f;
-            s_ref = s;
-            ++j;
+        for (int i = 0; i < NI; ++i) {
+            const int n = chan(i);
+            u[i] = 0.0f;
+            if (c_base != nullptr && n < N) {
+                u[i] = c_base[((size_t)b * K + k) * N + n];
+                if (extra_decay) u[i] *= rhos[n];
+            }
         }
-        const double dt = (double)(t0 - s_ref);
+        const int key = (int)(kv & 0x7fffffff);
+        int l = 0, r = T;
+        while (l < r) {
+            int m = (l + r) >> 1;
+            if (s_tok[m] < key) l = m + 1; else r = m;
+        }
+        const bool occurs = l < T && s_tok[l] == key;
+        // occurrences, 32 in registers (one per lane, `blk` the first); other tokens' read as "no more occurrences"
+        int blk = l, pos_l = 0x7fffffff;
+        auto fetch = [&]() { const int jj = blk + lane; pos_l = (jj < T && s_tok[jj] == key) ? s_pos[jj] : 0x7fffffff; };
+        if (occurs) fetch();
+        const bool first_listed = occurs && w.seed[(size_t)b * T + l] == k;
+        int s_ref = 0, j = l, known = -1;
+        for (int tile = 0; tile < nT; ++tile) {
+            const int t0 = tile * MBEMA_TILE_T;
+            if (first_listed) {
+                // the last occurrence before t0; its state stands in tok_state
+                int n, last = known;
+                while ((n = __popc(__ballot_sync(0xffffffffu, pos_l < t0))) == 32) {
+                    last = __shfl_sync(0xffffffffu, pos_l, 31);
+                    blk += 32;
+                    fetch();
+                }
+                if (n > 0) last = __shfl_sync(0xffffffffu, pos_l, n - 1);
+                if (last > known) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            int n = lane + 32 * i;
-            if (32 * i < N && n < N) {
+                    for (int i = 0; i < NI; ++i)
+                        if (chan(i) < N) u[i] = tok_state[((size_t)b * T + last) * N + chan(i)] + 1.0f;
+                    s_ref = known = last;
+                }
+            } else if (occurs) {
+                // a token listed once more: its chain belongs to the first entry, this one's state is walked
+                for (;;) {
+                    if (j - blk >= 32) { blk = j; fetch(); }
+                    const int s = __shfl_sync(0xffffffffu, pos_l, j - blk);
+                    if (s >= t0) break;
+                    const double dt = (double)(s - s_ref);
+#pragma unroll
+                    for (int i = 0; i < NI; ++i)
+                        if (V > 0 || 32 * i < N) u[i] = u[i] * (float)exp2(dt * l2r[i]) + 1.0f;
+                    s_ref = s;
+                    ++j;
+                }
+            }
+            const double dt = (double)(t0 - s_ref);
+            float v[NI];
+#pragma unroll
+            for (int i = 0; i < NI; ++i) {
+                const int n = chan(i);
+                v[i] = 0.0f;
                 // no occurrence yet: the power rho^t0 is the same for every slot of the CTA (table in shared memory)
-                const float pw = (s_ref == 0) ? pw_sh[tile * N + n] : (float)exp2(dt * l2r[i]);
-                const float v = u[i] * pw;
-                out[(size_t)tile * K * N + n] = v;
-                // operand format of the tensor-core attention kernels: fp16 of state / 64, saturated
-                reinterpret_cast<__half*>(out16)[(size_t)tile * K * N + n] = __float2half_rn(fminf(v * (1.0f / 64.0f), 65504.0f));
+                if (n < N) v[i] = u[i] * ((s_ref == 0) ? pw_sh[tile * N + n] : (float)exp2(dt * l2r[i]));
             }
+            put(tile, v);
         }
     }
 }
@@ -489,7 +569,7 @@ extern "C" int mbema_query_scan(const int64_t* x, const float* rhos, const float
     IndexWs w = carve_index_ws(workspace, B, T);
     rc = launch_sort_link(x, c_init_keys, w, B, T, c_init_keys ? K : 0, st);
     if (rc) return rc;
-    dim3 grid((unsigned)((T + CHAIN_WARPS - 1) / CHAIN_WARPS + COOP_BLOCKS), (unsigned)B);
+    dim3 grid((unsigned)((T + CHAIN_WARPS - 1) / CHAIN_WARPS + long_chain_blocks((int)T)), (unsigned)B);
     k_chain_scan<<<grid, CHAIN_WARPS * 32, 0, st>>>(w, rhos, c_init, doc_ids, C_seq, (int)T, (int)N, (int)K,
                                                     (flags & MBEMA_FLAG_CBASE_EXTRA_DECAY) ? 1 : 0);
     return check_launch();
@@ -515,15 +595,25 @@ extern "C" int mbema_tile_states(const int64_t* x, const int64_t* unique, const 
         rc = launch_sort_link(x, unique, w, B, T, K, st);
     }
     if (rc) return rc;
-    dim3 g1((unsigned)((T + CHAIN_WARPS - 1) / CHAIN_WARPS + COOP_BLOCKS), (unsigned)B);
+    dim3 g1((unsigned)((T + CHAIN_WARPS - 1) / CHAIN_WARPS + long_chain_blocks((int)T)), (unsigned)B);
     // a chain without a listed key keeps zero state in tok_state only if it is unlisted: such tokens own no slot,
     // so their rows are never read by the attention kernels; they are still written (query-scan semantics).
     k_chain_scan<<<g1, CHAIN_WARPS * 32, 0, st>>>(w, rhos, c_base, nullptr, tok_state, (int)T, (int)N, (int)K, extra);
     rc = check_launch();
     if (rc) return rc;
     const int nT = (int)((T + MBEMA_TILE_T - 1) / MBEMA_TILE_T);
-    dim3 g2((unsigned)((K + CHAIN_WARPS - 1) / CHAIN_WARPS), (unsigned)B);
-    k_tile_states<<<g2, CHAIN_WARPS * 32, (size_t)nT * N * sizeof(float), st>>>(w, unique, rhos, c_base, tile_state, (int)T, (int)N, (int)K, nT, extra);
+    // slots in turn per warp: enough to share the table of powers, not so many that fewer than two CTAs an SM are left
+    const int64_t per64 = B * K / (2 * 148 * CHAIN_WARPS);
+    const int per = (int)(per64 < 1 ? 1 : per64 > 16 ? 16 : per64);
+    size_t smem = (size_t)N * sizeof(double) + (size_t)nT * N * sizeof(float);
+    const int staged = smem + T * sizeof(int32_t) <= STAGE_BYTES ? 1 : 0;
+    if (staged) smem += T * sizeof(int32_t);
+    dim3 g2((unsigned)((K + (int64_t)CHAIN_WARPS * per - 1) / (CHAIN_WARPS * per)), (unsigned)B);
+    const bool wide = ((uintptr_t)tile_state & 15) == 0;        // N = 64, 128: the 16-bit copy then starts on 16 bytes too
+    auto go = [&](auto kernel) { kernel<<<g2, CHAIN_WARPS * 32, smem, st>>>(w, unique, rhos, c_base, tok_state, tile_state, (int)T, (int)N, (int)K, nT, extra, per, staged); };
+    if (wide && N == 64) go(k_tile_states<2>);
+    else if (wide && N == 128) go(k_tile_states<4>);
+    else go(k_tile_states<0>);
     rc = check_launch();
     if (rc) return rc;
     k_slot_order<<<(unsigned)((B + 127) / 128), 128, 0, st>>>(w.n_valid, kcount, (int)B);
@@ -568,7 +658,7 @@ extern "C" int mbema_query_scan_static(const int64_t* x, const float* rhos, cons
     IndexWs w = carve_index_ws(scratch, B, T);
     rc = launch_sort_link(x, c_init_keys, w, B, T, c_init_keys ? K : 0, st);
     if (rc) return rc;
-    dim3 grid((unsigned)((T + CHAIN_WARPS - 1) / CHAIN_WARPS + COOP_BLOCKS), (unsigned)B);
+    dim3 grid((unsigned)((T + CHAIN_WARPS - 1) / CHAIN_WARPS + long_chain_blocks((int)T)), (unsigned)B);
     k_chain_scan<<<grid, CHAIN_WARPS * 32, 0, st>>>(w, rhos, c_init, doc_ids, C_seq, (int)T, (int)N, (int)K,
                                                     (flags & MBEMA_FLAG_CBASE_EXTRA_DECAY) ? 1 : 0);
     return check_launch();
