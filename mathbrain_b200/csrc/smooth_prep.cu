@@ -14,19 +14,19 @@ __device__ __forceinline__ int sw_chunk(int r, int c8) { return r * 128 + ((c8 ^
 // ---------------------------------------------------------------------------------------------------------------
 // blocks [0, SEG_IMAGES * H * NCH): the W' image of (segment, head, column chunk): row i * 16 + dd holds
 // W[n, head * 64 + chunk * 16 + dd] rho_n^(node i of the segment), fp16, 64 x (the states carry 1/64) and, for SiLU,
-// 1/2 x (SiLU(x) = h + h tanh h, h = x / 2).  The remaining N blocks: one row of the Gram matrix each.
+// 1/2 x (SiLU(x) = h + h tanh h, h = x / 2).  The remaining N N / 8 blocks: a warp per entry of the Gram matrix (a warp for
+// eight of them, one after the other: 11 us; one each: 6.6 us).
 // ---------------------------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) k_weights(FlashArgs a, Ws w) {
     const int N = a.N, D = a.H * HD, NK = N >> 6, tid = threadIdx.x;
     const int n_img = SEG_IMAGES * a.H * NCH;
     if ((int)blockIdx.x >= n_img) {
-        const int n = blockIdx.x - n_img, lane = tid & 31;
-        for (int m = tid >> 5; m < N; m += 8) {
-            float s = 0.f;
-            for (int d = lane; d < D; d += 32) s = fmaf(a.W[(size_t)n * D + d], a.W[(size_t)m * D + d], s);
-            s = warp_sum(s);
-            if (lane == 0) w.gram[n * N + m] = s / (float)D;
-        }
+        const int pair = ((int)blockIdx.x - n_img) * 8 + (tid >> 5), n = pair / N, m = pair % N, lane = tid & 31;
+        float s = 0.f;
+#pragma unroll 4
+        for (int d = lane; d < D; d += 32) s = fmaf(a.W[(size_t)n * D + d], a.W[(size_t)m * D + d], s);
+        s = warp_sum(s);
+        if (lane == 0) w.gram[n * N + m] = s / (float)D;
         return;
     }
     const int c = blockIdx.x % NCH, h = (blockIdx.x / NCH) % a.H, img = blockIdx.x / (NCH * a.H);
@@ -265,15 +265,18 @@ __global__ void __launch_bounds__(256) k_items_fill(FlashArgs a, Items it) {
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// one CTA per (tile, sample): the levels.  |lambda . state|^2 tr(G) bounds v' G v; items whose bound could matter are
-// looked at closely, the others are not.
+// one CTA per (tile, sample): the levels.  v' G v <= |v|^2 times the largest absolute row sum of G (its largest eigenvalue is
+// no larger); items whose bound could matter are looked at closely, the others are not.  (The trace bounds it too, but
+// twenty times looser: with it a thousand items a tile were looked at, 84 us for 224 tiles.)
 // ---------------------------------------------------------------------------------------------------------------
 static constexpr int MAX_CHECKED = 1024;
+static constexpr int LV_THREADS = 1024, LV_ITEMS = 4;      // a warp looks at four items at once: one read of the Gram matrix for all
 
-__global__ void __launch_bounds__(256) k_levels(FlashArgs a, Items it, Ws w) {
+__global__ void __launch_bounds__(LV_THREADS) k_levels(FlashArgs a, Items it, Ws w) {
     __shared__ int chk[MAX_CHECKED], n_chk;
     __shared__ unsigned swing_sh[2], decay_sh;          // [0] items before the hot ones, [1] hot items
-    __shared__ float lam_sh[128], trace_sh;
+    __shared__ unsigned row_sh;
+    __shared__ float lam_sh[128];
     const int bt = blockIdx.y * a.nT + blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int N = a.N, NK = N >> 6;
     const int4 cnt = it.count[bt];
@@ -281,55 +284,70 @@ __global__ void __launch_bounds__(256) k_levels(FlashArgs a, Items it, Ws w) {
         if (tid == 0) w.level[bt] = w.level_bwd[bt] = 0;
         return;
     }
-    if (tid == 0) { n_chk = 0; swing_sh[0] = swing_sh[1] = decay_sh = 0u; }
+    if (tid == 0) { n_chk = 0; row_sh = 0u; swing_sh[0] = swing_sh[1] = decay_sh = 0u; }
     __syncthreads();
     if (tid < N) {
         const float lam = fabsf(logf(a.rhos[tid]));               // rho = 0: infinite, every step
         lam_sh[tid] = lam;
         atomicMax(&decay_sh, __float_as_uint(lam == lam ? lam : INFINITY));
     }
-    if (warp == 0) {
+    for (int n = warp; n < N; n += LV_THREADS / 32) {
         float t = 0.f;
-        for (int n = lane; n < N; n += 32) t += w.gram[n * N + n];
+        for (int m = lane; m < N; m += 32) t += fabsf(w.gram[n * N + m]);
         t = warp_sum(t);
-        if (lane == 0) trace_sh = t;
+        if (lane == 0) atomicMax(&row_sh, __float_as_uint(t));
     }
     __syncthreads();
-    const float trace = trace_sh;
-    const float look = (MAX_SWING / 64.0f) * (MAX_SWING / 64.0f) / fmaxf(trace, 1e-30f);
+    const float row_sum = __uint_as_float(row_sh);
+    const float look = (MAX_SWING / 64.0f) * (MAX_SWING / 64.0f) / fmaxf(row_sum, 1e-30f);
     const float* q = it.q + (size_t)bt * it.IB * IBLK;
-    for (int i = tid; i < cnt.w * IBLK; i += 256)
+    for (int i = tid; i < cnt.w * IBLK; i += LV_THREADS)
         if (!(q[i] <= look)) {
             const int at = atomicAdd(&n_chk, 1);
             if (at < MAX_CHECKED) chk[at] = i;
-            else atomicMax(&swing_sh[i >= cnt.y * IBLK], __float_as_uint(q[i] * trace));       // list full: the bound itself
+            else atomicMax(&swing_sh[i >= cnt.y * IBLK], __float_as_uint(q[i] * row_sum));       // list full: the bound itself
         }
     __syncthreads();
     const unsigned char* img = it.a_img + (size_t)bt * it.IB * NK * ATOM;
-    for (int j = warp; j < min(n_chk, MAX_CHECKED); j += 8) {      // a warp per item, a lane per channel
-        const int item = chk[j], r = item & (IBLK - 1);
-        float vl[4], y[4];
+    const int n_look = min(n_chk, MAX_CHECKED);
+    for (int j0 = warp * LV_ITEMS; j0 < n_look; j0 += LV_THREADS / 32 * LV_ITEMS) {      // a lane per channel
+        float vl[LV_ITEMS][4], y[LV_ITEMS][4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int n = lane + 32 * e;
-            vl[e] = y[e] = 0.f;
-            if (n < N)
-                vl[e] = __half2float(*reinterpret_cast<const __half*>(img + (size_t)(item / IBLK) * NK * ATOM + (n >> 6) * ATOM +
-                                                                      sw_chunk(r, (n >> 3) & 7) + (n & 7) * 2)) * (STATE_F16_UNSCALE * lam_sh[n]);
+        for (int g = 0; g < LV_ITEMS; ++g) {
+            const int item = chk[min(j0 + g, n_look - 1)], r = item & (IBLK - 1);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int n = lane + 32 * e;
+                vl[g][e] = y[g][e] = 0.f;
+                if (n < N)
+                    vl[g][e] = __half2float(*reinterpret_cast<const __half*>(img + (size_t)(item / IBLK) * NK * ATOM + (n >> 6) * ATOM +
+                                                                             sw_chunk(r, (n >> 3) & 7) + (n & 7) * 2)) * (STATE_F16_UNSCALE * lam_sh[n]);
+            }
         }
 #pragma unroll
         for (int e2 = 0; e2 < 4; ++e2) {
             if (32 * e2 >= N) break;
+#pragma unroll 4
             for (int l = 0; l < 32; ++l) {
-                const float vm = __shfl_sync(0xffffffffu, vl[e2], l);
                 const float* g = w.gram + (size_t)(32 * e2 + l) * N;
+                float gr[4];
 #pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    if (32 * e < N) y[e] = fmaf(vm, __ldg(g + lane + 32 * e), y[e]);
+                for (int e = 0; e < 4; ++e) gr[e] = 32 * e < N ? __ldg(g + lane + 32 * e) : 0.f;
+#pragma unroll
+                for (int i = 0; i < LV_ITEMS; ++i) {
+                    const float vm = __shfl_sync(0xffffffffu, vl[i][e2], l);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        if (32 * e < N) y[i][e] = fmaf(vm, gr[e], y[i][e]);
+                }
             }
         }
-        const float v = warp_sum(vl[0] * y[0] + vl[1] * y[1] + vl[2] * y[2] + vl[3] * y[3]);
-        if (lane == 0) atomicMax(&swing_sh[item >= cnt.y * IBLK], __float_as_uint(v >= 0.f ? v : (v < 0.f ? 0.f : INFINITY)));
+#pragma unroll
+        for (int i = 0; i < LV_ITEMS; ++i) {
+            const float v = warp_sum(vl[i][0] * y[i][0] + vl[i][1] * y[i][1] + vl[i][2] * y[i][2] + vl[i][3] * y[i][3]);
+            const int item = chk[min(j0 + i, n_look - 1)];
+            if (lane == 0) atomicMax(&swing_sh[item >= cnt.y * IBLK], __float_as_uint(v >= 0.f ? v : (v < 0.f ? 0.f : INFINITY)));
+        }
     }
     __syncthreads();
     if (tid == 0) {
@@ -354,8 +372,8 @@ int build_items(const FlashArgs& a, const Items& it, cudaStream_t st) {
 }
 
 int prepare(const FlashArgs& a, const Items& it, const Ws& w, cudaStream_t st) {
-    k_weights<<<SEG_IMAGES * a.H * NCH + a.N, 256, 0, st>>>(a, w);
-    k_levels<<<dim3(a.nT, a.B), 256, 0, st>>>(a, it, w);
+    k_weights<<<SEG_IMAGES * a.H * NCH + a.N * a.N / 8, 256, 0, st>>>(a, w);
+    k_levels<<<dim3(a.nT, a.B), LV_THREADS, 0, st>>>(a, it, w);
     return check_launch();
 }
 
