@@ -298,6 +298,8 @@ int mbema_feed_advance(const int64_t* x, const int32_t* fill, const float* C_seq
  * ---------------------------------------------------------------------------------------------- */
 int mbema_ce_rows(void* logits, int dtype, const int64_t* targets, float scale, float* loss_rows, int64_t R, int64_t V,
                   int64_t ld, void* stream);
+/* dst[i] = src[i] (add: dst[i] + src[i]): dst fp32, src bf16, n a multiple of 8, both 16-byte aligned.  Sums the chunks' dE. */
+int mbema_accumulate_bf16(float* dst, const void* src, int64_t n, int add, void* stream);
 
 /* ------------------------------------------------------------------------------------------------
  * Streaming decode with resident per-sequence slot state.  The reference has no decode loop; one step is one

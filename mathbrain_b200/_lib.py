@@ -59,6 +59,7 @@ SIGNATURES = {
     "mbema_feed_batch": (_i32, [_vp] * 9 + [_i64] * 6 + [_vp]),
     "mbema_feed_advance": (_i32, [_vp] * 9 + [_i64] * 5 + [_i32, _vp]),
     "mbema_ce_rows": (_i32, [_vp, _i32, _vp, _f32, _vp, _i64, _i64, _i64, _vp]),
+    "mbema_accumulate_bf16": (_i32, [_vp, _vp, _i64, _i32, _vp]),
     "mbema_slot_grad_scatter": (_i32, [_vp, _vp, _i32, _vp, _vp, _i64, _i64, _i64, _vp]),
 }
 

@@ -34,7 +34,8 @@ class LMHeadCrossEntropy(torch.autograd.Function):
             valid = (targets != ignore_index).nonzero(as_tuple=True)[0]          # positions that count
             n = int(valid.numel())                                              # one host synchronisation per step
             dh = torch.zeros(R, D, dtype=torch.float32, device=h.device)
-            dE = torch.zeros(ld, D, dtype=torch.float32, device=h.device)
+            own_sum = cdt == torch.bfloat16 and n > 0                           # the chunks' dE are summed by mbema_accumulate_bf16
+            dE = (torch.empty if own_sum else torch.zeros)(ld, D, dtype=torch.float32, device=h.device)
             loss = torch.zeros((), dtype=torch.float32, device=h.device)
             if n:
                 Ep = torch.zeros(ld, D, dtype=cdt, device=h.device)             # rows [V, ld) stay zero
@@ -52,10 +53,12 @@ class LMHeadCrossEntropy(torch.autograd.Function):
                                            hi - lo, V, ld, _stream())
                     _lib.check(rc, "mbema_ce_rows")
                     dh.index_copy_(0, valid[lo:hi], torch.mm(logits, Ep).float())
-                    if cdt == torch.float32:
-                        dE.addmm_(logits.t(), hv[lo:hi])
+                    if own_sum:
+                        part = torch.mm(logits.t(), hv[lo:hi])
+                        rc = lib.mbema_accumulate_bf16(_ptr(dE), _ptr(part), dE.numel(), 1 if lo else 0, _stream())
+                        _lib.check(rc, "mbema_accumulate_bf16")
                     else:
-                        dE.add_(torch.mm(logits.t(), hv[lo:hi]).float())
+                        dE.addmm_(logits.t(), hv[lo:hi])
                 loss = loss_rows.sum() / n
         ctx.save_for_backward(dh.to(h.dtype), dE[:V].to(E.dtype))
         return loss
