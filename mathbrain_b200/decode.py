@@ -74,9 +74,12 @@ class DecodeState:
 
     def attend(self, q, E_k, E_v, W_pe, t_now, V_total=None, use_silu=True, listed_only=False, mode=None):
         """O [B, H, 64] float32; see _attend.  Runs with the state's device current and refuses operands elsewhere."""
+        dev = self.state.get_device()
         for t in (q, E_k, E_v, W_pe):
-            if t.device != self.state.device:
+            if t.get_device() != dev:
                 raise _lib.MbemaError("decode: operand on %s, state on %s" % (t.device, self.state.device))
+        if dev == torch.cuda.current_device():
+            return self._attend(q, E_k, E_v, W_pe, t_now, V_total, use_silu, listed_only, mode)
         with torch.cuda.device(self.state.device):
             return self._attend(q, E_k, E_v, W_pe, t_now, V_total, use_silu, listed_only, mode)
 
@@ -126,6 +129,8 @@ class DecodeState:
         """C_q [B, N]; see _update.  Runs with the state's device current and refuses a token tensor elsewhere."""
         if tok.device != self.state.device:
             raise _lib.MbemaError("decode: tokens on %s, state on %s" % (tok.device, self.state.device))
+        if tok.get_device() == torch.cuda.current_device():
+            return self._update(tok, t_now)
         with torch.cuda.device(self.state.device):
             return self._update(tok, t_now)
 

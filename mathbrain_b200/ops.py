@@ -82,7 +82,7 @@ def options(**kw):
 # ---------------------------------------------------------------------------------------------
 def _require_cuda(*tensors):
     for t in tensors:
-        if t is not None and t.device.type != "cuda":
+        if t is not None and not t.is_cuda:
             raise _lib.MbemaError("mathbrain_b200 operators need CUDA tensors (got %s); there is no CPU path"
                                   % t.device)
 
@@ -96,15 +96,16 @@ def _on_tensor_device(fn):
     current stream while the buffers live where the tensors are); tensors on different devices are refused."""
     @functools.wraps(fn)
     def wrapper(*args, **kw):
-        dev = None
-        for a in list(args) + list(kw.values()):
+        dev = -1
+        for a in (*args, *kw.values()) if kw else args:
             t = a.tile_state if isinstance(a, TileStates) else a
-            if torch.is_tensor(t) and t.device.type == "cuda":
-                if dev is None:
-                    dev = t.device
-                elif t.device != dev:
-                    raise _lib.MbemaError("operands live on different devices (%s and %s)" % (dev, t.device))
-        if dev is None or dev.index == torch.cuda.current_device():
+            if isinstance(t, torch.Tensor) and t.is_cuda:
+                i = t.get_device()
+                if dev < 0:
+                    dev = i
+                elif i != dev:
+                    raise _lib.MbemaError("operands live on different devices (cuda:%d and cuda:%d)" % (dev, i))
+        if dev < 0 or dev == torch.cuda.current_device():
             return fn(*args, **kw)
         with torch.cuda.device(dev):
             return fn(*args, **kw)
@@ -123,8 +124,13 @@ def _f32_or_bf16(t):
     return t if t.dtype in (torch.float32, torch.bfloat16) else t.float()
 
 
+# Raw handle of a device's current stream: torch.cuda.current_stream() builds a Stream object, 4 us a call, several times
+# what the launch itself costs the host.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda index: torch.cuda.current_stream(index).cuda_stream)
+
+
 def _stream():
-    return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(torch.cuda.current_device())
 
 
 def _workspace(nbytes, device):
@@ -177,8 +183,8 @@ _tc_workspaces = {}
 
 
 def _tc_workspace(nbytes, device):
-    key = (device.index if device.index is not None else torch.cuda.current_device(),
-           torch.cuda.current_stream(device).cuda_stream)
+    index = device.index if device.index is not None else torch.cuda.current_device()
+    key = (index, _raw_stream(index))
     ws = _tc_workspaces.get(key)
     if ws is None or ws.numel() < nbytes:
         new = torch.zeros(max(int(nbytes), 4096), dtype=torch.uint8, device=device)
@@ -236,7 +242,7 @@ _index_cache = {"key": None, "ws": None, "x": None}     # "x" keeps the tensor a
 
 
 def _index_key(x):
-    return (x.data_ptr(), x._version, tuple(x.shape), x.device.index, torch.cuda.current_stream(x.device).cuda_stream)
+    return (x.data_ptr(), x._version, tuple(x.shape), x.device.index, _raw_stream(x.device.index))
 
 
 # ---------------------------------------------------------------------------------------------
