@@ -6,11 +6,14 @@
 //     S     [128 steps x 128] += Q'_c . K_c^T       K_c = E_k c_j, written by the gate warps
 //     O'_c  [128 steps x 64]  += P . V_c            P from tensor memory, V_c = E_v c_j
 // Warps: two gate warpgroups (a thread per item; half of a chunk's columns each), two softmax warpgroups (a thread per
-// step and half a block's items), one loader (bulk copies of A and W' images), one lane issuing the gate products and
-// one issuing S and P.V, so that neither waits for the other's operands.  All hand-offs are mbarriers with bounded waits.
+// step and half a block's items), one loader (bulk copies of A and W' images), and a lane each for the gate products, S
+// and P.V, so that none waits for another's operands.  All hand-offs are mbarriers with bounded waits.
 //
-// Bound: special functions and issue slots, not the tensor cores.  A block takes 4 * 64 tanh per item and one exponential
-// per item and step (3072 cycles of the special-function pipe at 16 a clock), 2560 cycles of tensor work.
+// The gate warps are the longest stage (some 1450 cycles a chunk, 5800 a block: 4 * 64 tanh an item and their coefficients), so
+// everything else is laid out to run beside them: scores and P have tensor memory of their own (the next block's S starts while P.V
+// reads P; the gate product has one accumulator, read at once), and V has six chunks (five for 128 channels, where the states take
+// the room) of which the gate runs two ahead of P.V.  With P over S and four V chunks a block took S, softmax, P.V and gate one
+// after the other: 1.05 ms a layer at B=56, T=512, N=64, 0.86 ms so; 1.14 and 1.03 ms at B=8, T=4096, N=128.
 #include "smooth.cuh"
 #include "smooth_dev.cuh"
 
@@ -22,37 +25,43 @@ using namespace ptx;
 namespace fwd {
 
 static constexpr int GATE_WARPS = 8, SM_WARPS = 8;
-static constexpr int W_LOAD = 16, W_GATE = 17, W_ATT = 18;       // warp 19 only fills the warpgroup
+static constexpr int W_LOAD = 16, W_GATE = 17, W_SCORE = 18, W_PV = 19;
 static constexpr int THREADS = 20 * 32;      // launched with 96 registers a thread: 61440 = 4 * 128 * 104 + 128 * 64
-static constexpr uint32_t T_O = 0, T_S = 256, T_PRE = 384;     // tensor-memory columns
+static constexpr uint32_t T_O = 0, T_S = 256, T_P = 384, T_PRE = 448;     // tensor-memory columns
 static constexpr float RESCALE = 8.0f;      // log2 units the softmax reference may lag behind (P <= 2^8 in fp16)
 
 struct Bars {
-    uint64_t a_full[2], a_free[2], w_full[2], w_free[2], pre_full[2], pre_empty[2], kv_full[NCH], k_free[2], v_free[NCH];
-    uint64_t s_full, p_full, mx_full, o_full, drain;
+    uint64_t a_full, a_free, w_full[2], w_free[2], pre_full, pre_empty, kv_full[NCH], k_free[2], v_free[6];
+    uint64_t s_full, s_free, p_full, mx_full, v_full, pv_done, o_full, drain;
     uint32_t tmem_base;
     int abort_flag, drain_flag;
     unsigned spin_limit;
 };
 
-static constexpr int Q_OFF = 0, A_OFF = Q_OFF + NCH * ATOM, W_OFF = A_OFF + 2 * ATOM, K_OFF = W_OFF + 2 * WPIECE, V_OFF = K_OFF + 2 * ATOM,
-                     MX_OFF = V_OFF + NCH * ATOM, BAR_OFF = MX_OFF + 4 * TM * 4, SMEM = BAR_OFF + 512 + 1024;
-static_assert(sizeof(Bars) <= 512 && SMEM <= 227 * 1024, "shared memory");
+template <int NK> struct L {
+    static constexpr int NV = NK == 1 ? 6 : 5;          // V chunks in flight
+    static constexpr int Q = 0, A = Q + NCH * ATOM, W = A + NK * ATOM, K = W + 2 * WPIECE, V = K + 2 * ATOM, MX = V + NV * ATOM,
+                         BAR = MX + 4 * TM * 4, SMEM = BAR + 512;
+    static_assert(sizeof(Bars) <= 512 && SMEM <= 227 * 1024, "shared memory");
+};
 
 template <bool SILU, int NK, bool EF32>
 __global__ void __launch_bounds__(THREADS, 1) k_smooth_fwd(FlashArgs a, Items it, Ws w, int* status) {
-    extern __shared__ unsigned char smem_raw[];
-    unsigned char* sm = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-    Bars* bars = reinterpret_cast<Bars*>(sm + BAR_OFF);
-    float* mx_sh = reinterpret_cast<float*>(sm + MX_OFF);
+    extern __shared__ __align__(1024) unsigned char sm[];
+    using M = L<NK>;
+    Bars* bars = reinterpret_cast<Bars*>(sm + M::BAR);
+    float* mx_sh = reinterpret_cast<float*>(sm + M::MX);
     volatile int* abort_flag = &bars->abort_flag;
-    constexpr int NA = NK == 1 ? 2 : 1;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int tile = blockIdx.x, h = blockIdx.y, b = a.order ? a.order[blockIdx.z] : (int)blockIdx.z;
     const int bt = b * a.nT + tile, t0 = tile * TM, D = a.H * HD;
     const int Lb = a.seq_lens ? min(max(a.seq_lens[b], 0), a.T) : a.T;
     const int level = w.level[bt];
     if (level == LEVEL_EXACT) return;
+    if (smem_u32(sm) & 1023u) {        // the swizzled tiles need it; there is no room to align by hand
+        if (tid == 0) atomicOr(status, 1 | (31 << 8));
+        return;
+    }
     const size_t row0 = ((size_t)b * a.H + h) * a.T + t0;
     if (t0 >= Lb) {          // a tile beyond the valid length
         for (int i = tid; i < min(TM, a.T - t0) * (HD / 4); i += THREADS)
@@ -61,15 +70,14 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_fwd(FlashArgs a, Items it
         return;
     }
     if (tid == 0) {
-        for (int i = 0; i < 2; ++i) {
-            mbar_init(&bars->a_full[i], 1); mbar_init(&bars->a_free[i], 1);
-            mbar_init(&bars->w_full[i], 1); mbar_init(&bars->w_free[i], 1);
-            mbar_init(&bars->pre_full[i], 1); mbar_init(&bars->pre_empty[i], GATE_WARPS);
-            mbar_init(&bars->k_free[i], 1);
-        }
-        for (int i = 0; i < NCH; ++i) { mbar_init(&bars->kv_full[i], GATE_WARPS); mbar_init(&bars->v_free[i], 1); }
-        mbar_init(&bars->s_full, 1); mbar_init(&bars->p_full, SM_WARPS); mbar_init(&bars->mx_full, SM_WARPS);
-        mbar_init(&bars->o_full, 1); mbar_init(&bars->drain, 2);
+        mbar_init(&bars->a_full, 1); mbar_init(&bars->a_free, 1);
+        mbar_init(&bars->pre_full, 1); mbar_init(&bars->pre_empty, GATE_WARPS);
+        for (int i = 0; i < 2; ++i) { mbar_init(&bars->w_full[i], 1); mbar_init(&bars->w_free[i], 1); mbar_init(&bars->k_free[i], 1); }
+        for (int i = 0; i < NCH; ++i) mbar_init(&bars->kv_full[i], GATE_WARPS);
+        for (int i = 0; i < M::NV; ++i) mbar_init(&bars->v_free[i], 1);
+        mbar_init(&bars->s_full, 1); mbar_init(&bars->s_free, SM_WARPS); mbar_init(&bars->p_full, SM_WARPS);
+        mbar_init(&bars->mx_full, SM_WARPS); mbar_init(&bars->v_full, 1); mbar_init(&bars->pv_done, 1);
+        mbar_init(&bars->o_full, 1); mbar_init(&bars->drain, 3);
         bars->abort_flag = *reinterpret_cast<volatile int*>(status);      // an earlier CTA gave up: do nothing
         bars->drain_flag = 0;
         bars->spin_limit = a.test_withhold ? 64u : MBEMA_SPIN_LIMIT;
@@ -89,7 +97,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_fwd(FlashArgs a, Items it
             const float4 v = t0 + t < Lb ? ld4_dyn_f32(a.Q, a.q_dt, (row0 + t) * HD + c * 16 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
             q[i] = v.x; q[i + 1] = v.y; q[i + 2] = v.z; q[i + 3] = v.w;
         }
-        store_basis_rows(sm + Q_OFF + c * ATOM, t, q, beta, 0.125f * 1.4426950409f);
+        store_basis_rows(sm + M::Q + c * ATOM, t, q, beta, 0.125f * 1.4426950409f);
     }
     fence_proxy_async_smem();
     tc_fence_before_sync();
@@ -126,28 +134,29 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_fwd(FlashArgs a, Items it
                     nk = load_e<EF32>(a.Ek, off);
                     nv = load_e<EF32>(a.Ev, off);
                 }
-                const int st = c & 1, use = 2 * i + (c >> 1);
-                if (!(alive = warp_wait(&bars->pre_full[st], (uint32_t)(use & 1), abort_flag, 1, lim))) break;
+                const int st = c & 1, use = 2 * i + (c >> 1), n = 4 * i + c;
+                if (!(alive = warp_wait(&bars->pre_full, (uint32_t)(n & 1), abort_flag, 1, lim))) break;
                 tc_fence_after_sync();
                 float x[NJ][8];
 #pragma unroll
-                for (int j = 0; j < NJ; ++j) tmem_ld_32x32b_x8(t_pre + st * 64 + j * 16, x[j]);
+                for (int j = 0; j < NJ; ++j) tmem_ld_32x32b_x8(t_pre + j * 16, x[j]);
                 tmem_wait_ld();
                 tc_fence_before_sync();
                 __syncwarp();
-                if (lane == 0 && !(a.test_withhold && use == 0)) mbar_arrive(&bars->pre_empty[st]);
+                if (lane == 0 && !(a.test_withhold && n == 0)) mbar_arrive(&bars->pre_empty);
                 uint32_t cf[NJ][4], none[1][4];
                 gate_coefficients<SILU, false>(x, cf, none);
                 if (use >= 1 && !(alive = warp_wait(&bars->k_free[st], (uint32_t)((use - 1) & 1), abort_flag, 2, lim))) break;
-                unsigned char* kd = sm + K_OFF + st * ATOM + r * 128;
+                unsigned char* kd = sm + M::K + st * ATOM + r * 128;
                 uint32_t e2[4], f2[4];
 #pragma unroll
                 for (int p = 0; p < 4; ++p) { e2[p] = e_pair<EF32>(ek, p); f2[p] = e_pair<EF32>(ev, p); }
 #pragma unroll
                 for (int j = 0; j < NJ; ++j)
                     st_shared_v4(kd + (((2 * j + wg) ^ x7) << 4), mul_f16x2(cf[j][0], e2[0]), mul_f16x2(cf[j][1], e2[1]), mul_f16x2(cf[j][2], e2[2]), mul_f16x2(cf[j][3], e2[3]));
-                if (i >= 1 && !(alive = warp_wait(&bars->v_free[c], (uint32_t)((i - 1) & 1), abort_flag, 3, lim))) break;
-                unsigned char* vd = sm + V_OFF + c * ATOM + r * 128;
+                const int vb = n % M::NV;
+                if (n >= M::NV && !(alive = warp_wait(&bars->v_free[vb], (uint32_t)((n / M::NV - 1) & 1), abort_flag, 3, lim))) break;
+                unsigned char* vd = sm + M::V + vb * ATOM + r * 128;
 #pragma unroll
                 for (int j = 0; j < NJ; ++j)
                     st_shared_v4(vd + (((2 * j + wg) ^ x7) << 4), mul_f16x2(cf[j][0], f2[0]), mul_f16x2(cf[j][1], f2[1]), mul_f16x2(cf[j][2], f2[2]), mul_f16x2(cf[j][3], f2[3]));
@@ -180,6 +189,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_fwd(FlashArgs a, Items it
             tmem_ld_32x32b_x32(t_row + T_S + half * 64, s);
             tmem_ld_32x32b_x32(t_row + T_S + half * 64 + 32, s + 32);
             tmem_wait_ld();
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars->s_free);          // the next block's scores may be written
             if (!__all_sync(0xffffffffu, (mcur.x & mcur.y) == 0xffffffffu)) {
 #pragma unroll
                 for (int k = 0; k < 32; ++k) {
@@ -198,13 +210,16 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_fwd(FlashArgs a, Items it
             __syncwarp();
             if (lane == 0) mbar_arrive(&bars->mx_full);
             if (!(alive = warp_wait(&bars->mx_full, (uint32_t)(i & 1), abort_flag, 5, lim))) break;
+            // the products of the block before have read P and left O'
+            if (i >= 1 && !(alive = warp_wait(&bars->pv_done, (uint32_t)((i - 1) & 1), abort_flag, 17, lim))) break;
+            tc_fence_after_sync();
             const float mb = fmaxf(fmaxf(b0, b1), mx[(half ^ 1) * TM + row]);
             const bool up = mb > m + RESCALE;
             if (__any_sync(0xffffffffu, up)) {
                 const float al = up ? ex2_approx(m - mb) : 1.0f;       // m = -inf: 0
                 l *= al;
                 if (up) m = mb;
-                if (i > 0) {       // this half's columns of O' (the products of the earlier blocks completed before S did)
+                if (i > 0) {       // this half's columns of O'
 #pragma unroll 1
                     for (int k = 0; k < 128; k += 16) {
                         float o[16];
@@ -218,7 +233,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_fwd(FlashArgs a, Items it
             }
             const float mm = m == -INFINITY ? 0.f : m;
             float l0 = 0.f, l1 = 0.f;
-            // P as fp16 pairs over the half's own score columns (all of them are in registers by now)
+            // P as fp16 pairs
 #pragma unroll
             for (int k = 0; k < 64; k += 16) {
                 uint32_t p2[8];
@@ -228,7 +243,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_fwd(FlashArgs a, Items it
                     l0 += p; l1 += q;
                     p2[e] = pack_f16x2(p, q);
                 }
-                tmem_st_x8(t_row + T_S + half * 64 + k / 2, p2);
+                tmem_st_x8(t_row + T_P + half * 32 + k / 2, p2);
             }
             l += l0 + l1;
             tmem_wait_st();
@@ -287,59 +302,57 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_fwd(FlashArgs a, Items it
         if (warp == W_LOAD && lane == 0) {
             // ==================================================== loader
             const unsigned char* img = it.a_img + (size_t)bt * it.IB * NK * ATOM;
-            int np = 0;
+            int np = 0, na = 0;
             bool alive = true;
             for (int i = 0; i < n_it && alive; ++i) {
                 const int seg = i / n_blk, blk = i - seg * n_blk;
                 const unsigned char* wi = w.w_img + (size_t)((((1 << level) - 1 + seg) * a.H + h) * NCH) * NK * WPIECE;
-                const int sa = i % NA, ua = i / NA;
-                if (ua >= 1 && !(alive = mbar_wait(&bars->a_free[sa], (uint32_t)((ua - 1) & 1), abort_flag, 8, lim))) break;
-                mbar_expect_tx(&bars->a_full[sa], NK * ATOM);
-                bulk_load(sm + A_OFF + sa * ATOM, img + (size_t)blk * NK * ATOM, NK * ATOM, &bars->a_full[sa]);
+                if (i >= 1 && !(alive = mbar_wait(&bars->a_free, (uint32_t)((i - 1) & 1), abort_flag, 8, lim))) break;
+                mbar_expect_tx(&bars->a_full, NK * ATOM);
+                bulk_load(sm + M::A, img + (size_t)blk * NK * ATOM, NK * ATOM, &bars->a_full);
+                ++na;
                 for (int p = 0; p < NCH * NK; ++p, ++np) {
                     const int sw = np & 1, uw = np >> 1;
                     if (uw >= 1 && !(alive = mbar_wait(&bars->w_free[sw], (uint32_t)((uw - 1) & 1), abort_flag, 9, lim))) break;
                     mbar_expect_tx(&bars->w_full[sw], WPIECE);
-                    bulk_load(sm + W_OFF + sw * WPIECE, wi + (size_t)p * WPIECE, WPIECE, &bars->w_full[sw]);
+                    bulk_load(sm + M::W + sw * WPIECE, wi + (size_t)p * WPIECE, WPIECE, &bars->w_full[sw]);
                 }
-                if (!alive) mbar_wait<100>(&bars->a_full[sa], (uint32_t)(ua & 1), &bars->drain_flag, 10);
             }
-            // no copy of this CTA is in flight when it ends (the last A tile landed before its products could be issued)
+            // no copy of this CTA is in flight when it ends
+            if (na > 0) mbar_wait<100>(&bars->a_full, (uint32_t)((na - 1) & 1), &bars->drain_flag, 10);
             for (int s = 0; s < 2; ++s)
                 if (np > s) mbar_wait<100>(&bars->w_full[s], (uint32_t)(((np - 1 - s) >> 1) & 1), &bars->drain_flag, 10);
-            for (int i = max(0, n_it - NA); i < n_it && alive; ++i)
-                mbar_wait<100>(&bars->a_full[i % NA], (uint32_t)((i / NA) & 1), &bars->drain_flag, 10);
         } else if (warp == W_GATE && lane == 0) {
             // ==================================================== gate products
             const uint32_t idesc = umma_idesc_16(IBLK, 64, 0, 0, 0, 0);
             int np = 0;
             bool alive = true;
             for (int i = 0; i < n_it && alive; ++i) {
-                const int sa = i % NA;
-                if (!(alive = mbar_wait(&bars->a_full[sa], (uint32_t)((i / NA) & 1), abort_flag, 11, lim))) break;
+                if (!(alive = mbar_wait(&bars->a_full, (uint32_t)(i & 1), abort_flag, 11, lim))) break;
                 for (int c = 0; c < NCH && alive; ++c) {
-                    const int use = 2 * i + (c >> 1);
-                    if (use >= 1 && !(alive = mbar_wait(&bars->pre_empty[c & 1], (uint32_t)((use - 1) & 1), abort_flag, 12, lim))) break;
+                    const int n = 4 * i + c;
+                    if (n >= 1 && !(alive = mbar_wait(&bars->pre_empty, (uint32_t)((n - 1) & 1), abort_flag, 12, lim))) break;
                     for (int p = 0; p < NK; ++p, ++np) {
                         if (!(alive = mbar_wait(&bars->w_full[np & 1], (uint32_t)((np >> 1) & 1), abort_flag, 13, lim))) break;
                         tc_fence_after_sync();
-                        const uint32_t ab = smem_u32(sm + A_OFF + (sa + p) * ATOM), wb = smem_u32(sm + W_OFF + (np & 1) * WPIECE);
+                        const uint32_t ab = smem_u32(sm + M::A + p * ATOM), wb = smem_u32(sm + M::W + (np & 1) * WPIECE);
 #pragma unroll
                         for (int k = 0; k < 4; ++k)
-                            umma_bf16_ss(tmem + T_PRE + (c & 1) * 64, umma_desc_k_sw128(ab + k * 32), umma_desc_k_sw128(wb + k * 32), idesc, (p | k) != 0);
+                            umma_bf16_ss(tmem + T_PRE, umma_desc_k_sw128(ab + k * 32), umma_desc_k_sw128(wb + k * 32), idesc, (p | k) != 0);
                         umma_commit(&bars->w_free[np & 1]);
                     }
-                    if (alive) umma_commit(&bars->pre_full[c & 1]);
+                    if (alive) umma_commit(&bars->pre_full);
                 }
-                if (alive) umma_commit(&bars->a_free[sa]);
+                if (alive) umma_commit(&bars->a_free);
             }
             umma_commit(&bars->drain);
-        } else if (warp == W_ATT && lane == 0) {
-            // ==================================================== S and P.V
-            const uint32_t id_s = umma_idesc_16(TM, IBLK, 0, 0, 0, 0), id_o = umma_idesc_16(TM, 64, 0, 1, 0, 0);
-            const uint32_t qb = smem_u32(sm + Q_OFF), kb = smem_u32(sm + K_OFF), vb = smem_u32(sm + V_OFF);
+        } else if (warp == W_SCORE && lane == 0) {
+            // ==================================================== S
+            const uint32_t id_s = umma_idesc_16(TM, IBLK, 0, 0, 0, 0);
+            const uint32_t qb = smem_u32(sm + M::Q), kb = smem_u32(sm + M::K);
             bool alive = true;
             for (int i = 0; i < n_it && alive; ++i) {
+                if (i >= 1 && !(alive = mbar_wait(&bars->s_free, (uint32_t)((i - 1) & 1), abort_flag, 18, lim))) break;
                 for (int c = 0; c < NCH; ++c) {
                     if (!(alive = mbar_wait(&bars->kv_full[c], (uint32_t)(i & 1), abort_flag, 14, lim))) break;
                     tc_fence_after_sync();
@@ -349,16 +362,26 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_fwd(FlashArgs a, Items it
                     umma_commit(&bars->k_free[c & 1]);
                 }
                 if (!alive) break;
+                mbar_arrive(&bars->v_full);          // the block's V chunks, seen here on kv_full, for the lane that reads them
                 umma_commit(&bars->s_full);
+            }
+            umma_commit(&bars->drain);
+        } else if (warp == W_PV && lane == 0) {
+            // ==================================================== P.V
+            const uint32_t id_o = umma_idesc_16(TM, 64, 0, 1, 0, 0), vb = smem_u32(sm + M::V);
+            bool alive = true;
+            for (int i = 0; i < n_it && alive; ++i) {
+                if (!(alive = mbar_wait(&bars->v_full, (uint32_t)(i & 1), abort_flag, 19, lim))) break;
                 if (!(alive = mbar_wait(&bars->p_full, (uint32_t)(i & 1), abort_flag, 15, lim))) break;
                 tc_fence_after_sync();
                 for (int c = 0; c < NCH; ++c) {
+                    const int slot = (4 * i + c) % M::NV;
 #pragma unroll
                     for (int k = 0; k < 8; ++k)
-                        umma_16_ts(tmem + T_O + c * 64, tmem + T_S + (k < 4 ? k * 8 : 64 + (k - 4) * 8),
-                                   umma_desc_mn_sw128(vb + c * ATOM + k * 2048, ATOM, 1024), id_o, (i | k) != 0);
-                    umma_commit(&bars->v_free[c]);
+                        umma_16_ts(tmem + T_O + c * 64, tmem + T_P + k * 8, umma_desc_mn_sw128(vb + slot * ATOM + k * 2048, ATOM, 1024), id_o, (i | k) != 0);
+                    umma_commit(&bars->v_free[slot]);
                 }
+                umma_commit(&bars->pv_done);
             }
             umma_commit(&bars->o_full);
             umma_commit(&bars->drain);
@@ -381,8 +404,8 @@ int forward(const FlashArgs& a, const Items& it, const Ws& w, int* status, cudaS
     const dim3 grid(a.nT, a.H, a.B);
 #define MBEMA_SMOOTH(S_, NK_, E_)                                                                                             \
     do {                                                                                                                       \
-        MBEMA_CUDA_TRY(cudaFuncSetAttribute(fwd::k_smooth_fwd<S_, NK_, E_>, cudaFuncAttributeMaxDynamicSharedMemorySize, fwd::SMEM)); \
-        fwd::k_smooth_fwd<S_, NK_, E_><<<grid, fwd::THREADS, fwd::SMEM, st>>>(a, it, w, status);                                    \
+        MBEMA_CUDA_TRY(cudaFuncSetAttribute(fwd::k_smooth_fwd<S_, NK_, E_>, cudaFuncAttributeMaxDynamicSharedMemorySize, fwd::L<NK_>::SMEM)); \
+        fwd::k_smooth_fwd<S_, NK_, E_><<<grid, fwd::THREADS, fwd::L<NK_>::SMEM, st>>>(a, it, w, status);                                    \
     } while (0)
 #define MBEMA_SMOOTH_E(S_, NK_) do { if (a.e_dt == MBEMA_F32) MBEMA_SMOOTH(S_, NK_, true); else MBEMA_SMOOTH(S_, NK_, false); } while (0)
     if (a.N == 64) { if (a.silu) MBEMA_SMOOTH_E(true, 1); else MBEMA_SMOOTH_E(false, 1); }
