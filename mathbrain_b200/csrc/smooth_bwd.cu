@@ -7,6 +7,8 @@
 //                  dE_k, dE_v, and the gate's node gradients dpre from them; dW += A^T . (sum_i dpre_i, sum_i theta_i dpre_i)
 // W_pe's gradient takes the node powers rho^tau_i as a0 + a1 theta_i (two products instead of four): the part left out is
 // (lambda * half tile)^2 / 4 <= 5e-4 of the fastest channel (MAX_DECAY_BWD), a rounding of the fp16 operand.
+// Its products take two chunks at once (64 columns): products of 32 cost the tensor pipe as much, 2.40 ms a layer at B=56, T=512,
+// N=64 against 2.34.
 //
 // Two gate warpgroups (a thread per item, half of a chunk's columns each), two step warpgroups (softmax: a thread per item and half
 // the steps; then a thread per step for dQ), a loader lane and two issuing lanes.  Registers and tensor memory hold all
@@ -33,7 +35,7 @@ static constexpr float LN2 = 0.6931471806f;
 struct Bars {
     uint64_t a_full, w_full[2], w_free[2], do_full[2], do_free[2];
     uint64_t pre1_full[2], pre2_full[2], pre_empty[2], kv_full[2], kv_free[2], sdp_full, s_read, pds_full;
-    uint64_t dkv_full[2], dkv_empty, kg_full[2], kg_free[2], dq_full[2], dq_empty, dpre_full[2], dp_free[2], blk_done, flushed, drain;
+    uint64_t dkv_full[2], dkv_empty, kg_full[2], kg_free[2], dq_full[2], dq_empty, dpre_full[2], dp_free, blk_done, flushed, drain;
     uint32_t tmem_base;
     int abort_flag, drain_flag;
     unsigned spin_limit, dmax, pmax;
@@ -87,11 +89,11 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
             mbar_init(&bars->pre1_full[i], 1); mbar_init(&bars->pre2_full[i], 1); mbar_init(&bars->pre_empty[i], GATE_WARPS);
             mbar_init(&bars->kv_full[i], GATE_WARPS); mbar_init(&bars->kv_free[i], 1);
             mbar_init(&bars->dkv_full[i], 1); mbar_init(&bars->kg_full[i], GATE_WARPS); mbar_init(&bars->kg_free[i], 1);
-            mbar_init(&bars->dq_full[i], 1); mbar_init(&bars->dpre_full[i], GATE_WARPS); mbar_init(&bars->dp_free[i], 1);
+            mbar_init(&bars->dq_full[i], 1); mbar_init(&bars->dpre_full[i], GATE_WARPS);
         }
         mbar_init(&bars->sdp_full, 1); mbar_init(&bars->s_read, SM_WARPS); mbar_init(&bars->pds_full, SM_WARPS);
         mbar_init(&bars->dkv_empty, GATE_WARPS); mbar_init(&bars->dq_empty, 4);
-        mbar_init(&bars->blk_done, 1); mbar_init(&bars->flushed, GATE_WARPS); mbar_init(&bars->drain, 2);
+        mbar_init(&bars->dp_free, 1); mbar_init(&bars->blk_done, 1); mbar_init(&bars->flushed, GATE_WARPS); mbar_init(&bars->drain, 2);
         bars->abort_flag = *reinterpret_cast<volatile int*>(status);
         bars->drain_flag = 0;
         bars->spin_limit = a.test_withhold ? 64u : MBEMA_SPIN_LIMIT;
@@ -319,11 +321,11 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
                         red_v4(gv + q * 4, ovv[0] * ov, ovv[1] * ov, ovv[2] * ov, ovv[3] * ov);
                     }
                 }
-                // the tile of the moments: free once the dW product before has read it
-                if (c >= 1 && !(alive = warp_wait(&bars->dp_free[(c - 1) & 1], (uint32_t)((2 * i + ((c - 1) >> 1)) & 1), abort_flag, 7, lim))) break;
+                // the tile of the moments takes two chunks: free once the dW product of the first two has read it
+                if (c == 2 && !(alive = warp_wait(&bars->dp_free, (uint32_t)(i & 1), abort_flag, 7, lim))) break;
                 unsigned char* zd = sm + M::B1 + r * 128;
-                st_shared_v4(zd + ((wg ^ x7) << 4), m0[0], m0[1], m0[2], m0[3]);
-                st_shared_v4(zd + (((2 + wg) ^ x7) << 4), m1[0], m1[1], m1[2], m1[3]);
+                st_shared_v4(zd + (((4 * st + wg) ^ x7) << 4), m0[0], m0[1], m0[2], m0[3]);
+                st_shared_v4(zd + (((4 * st + 2 + wg) ^ x7) << 4), m1[0], m1[1], m1[2], m1[3]);
                 fence_proxy_async_smem();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&bars->dpre_full[st]);
@@ -543,7 +545,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
         } else if (warp == W_ATT && lane == 0) {
             // ==================================================== all other products
             const uint32_t id_s = umma_idesc_16(IBLK, TM, 0, 0, 0, 0), id_kv = umma_idesc_16(IBLK, 64, 0, 1, 0, 0),
-                           id_q = umma_idesc_16(TM, 64, 1, 1, 0, 0), id_w = umma_idesc_16(128, 32, 1, 1, 0, 0);
+                           id_q = umma_idesc_16(TM, 64, 1, 1, 0, 0), id_w = umma_idesc_16(128, 64, 1, 1, 0, 0);
             const uint32_t qb = smem_u32(sm + M::Q), db = smem_u32(sm + M::DO), b0 = smem_u32(sm + M::B0), b1 = smem_u32(sm + M::B1),
                            ds = smem_u32(sm + M::DS), ab = smem_u32(sm + M::A);
             int nd = 0;
@@ -556,16 +558,17 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
                 return db + (nd & 1) * ATOM;
             };
             auto do_release = [&]() { if (NK == 2) { umma_commit(&bars->do_free[nd & 1]); ++nd; } };
-            auto dw = [&](int i, int c) {
-                if (!(alive = mbar_wait(&bars->dpre_full[c & 1], (uint32_t)((2 * i + (c >> 1)) & 1), abort_flag, 22, lim))) return;
+            auto dw = [&](int i, int pair) {          // chunks 2 pair and 2 pair + 1
+                for (int st = 0; st < 2; ++st)
+                    if (!(alive = mbar_wait(&bars->dpre_full[st], (uint32_t)((2 * i + pair) & 1), abort_flag, 22, lim))) return;
                 const int seg = i / n_blk, blk = i - seg * n_blk;
-                if (c == 0 && blk == 0 && seg > 0 && !(alive = mbar_wait(&bars->flushed, (uint32_t)((seg - 1) & 1), abort_flag, 23, lim))) return;
+                if (pair == 0 && blk == 0 && seg > 0 && !(alive = mbar_wait(&bars->flushed, (uint32_t)((seg - 1) & 1), abort_flag, 23, lim))) return;
                 tc_fence_after_sync();
                 // M = 128 channels; with 64 the second half reads the tile behind the states and is not used
 #pragma unroll
                 for (int k = 0; k < 8; ++k)
-                    umma_bf16_ss(tmem + T_DW + c * 32, umma_desc_mn_sw128(ab + k * 2048, ATOM, 1024), umma_desc_mn_sw128(b1 + k * 2048, ATOM, 1024), id_w, (blk | k) != 0);
-                umma_commit(&bars->dp_free[c & 1]);
+                    umma_bf16_ss(tmem + T_DW + pair * 64, umma_desc_mn_sw128(ab + k * 2048, ATOM, 1024), umma_desc_mn_sw128(b1 + k * 2048, ATOM, 1024), id_w, (blk | k) != 0);
+                if (pair == 0) umma_commit(&bars->dp_free);
             };
             for (int i = 0; i < n_it && alive; ++i) {
                 if (i >= 1 && !(alive = mbar_wait(&bars->dkv_empty, 1u, abort_flag, 24, lim))) break;      // chunk 3 of the block before
@@ -601,6 +604,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
                         umma_16_ts(tmem + T_DP + 64, tmem + T_S + k * 8, umma_desc_mn_sw128(dt + k * 2048, ATOM, 1024), id_kv, k != 0);
                     do_release();
                     umma_commit(&bars->dkv_full[c & 1]);
+                    if (c == 2) dw(i, 0);
+                    if (!alive) break;
                     if (!(alive = mbar_wait(&bars->kg_full[c & 1], (uint32_t)((2 * i + (c >> 1)) & 1), abort_flag, 28, lim))) break;
                     if (4 * i + c >= 1 && c >= 1 && !(alive = mbar_wait(&bars->dq_empty, (uint32_t)((c - 1) & 1), abort_flag, 29, lim))) break;
                     tc_fence_after_sync();
@@ -609,10 +614,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
                         umma_bf16_ss(tmem + T_DQ, umma_desc_mn_sw128(ds + k * 2048, ATOM, 1024), umma_desc_mn_sw128(b0 + k * 2048, ATOM, 1024), id_q, k != 0);
                     umma_commit(&bars->dq_full[c & 1]);
                     umma_commit(&bars->kg_free[c & 1]);
-                    if (c >= 1) dw(i, c - 1);
-                    if (!alive) break;
                 }
-                if (alive) dw(i, NCH - 1);
+                if (alive) dw(i, 1);
                 if (alive) umma_commit(&bars->blk_done);
             }
             umma_commit(&bars->drain);
