@@ -141,9 +141,9 @@ class _Telemetry:
     """Optional bookkeeping for the benchmark: kernel-launch counts per entry point and CUDA-event pairs around
     selected entry points (recorded on the launching stream)."""
 
-    # kernels launched by one call of each C entry point
-    KERNELS = {"mbema_query_scan": 2, "mbema_tile_states": 4, "mbema_qgate_fwd": 1, "mbema_qgate_bwd": 2,
-               "mbema_flash_fwd": 1, "mbema_flash_bwd": 2}
+    # kernels launched by one call of each C entry point (tensor-core mode; the snapshots with their items)
+    KERNELS = {"mbema_query_scan": 2, "mbema_tile_states": 6, "mbema_qgate_fwd": 1, "mbema_qgate_bwd": 2,
+               "mbema_flash_fwd": 4, "mbema_flash_bwd": 5}
 
     def __init__(self):
         self.enabled = False
