@@ -66,6 +66,7 @@ __device__ __forceinline__ void build_state_rows(const FlashArgs& a, int b, int 
 static constexpr int FS_SMS = 148;
 static int slot_parts(const FlashArgs& a, int ctas_per_sm) {
     const long long ctas = 2LL * a.nT * a.H * a.B;
+    if (ctas <= 0) return 1;                                                  // an empty call: the size queries come here
     const long long want = (ctas_per_sm * FS_SMS + ctas - 1) / ctas;
     return (int)(want < 1 ? 1 : want > 1 + a.K / 4 ? 1 + a.K / 4 : want);       // four slots a part at least
 }

@@ -45,6 +45,15 @@ def test_argument_errors_before_launch(lib):
     assert lib.mbema_query_scan_workspace_bytes(2, 128) >= 4 * 2 * 128 * 4
 
 
+@pytest.mark.parametrize("B,H,T", [(0, 8, 128), (2, 0, 128), (2, 8, 0)])
+def test_workspace_sizes_of_empty_calls(lib, B, H, T):
+    """An empty batch is a supported call and asks for its workspace first; empty heads or steps are refused by the call
+    itself, not by the size query."""
+    for query in (lib.mbema_flash_fwd_workspace_bytes, lib.mbema_flash_bwd_workspace_bytes):
+        for mode in (0, 1, 0 | 64, 1 | 64):
+            assert 0 < query(B, H, T, 64, 64, 100, mode) < 1 << 22
+
+
 def test_operators_refuse_cpu_tensors():
     import mathbrain_b200 as mb
     with pytest.raises(mb._lib.MbemaError):

@@ -159,3 +159,12 @@ def test_bounded_waits_give_up_cleanly(mb):
     assert mb.device_status() & 1
     mb.ops.clear_status()
     compare(attend(mb, c, V, "tc_bf16"), attend(mb, c, V, "fp32"))
+
+
+@pytest.mark.parametrize("mode", ["tc_bf16", "fp32"])
+def test_empty_batch(mb, mode):
+    c, V = case(3, 130, 40, 64)
+    for k in ("x", "unique", "c_base", "Q", "Ek", "Ev", "dO"):
+        c[k] = c[k][:0]
+    out = attend(mb, c, V, mode)
+    assert out["O"].shape == c["Q"].shape and float(out["dW"].abs().max()) == 0.0
