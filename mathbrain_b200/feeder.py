@@ -42,12 +42,27 @@ class ChunkFeeder:
         self.n_seen[docs] = 0
         self.t0[docs] = 0
 
+    def _same_device(self, *operands):
+        """Every tensor whose address goes to a kernel, the resident ones included (a program may have put others in their
+        place), is on the state's device; resident ones of another type or layout are brought into the kernels'."""
+        dev = self.state.device
+        for t in operands:
+            if t.device != dev:
+                raise _lib.MbemaError("ChunkFeeder: operand on %s, state on %s" % (t.device, dev))
+        B, V, N, cap = self.B, self.V, self.N, self.cap
+        for name, dtype, shape in (("state", torch.float32, (B, V, N)), ("last_t", torch.int32, (B, V)), ("seen", torch.int64, (B, cap)),
+                                   ("n_seen", torch.int64, (B,)), ("t0", torch.int32, (B,)), ("rhos", torch.float32, (N,))):
+            t = getattr(self, name)
+            if t.device != dev or t.shape != shape:
+                raise _lib.MbemaError("ChunkFeeder: %s is %s on %s, expected %s on %s" % (name, tuple(t.shape), t.device, shape, dev))
+            if t.dtype != dtype or not t.is_contiguous():
+                setattr(self, name, t.to(dtype).contiguous())
+
     def next_batch(self, x, fill):
         """Wire format of the next chunk of every document: dict(unique_slots [B, K] int64 (0-padded, as the collate
         function pads), pad_mask [B, K] bool, c_base [B, K, N] float32, K_max).  x [B, T] int64, fill [B] valid lengths."""
         _require_cuda(x, fill)
-        if x.device != self.state.device:
-            raise _lib.MbemaError("ChunkFeeder: chunk on %s, state on %s" % (x.device, self.state.device))
+        self._same_device(x, fill)
         with torch.cuda.device(self.state.device):
             return self._next_batch(x, fill)
 
@@ -81,8 +96,7 @@ class ChunkFeeder:
         LAST occurrence plus one (C_seq from compute_query_ema_history on this chunk), stamped with that step; tokens seen
         for the first time join the document's list.  Raises if a list would overflow."""
         _require_cuda(x, fill, C_seq)
-        if x.device != self.state.device:
-            raise _lib.MbemaError("ChunkFeeder: chunk on %s, state on %s" % (x.device, self.state.device))
+        self._same_device(x, fill, C_seq)
         with torch.cuda.device(self.state.device):
             self._advance(x, fill, C_seq)
 
