@@ -32,7 +32,7 @@ class ChunkFeeder:
         self.seen = torch.zeros(self.B, self.cap, dtype=torch.int64, device=dev)             # tokens seen so far, per document
         self.n_seen = torch.zeros(self.B, dtype=torch.int64, device=dev)
         self.t0 = torch.zeros(self.B, dtype=torch.int32, device=dev)                         # step of the next chunk's first token
-        self._widest = None        # widest slot list of a next_batch that no advance has followed yet
+        self._widest = None        # (widest slot list, the seen lists it was read from) of a next_batch that no advance has followed yet
 
     def reset(self, docs):
         """Start new documents in the given rows (a tensor or list of row numbers)."""
@@ -58,6 +58,19 @@ class ChunkFeeder:
             if t.dtype != dtype or not t.is_contiguous():
                 setattr(self, name, t.to(dtype).contiguous())
 
+    def _lists(self):
+        """The seen lists as they stand: the tensors with their version counters, which in-place changes raise (tensors made
+        under inference_mode have none)."""
+        return [(t, None if t.is_inference() else t._version) for t in (self.seen, self.n_seen)]
+
+    def _longest_possible(self, T):
+        """No seen list is longer after a chunk of T tokens: the lists of the next_batch just before hold every token seen so
+        far, unless the program has changed them since."""
+        widest, self._widest = self._widest, None
+        if widest is None or any(a is not b or v is None or v != w for (a, v), (b, w) in zip(widest[1], self._lists())):
+            return self.cap + 1
+        return min(widest[0] + T, self.V)
+
     def next_batch(self, x, fill):
         """Wire format of the next chunk of every document: dict(unique_slots [B, K] int64 (0-padded, as the collate
         function pads), pad_mask [B, K] bool, c_base [B, K, N] float32, K_max).  x [B, T] int64, fill [B] valid lengths."""
@@ -81,8 +94,9 @@ class ChunkFeeder:
         rc = lib.mbema_feed_lists(_ptr(x), _ptr(fill), _ptr(self.seen), _ptr(self.n_seen), _ptr(lists), _ptr(counts), B, T, self.V,
                                   self.cap, _stream())
         _lib.check(rc, "mbema_feed_lists")
-        self._widest = int(counts[B])                                            # the one host synchronisation
-        K = max(16, self._widest)
+        widest = int(counts[B])                                                  # the one host synchronisation
+        self._widest = widest, self._lists()
+        K = max(16, widest)
         unique = torch.empty(B, K, dtype=torch.int64, device=dev)
         pad_mask = torch.empty(B, K, dtype=torch.bool, device=dev)
         c_base = torch.empty(B, K, self.N, dtype=torch.float32, device=dev)
@@ -113,10 +127,8 @@ class ChunkFeeder:
                                                 _stream())
             _lib.check(rc, "mbema_feed_advance")
 
-        # The lists of the next_batch before this call hold every token seen so far, so no list grows past their width plus T.
-        # Where that rules an overflow out, nothing is asked of the device (a read back costs as much as the three kernels).
-        bound, self._widest = (self.cap + 1 if self._widest is None else min(self._widest + T, self.V)), None
-        if bound > self.cap:
+        # Where an overflow is ruled out nothing is asked of the device (a read back costs as much as the three kernels).
+        if self._longest_possible(T) > self.cap:
             status = torch.zeros(1, dtype=torch.int32, device=x.device)
             call(status, 1)
             if int(status) > self.cap:

@@ -44,3 +44,16 @@ def test_resident_tensors_of_another_device_or_shape(feeder, name):
         with pytest.raises(_lib.MbemaError, match=name):
             feeder.advance(ops["x"], ops["fill"], ops["C_seq"])
         setattr(feeder, name, held)
+
+
+def test_changed_lists_are_checked_on_the_device(feeder):
+    """The widest list that next_batch read bounds the lists after the chunk only while they are the ones it was read from."""
+    def after(change):
+        feeder._widest = 3, feeder._lists()
+        change()
+        return feeder._longest_possible(4)
+    assert after(lambda: None) == 7 and feeder._widest is None
+    assert feeder._longest_possible(4) > feeder.cap                        # no next_batch before
+    for change in (lambda: feeder.n_seen.fill_(6), lambda: feeder.seen.zero_(), lambda: feeder.reset([0]),
+                   lambda: setattr(feeder, "n_seen", feeder.n_seen.clone()), lambda: setattr(feeder, "seen", feeder.seen.clone())):
+        assert after(change) > feeder.cap

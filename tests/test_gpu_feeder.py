@@ -102,7 +102,12 @@ def test_feeder_vocabulary_of_several_segments_and_strided_lengths():
         feeder.advance(xd, fill, C_seq)
         assert feeder.n_seen.cpu().tolist() == [len(np.unique(h)) for h in history]
     before = feeder.state.clone()
-    feeder.n_seen.fill_(250)                # set by the program, as when it restores a saved state
-    with pytest.raises(mb._lib.MbemaError):
-        feeder.advance(torch.arange(B * T).view(B, T).cuda() + 1000, fill, C_seq)
-    assert torch.equal(feeder.state, before)
+    chunk = torch.arange(B * T).view(B, T).cuda() + 1000
+    for prepared in (False, True):
+        if prepared:
+            feeder.n_seen.fill_(3)
+            feeder.next_batch(chunk, fill)
+        feeder.n_seen.fill_(250)            # set by the program, as when it restores a saved state
+        with pytest.raises(mb._lib.MbemaError):
+            feeder.advance(chunk, fill, C_seq)
+        assert torch.equal(feeder.state, before) and feeder.n_seen.cpu().tolist() == [250, 250]
