@@ -14,8 +14,10 @@
 // the steps; then a thread per step for dQ), a loader lane and two issuing lanes.  Registers and tensor memory hold all
 // that shared memory (224 KB: Q' 64, dO' 64, states 16, dS 32, W' 16, two operand tiles 32) has no room for; for 128
 // channels dO' is streamed through two stages from a copy in the workspace instead.
-// The 16-bit gradients are scaled by powers of two: P by 2^kappa from the share of the listed slots in the softmax,
-// dO by 2^e from its largest value.
+// The 16-bit gradients are scaled by powers of two, so that none leaves the fp16 range whatever the values: P by 2^kappa from
+// the share of the listed slots in the softmax, dO by 2^e from its largest value, dS per block from the largest P |dP - D| of
+// its items (|dP - D| has no bound of its own: it is of the size of dO times the values), the moments per block from a bound on
+// the sums in them; dW, summed in tensor memory, leaves it when its unit changes.
 #include "smooth.cuh"
 #include "smooth_dev.cuh"
 
@@ -35,17 +37,21 @@ static constexpr float LN2 = 0.6931471806f;
 struct Bars {
     uint64_t a_full, w_full[2], w_free[2], do_full[2], do_free[2];
     uint64_t pre1_full[2], pre2_full[2], pre_empty[2], kv_full[2], kv_free[2], sdp_full, s_read, pds_full;
-    uint64_t dkv_full[2], dkv_empty, kg_full[2], kg_free[2], dq_full[2], dq_empty, dpre_full[2], dp_free, blk_done, flushed, drain;
+    uint64_t dkv_full[2], dkv_empty, kg_full[2], kg_free[2], dq_full[2], dq_empty, dpre_full[2], dp_free, blk_done, drain;
     uint32_t tmem_base;
     int abort_flag, drain_flag;
-    unsigned spin_limit, dmax, pmax;
+    unsigned spin_limit, dmax, pmax, qmax;
+    // of the block worked on, per warp: largest P |dP - D| of an item (a bound on it), |dP - D|, P; largest |E / 4|
+    alignas(16) float red_b[SM_WARPS], red_x[SM_WARPS], red_p[SM_WARPS], red_e[GATE_WARPS];
+    float fs[GATE_WARPS], fm[GATE_WARPS];      // its factors of dS and of the moments, a copy per gate warp
+    int dw_fresh;                              // its dW products start the sums anew
 };
 
 template <int NK> struct L {
     static constexpr int NDO = NK == 1 ? NCH : 2;
     static constexpr int Q = 0, DO = Q + NCH * ATOM, A = DO + NDO * ATOM, DS = A + NK * ATOM, W = DS + 2 * ATOM, B0 = W + 2 * WPIECE,
-                         B1 = B0 + ATOM, LSE = B1 + ATOM, DL = LSE + TM * 4, BAR = DL + TM * 4, SMEM = BAR + 448 + 1024;
-    static_assert(sizeof(Bars) <= 448 && SMEM <= 227 * 1024, "shared memory");
+                         B1 = B0 + ATOM, LSE = B1 + ATOM, DL = LSE + TM * 4, BAR = DL + TM * 4, SMEM = BAR + 640 + 1024;
+    static_assert(sizeof(Bars) <= 640 && BAR % 16 == 0 && SMEM <= 227 * 1024, "shared memory");
 };
 
 __device__ __forceinline__ f32x2 unpack_h2(uint32_t v) {
@@ -55,6 +61,31 @@ __device__ __forceinline__ f32x2 unpack_h2(uint32_t v) {
 __device__ __forceinline__ void red_v4(float* p, float a, float b, float c, float d) {
     asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
 }
+
+__device__ __forceinline__ uint32_t max_f16x2(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("max.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+__device__ __forceinline__ float larger_half(uint32_t v) {
+    const float2 f = unpack_f16x2(v);
+    return fmaxf(f.x, f.y);
+}
+__device__ __forceinline__ float warp_max(float v) {      // v >= 0
+    return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v)));
+}
+__device__ __forceinline__ float max8(const float* p) {
+    const float4 u = *reinterpret_cast<const float4*>(p), v = *reinterpret_cast<const float4*>(p + 4);
+    return fmaxf(fmaxf(fmaxf(u.x, u.y), fmaxf(u.z, u.w)), fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)));
+}
+// 2^14 <= v * scale < 2^15, a power of two between 2^-lo and 2^hi
+__device__ __forceinline__ float scale_to_f16(float v, int lo, int hi) {
+    const int e = 14 - ((int)(__float_as_uint(v) >> 23) - 127);
+    return __uint_as_float((uint32_t)(127 + max(-lo, min(hi, e))) << 23);
+}
+__device__ __forceinline__ float inverse(float power_of_two) { return __uint_as_float((254u << 23) - __float_as_uint(power_of_two)); }
+// factor of dS beside those of P and dO: neither P |dP - D| nor |dP - D| leaves the fp16 range
+__device__ __forceinline__ float ds_scale(const Bars* bars) { return scale_to_f16(fmaxf(max8(bars->red_b), max8(bars->red_x)), 60, 16); }
 
 template <bool SILU, int NK, bool EF32>
 __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it, Ws w, int* status) {
@@ -93,12 +124,13 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
         }
         mbar_init(&bars->sdp_full, 1); mbar_init(&bars->s_read, SM_WARPS); mbar_init(&bars->pds_full, SM_WARPS);
         mbar_init(&bars->dkv_empty, GATE_WARPS); mbar_init(&bars->dq_empty, 4);
-        mbar_init(&bars->dp_free, 1); mbar_init(&bars->blk_done, 1); mbar_init(&bars->flushed, GATE_WARPS); mbar_init(&bars->drain, 2);
+        mbar_init(&bars->dp_free, 1); mbar_init(&bars->blk_done, 1); mbar_init(&bars->drain, 2);
         bars->abort_flag = *reinterpret_cast<volatile int*>(status);
         bars->drain_flag = 0;
         bars->spin_limit = a.test_withhold ? 64u : MBEMA_SPIN_LIMIT;
         bars->dmax = 0u;
         bars->pmax = 0u;
+        bars->qmax = 0u;
         fence_barrier_init();
     }
     if (warp == W_GATE) {
@@ -116,12 +148,15 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
         basis(t, level, beta);
         float* scr = reinterpret_cast<float*>(sm + M::B0);     // [4][128] partial sums of dO . O
         if (tid < TM * NCH) {
-            float dot = 0.f, mx = 0.f;
+            float dot = 0.f, mx = 0.f, qm = 0.f;
 #pragma unroll
             for (int i = 0; i < 16; i += 4) {
                 const float4 q = ok ? ld4_dyn_f32(a.Q, a.q_dt, (row0 + t) * HD + c * 16 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
                 v[i] = q.x; v[i + 1] = q.y; v[i + 2] = q.z; v[i + 3] = q.w;
+                qm = fmaxf(qm, fmaxf(fmaxf(fabsf(q.x), fabsf(q.y)), fmaxf(fabsf(q.z), fabsf(q.w))));
             }
+            qm = warp_max(qm);
+            if (lane == 0) atomicMax(&bars->qmax, __float_as_uint(qm));
             store_basis_rows(sm + M::Q + c * ATOM, t, v, beta, 0.125f * 1.4426950409f);
 #pragma unroll
             for (int i = 0; i < 16; i += 4) {
@@ -143,7 +178,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
         }
         __syncthreads();
         const float dm = __uint_as_float(bars->dmax);
-        if (dm > 0.f && dm < INFINITY) e2 = exp2f((float)min(-ilogbf(dm), 90));      // largest |dO| in [1, 2)
+        if (dm > 0.f && dm < INFINITY) e2 = exp2f((float)max(min(-ilogbf(dm), 90), -100));      // largest |dO| in [1, 2)
         kappa = 15.f + floorf(-log2f(fminf(fmaxf(__uint_as_float(bars->pmax), 1.0f / 512.0f), 1.0f)));
         if (tid < TM * NCH) {
 #pragma unroll
@@ -168,7 +203,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
     const int n_items = it.count[bt].x, n_blk = it.count[bt].y;          // the hot slots are the every-step kernel's
     const int n_it = bars->abort_flag ? 0 : n_blk << level;
     const unsigned* lim = &bars->spin_limit;
-    const float unit = exp2f(kappa - 4.0f) * e2 ;         // dS, dK, dc and dpre carry this factor (dS ln 2 more)
+    const float unit = exp2f(kappa) * e2;        // factor of P dO; dS, dK, dc and dpre carry it times the block's factor (dS ln 2 more)
 
     if (warp < GATE_WARPS) {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
@@ -176,7 +211,37 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
         const int wg = warp >> 2, r = tid & 127, x7 = r & 7;
         const uint32_t t_lane = tmem + ((uint32_t)((warp & 3) * 32) << 16);
         const int2* meta = it.meta + (size_t)bt * it.IB * IBLK + r;
-        const float oe = 0.25f / unit, ov = oe * 0.0625f;
+        const float ov = 0.25f / unit;
+        float fw = 0.f;          // factor of dS times that of the moments, the unit of the dW sums
+        // the dW sums in tensor memory: lane n, chunks 2 wg and 2 wg + 1
+        auto flush = [&](int seg, bool first) {
+            tc_fence_after_sync();
+            if (r < N) {         // whole warps
+                const float len = (float)(TM >> level), l2 = log2f(a.rhos[r]);
+                const float mid = (float)seg * len + 0.5f * (len - 1.0f), ha = 0.5f * len * 0.9238795325f, hb = 0.5f * len * 0.3826834324f;
+                const float pa = exp2f(l2 * (mid + ha)), pb = exp2f(l2 * (mid + hb)), pc = exp2f(l2 * (mid - hb)), pd = exp2f(l2 * (mid - ha));
+                const float sc = STATE_F16_UNSCALE / unit * inverse(fw);
+                const float r0 = 0.25f * (pa + pb + pc + pd) * sc, r1 = 0.5f * (0.9238795325f * (pa - pd) + 0.3826834324f * (pb - pc)) * sc;
+#pragma unroll 1
+                for (int q = 0; q < 4; ++q) {
+                    float d0[8], d1[8];
+                    const uint32_t td = t_lane + T_DW + wg * 64 + (q >> 1) * 32 + (q & 1) * 8;
+                    tmem_ld_32x32b_x8(td, d0);
+                    tmem_ld_32x32b_x8(td + 16, d1);
+                    tmem_wait_ld();
+                    float* o = part + (size_t)r * 128 + (2 * wg + (q >> 1)) * 16 + (q & 1) * 8;
+#pragma unroll
+                    for (int dd = 0; dd < 8; dd += 4) {
+                        const float4 v = make_float4(r0 * d0[dd] + r1 * d1[dd], r0 * d0[dd + 1] + r1 * d1[dd + 1], r0 * d0[dd + 2] + r1 * d1[dd + 2],
+                                                     r0 * d0[dd + 3] + r1 * d1[dd + 3]);
+                        if (first) *reinterpret_cast<float4*>(o + dd) = v;
+                        else red_v4(o + dd, v.x, v.y, v.z, v.w);
+                    }
+                }
+            }
+            tc_fence_before_sync();
+        };
+        bool first = true;
         size_t eo = 0;          // this item's E columns of chunk 0
         ERow<EF32> ek, ev;
         if (n_it > 0) {
@@ -187,6 +252,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
         bool alive = true;
         for (int i = 0; i < n_it && alive; ++i) {
             const int blk = i % n_blk;
+            uint32_t em = 0u;        // largest |E / 4|
             // ---------------------------------------------------- first pass: K_c and V_c
 #pragma unroll 1
             for (int c = 0; c < NCH; ++c) {
@@ -216,10 +282,17 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
                 for (int t = 0; t < 2; ++t) {      // K to the first tile, V to the one behind it
                     uint32_t e4[4];
 #pragma unroll
-                    for (int p = 0; p < 4; ++p) e4[p] = e_pair<EF32>(t == 0 ? ek : ev, p);
+                    for (int p = 0; p < 4; ++p) {
+                        e4[p] = e_pair<EF32>(t == 0 ? ek : ev, p);
+                        em = max_f16x2(em, e4[p] & 0x7fff7fffu);
+                    }
 #pragma unroll
                     for (int j = 0; j < NJ; ++j)
                         st_shared_v4(kd + t * ATOM + (((2 * j + wg) ^ x7) << 4), mul_f16x2(cf[j][0], e4[0]), mul_f16x2(cf[j][1], e4[1]), mul_f16x2(cf[j][2], e4[2]), mul_f16x2(cf[j][3], e4[3]));
+                }
+                if (c == NCH - 1) {
+                    const float m = warp_max(larger_half(em));
+                    if (lane == 0) bars->red_e[warp] = m;
                 }
                 fence_proxy_async_smem();
                 __syncwarp();
@@ -263,11 +336,30 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
                 fence_proxy_async_smem();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&bars->kg_full[st]);
+                if (c == 0) {      // the block's factors: red_e of all gate warps, red_b, red_x and red_p of the step warps
+                    if (!(alive = warp_wait(&bars->kv_full[1], 1u, abort_flag, 3, lim) && warp_wait(&bars->pds_full, (uint32_t)(i & 1), abort_flag, 8, lim))) break;
+                    // what the moments are at most: 128 steps, basis of at most 1.85, four coefficients into each of four nodes, a
+                    // derivative below 1.1; dS, P, dO (below 2) and q (log2(e) / 8) at their largest
+                    constexpr float SUM = 128.0f * 1.85f * 16.0f * 1.1f;
+                    const float f = ds_scale(bars), qm = 0.125f * 1.4426950409f * __uint_as_float(bars->qmax);
+                    const float top = SUM * f * max8(bars->red_e) * (qm * max8(bars->red_b) + 2.0f * max8(bars->red_p));
+                    const float fits = f * scale_to_f16(top, 50, 30);
+                    // The unit stays while the blocks fit (64 times smaller than the first one needs: rarely more than one unit a segment);
+                    // a smaller one, or a new segment, and what has been summed leaves tensor memory (blk_done has been waited for).
+                    const bool fresh = blk == 0 || fw > fits;
+                    if (fresh) {
+                        if (i > 0) { flush((i - 1) / n_blk, first); first = false; }
+                        fw = fits * 0.015625f;
+                    }
+                    if (lane == 0) { bars->fs[warp] = f; bars->fm[warp] = fw * inverse(f); bars->dw_fresh = fresh; }
+                    __syncwarp();
+                }
                 if (!(alive = warp_wait(&bars->dkv_full[st], (uint32_t)(use & 1), abort_flag, 6, lim))) break;
                 tc_fence_after_sync();
                 float* gk = a.dEk + eo + c * 16;
                 float* gv = a.dEv + eo + c * 16;
                 const bool live = blk * IBLK + r < n_items;
+                const float fs = bars->fs[warp], fm = bars->fm[warp], oe = ov * inverse(fs);
                 uint32_t m0[4], m1[4];
 #pragma unroll
                 for (int q = 0; q < 2; ++q) {      // four columns at a time
@@ -288,7 +380,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
                     for (int p = 0; p < 2; ++p) {
                         const int pp = 2 * q + p;
                         const f32x2 e = unpack_h2(e_pair<EF32>(ek, pp)), f0 = unpack_h2(e_pair<EF32>(ev, pp));
-                        const f32x2 f = mul2(f0, pack2(0.0625f, 0.0625f));
+                        const f32x2 f = mul2(f0, pack2(fs, fs));
                         f32x2 dc[NJ], sk = 0ull, sv = 0ull;
 #pragma unroll
                         for (int j = 0; j < NJ; ++j) {
@@ -305,9 +397,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
                             d0 = mul2(d0, unpack_h2(sp[0][pp])); d1 = mul2(d1, unpack_h2(sp[1][pp]));
                             d2 = mul2(d2, unpack_h2(sp[2][pp])); d3 = mul2(d3, unpack_h2(sp[3][pp]));
                         }
-                        // moments over the nodes, an eighth of the unit
-                        const f32x2 c8 = pack2(0.125f, 0.125f), ta = pack2(0.125f * 0.9238795325f, 0.125f * 0.9238795325f),
-                                    tb = pack2(0.125f * 0.3826834324f, 0.125f * 0.3826834324f);
+                        // moments over the nodes
+                        const float fa = fm * 0.9238795325f, fb = fm * 0.3826834324f;
+                        const f32x2 c8 = pack2(fm, fm), ta = pack2(fa, fa), tb = pack2(fb, fb);
                         const f32x2 s = mul2(add2(add2(d0, d3), add2(d1, d2)), c8);
                         const f32x2 x = fma2(fma2(d2, m, d1), tb, mul2(fma2(d3, m, d0), ta));
                         float lo, hi;
@@ -333,40 +425,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
                 ev = nv;
             }
             eo = eo_next;
-            if (alive && blk == n_blk - 1) {
-                // the segment's dW: lane n, chunks 2 wg and 2 wg + 1
-                if (!(alive = warp_wait(&bars->blk_done, (uint32_t)(i & 1), abort_flag, 8, lim))) break;
-                tc_fence_after_sync();
-                const int seg = i / n_blk;
-                float d[64];
-                tmem_ld_32x32b_x32(t_lane + T_DW + wg * 64, d);
-                tmem_ld_32x32b_x32(t_lane + T_DW + wg * 64 + 32, d + 32);
-                tmem_wait_ld();
-                tc_fence_before_sync();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&bars->flushed);
-                if (r < N) {
-                    const float len = (float)(TM >> level), l2 = log2f(a.rhos[r]);
-                    const float mid = (float)seg * len + 0.5f * (len - 1.0f), ha = 0.5f * len * 0.9238795325f, hb = 0.5f * len * 0.3826834324f;
-                    const float pa = exp2f(l2 * (mid + ha)), pb = exp2f(l2 * (mid + hb)), pc = exp2f(l2 * (mid - hb)), pd = exp2f(l2 * (mid - ha));
-                    const float sc = 8.0f * STATE_F16_UNSCALE / unit;
-                    const float r0 = 0.25f * (pa + pb + pc + pd) * sc, r1 = 0.5f * (0.9238795325f * (pa - pd) + 0.3826834324f * (pb - pc)) * sc;
-#pragma unroll
-                    for (int q = 0; q < 2; ++q)
-#pragma unroll
-                        for (int dd = 0; dd < 16; dd += 4) {
-                            float4* o = reinterpret_cast<float4*>(part + (size_t)r * 128 + (2 * wg + q) * 16 + dd);
-                            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-                            if (seg > 0) v = *o;
-                            v.x += r0 * d[q * 32 + dd] + r1 * d[q * 32 + 16 + dd];
-                            v.y += r0 * d[q * 32 + dd + 1] + r1 * d[q * 32 + 16 + dd + 1];
-                            v.z += r0 * d[q * 32 + dd + 2] + r1 * d[q * 32 + 16 + dd + 2];
-                            v.w += r0 * d[q * 32 + dd + 3] + r1 * d[q * 32 + 16 + dd + 3];
-                            *o = v;
-                        }
-                }
-            }
         }
+        if (n_it > 0 && alive && warp_wait(&bars->blk_done, (uint32_t)((n_it - 1) & 1), abort_flag, 8, lim)) flush((n_it - 1) / n_blk, first);
         if (n_blk == 0)
             for (int i = tid; i < N * (HD / 4); i += GATE_WARPS * 32)
                 *reinterpret_cast<float4*>(part + (i / (HD / 4)) * 128 + (i % (HD / 4)) * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -376,8 +436,6 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
         const int half = (warp >> 2) & 1, r = tid & 127, x7 = r & 7;
         const uint32_t t_lane = tmem + ((uint32_t)((warp & 3) * 32) << 16);
         const int2* meta = it.meta + (size_t)bt * it.IB * IBLK + r;
-        float beta[NJ];
-        basis(r, level, beta);
         float acc[2][16];
 #pragma unroll
         for (int e = 0; e < 16; ++e) acc[0][e] = acc[1][e] = 0.f;
@@ -412,25 +470,46 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
 #pragma unroll
                 for (int e = 0; e < 16; e += 2) p2[k * 8 + e / 2] = pack_f16x2_sat(ex2_approx(s[e]), ex2_approx(s[e + 1]));
             }
+            // this item's part in the choice of the block's factor of dS
+            uint32_t pm2 = 0u;
+            float xm = 0.f;
+#pragma unroll
+            for (int k = 0; k < 32; ++k) pm2 = max_f16x2(pm2, p2[k]);
+#pragma unroll 1
+            for (int tb = half * 64; tb < half * 64 + 64; tb += 16) {
+                float dp[16];
+                tmem_ld_32x32b_x16(t_lane + T_DP + tb, dp);
+                tmem_wait_ld();
+#pragma unroll
+                for (int e = 0; e < 16; e += 4) {
+                    const float4 dl = *reinterpret_cast<const float4*>(dl_sh + tb + e);
+                    xm = fmaxf(fmaxf(fmaxf(xm, fabsf(dp[e] - dl.x)), fmaxf(fabsf(dp[e + 1] - dl.y), fabsf(dp[e + 2] - dl.z))), fabsf(dp[e + 3] - dl.w));
+                }
+            }
+            const float pm = larger_half(pm2);
+            if (pm == 0.f) xm = 0.f;
+            const float wb = warp_max(pm * xm), wx = warp_max(xm), wp = warp_max(pm);
+            if (lane == 0) { bars->red_b[warp - GATE_WARPS] = wb; bars->red_x[warp - GATE_WARPS] = wx; bars->red_p[warp - GATE_WARPS] = wp; }
             tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) mbar_arrive(&bars->s_read);
             if (!(alive = warp_wait(&bars->s_read, (uint32_t)(i & 1), abort_flag, 10, lim))) break;
             tc_fence_after_sync();
+            const float fs = ds_scale(bars), cs = LN2 * fs;
             // the scores have been read by both halves: P^T takes their first 64 columns, dS^T the other 64
-#pragma unroll
-            for (int k = 0; k < 2; ++k) tmem_st_x16(t_lane + T_S + half * 32 + k * 16, *reinterpret_cast<const uint32_t(*)[16]>(p2 + k * 16));
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 const int tb = half * 64 + k * 16;
                 float dp[16];
                 uint32_t d2[8];
                 tmem_ld_32x32b_x16(t_lane + T_DP + tb, dp);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) d2[e] = p2[k * 8 + e];
+                tmem_st_x8(t_lane + T_S + half * 32 + k * 8, d2);
                 tmem_wait_ld();
 #pragma unroll
                 for (int e = 0; e < 16; e += 4) {
                     const float4 dl = *reinterpret_cast<const float4*>(dl_sh + tb + e);
-                    constexpr float cs = LN2 / 16.0f;
                     d2[e / 2] = mul_f16x2(p2[k * 8 + e / 2], pack_f16x2_sat((dp[e] - dl.x) * cs, (dp[e + 1] - dl.y) * cs));
                     d2[e / 2 + 1] = mul_f16x2(p2[k * 8 + e / 2 + 1], pack_f16x2_sat((dp[e + 2] - dl.z) * cs, (dp[e + 3] - dl.w) * cs));
                 }
@@ -444,6 +523,13 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) mbar_arrive(&bars->pds_full);
+            int rr = r;
+            asm volatile("" : "+r"(rr));          // formed here in every block, not kept in registers
+            float beta[NJ];
+            basis(rr, level, beta);
+            const float inv = inverse(fs);
+#pragma unroll
+            for (int e = 0; e < NJ; ++e) beta[e] *= inv;
 #pragma unroll
             for (int cc = 0; cc < 2; ++cc) {
                 if (!(alive = warp_wait(&bars->dq_full[half], (uint32_t)((2 * i + cc) & 1), abort_flag, 11, lim))) break;
@@ -461,7 +547,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
                         if (lane == 0) mbar_arrive(&bars->dq_empty);
                     }
 #pragma unroll
-                    for (int e = 0; e < 16; ++e) acc[cc][e] = j == 0 ? acc[cc][e] + v[0][e] : fmaf(beta[j], v[j & 1][e], acc[cc][e]);
+                    for (int e = 0; e < 16; ++e) acc[cc][e] = fmaf(beta[j], v[j & 1][e], acc[cc][e]);
                 }
             }
             if (!alive) break;
@@ -561,13 +647,12 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
             auto dw = [&](int i, int pair) {          // chunks 2 pair and 2 pair + 1
                 for (int st = 0; st < 2; ++st)
                     if (!(alive = mbar_wait(&bars->dpre_full[st], (uint32_t)((2 * i + pair) & 1), abort_flag, 22, lim))) return;
-                const int seg = i / n_blk, blk = i - seg * n_blk;
-                if (pair == 0 && blk == 0 && seg > 0 && !(alive = mbar_wait(&bars->flushed, (uint32_t)((seg - 1) & 1), abort_flag, 23, lim))) return;
                 tc_fence_after_sync();
+                const bool fresh = *reinterpret_cast<volatile int*>(&bars->dw_fresh) != 0;
                 // M = 128 channels; with 64 the second half reads the tile behind the states and is not used
 #pragma unroll
                 for (int k = 0; k < 8; ++k)
-                    umma_bf16_ss(tmem + T_DW + pair * 64, umma_desc_mn_sw128(ab + k * 2048, ATOM, 1024), umma_desc_mn_sw128(b1 + k * 2048, ATOM, 1024), id_w, (blk | k) != 0);
+                    umma_bf16_ss(tmem + T_DW + pair * 64, umma_desc_mn_sw128(ab + k * 2048, ATOM, 1024), umma_desc_mn_sw128(b1 + k * 2048, ATOM, 1024), id_w, k != 0 || !fresh);
                 if (pair == 0) umma_commit(&bars->dp_free);
             };
             for (int i = 0; i < n_it && alive; ++i) {

@@ -76,6 +76,18 @@ def compare(out, ref):
         assert rel_err(out[k].float(), ref[k].float()) < (TOL_O if k == "O" else TOL_GRAD), k
 
 
+def compare_rows(out, ref, names=("dEk", "dEv", "dQ"), floor=1e-3):
+    """Every row against its own size (2-norm), down to `floor` of the largest row: the largest rows are the hot slots', which the
+    every-step kernel makes, many times the size of the others."""
+    for k in names:
+        a, b = out[k].double().flatten(0, -2), ref[k].double().flatten(0, -2)
+        assert bool(torch.isfinite(a).all()), k
+        n = b.norm(dim=1)
+        live = n > floor * n.max()
+        err = ((a - b).norm(dim=1) / n)[live]
+        assert float(err.max()) < TOL_GRAD, (k, float(err.max()))
+
+
 @pytest.mark.parametrize("N", [64, 128])
 @pytest.mark.parametrize("T,K", [(1, 1), (127, 17), (128, 16), (129, 144), (130, 145), (300, 400), (513, 1100)])
 def test_edges_of_tiles_and_item_blocks(mb, N, T, K):
@@ -97,6 +109,38 @@ def test_segments_of_large_pre_activations(mb, std):
     c, V = case(77, 200, 200, 64, std=std, state=20.0)
     c["Ek"], c["Ev"] = c["Ek"] * 0.1 / std, c["Ev"] * 0.1 / std      # scores stay near one
     compare(attend(mb, c, V, "tc_bf16"), attend(mb, c, V, "fp32"))
+
+
+@pytest.mark.parametrize("N,H", [(64, 2), (64, 6), (128, 4)])
+def test_rows_of_small_gradients(mb, N, H):
+    c, V = case(21, 300, 500, N, H=H, unlisted=0.0)
+    compare_rows(attend(mb, c, V, "tc_bf16"), attend(mb, c, V, "fp32"), names=("dEk", "dEv"), floor=1e-4)
+
+
+@pytest.mark.parametrize("N", [64, 128])
+@pytest.mark.parametrize("ev", [0.01, 1.0, 30.0])
+def test_values_and_gradients_of_any_size_in_a_peaked_softmax(mb, N, ev):
+    """Two slots of moderate state (not among the hot ones) share every row's softmax and dO points along the difference of their
+    values: |dP - D| is thousands of times max |dO| for ev = 30."""
+    c, V = case(8, 300, 200, N, unlisted=0.0, state=20.0)
+    listed = c["unique"] >= 0
+    pair = torch.tensor([50, 60], device="cuda")
+    c["x"] = torch.where((c["x"][..., None] == c["unique"][:, None, pair]).any(-1), c["unique"][:, :1].clamp_min(0), c["x"])
+    c["c_base"][:, pair] = 4.0
+    c["W"] = c["W"].abs() + 0.01                     # gates of one sign
+    c["Q"] = torch.ones_like(c["Q"]) * 0.5
+    c["Ek"] = torch.zeros_like(c["Ek"])
+    scale = 16.0 / (4.0 * float(c["W"].sum(0).mean()) * 64 * 0.5 / 8)
+    c["Ek"][:, pair] = scale
+    c["Ek"][:, pair[1], ::2] *= 1.5                  # (equal keys would cancel in dQ)
+    c["Ek"][:, pair[1], 1::2] *= 0.5
+    g = torch.Generator().manual_seed(2)
+    c["Ev"] = ((torch.randn(c["Ev"].shape, generator=g) * ev).cuda() * listed[..., None]).to(c["Ev"].dtype)
+    d = torch.sign(c["Ev"][:, pair[0]].float() - c["Ev"][:, pair[1]].float())
+    c["dO"] = d.view(d.shape[0], -1, 1, 64).expand(-1, -1, c["x"].shape[1], -1).contiguous() * 0.01
+    out, ref = attend(mb, c, V, "tc_bf16"), attend(mb, c, V, "fp32")
+    compare_rows(out, ref)
+    assert rel_err(out["dW"], ref["dW"]) < TOL_GRAD
 
 
 @pytest.mark.parametrize("silu,dtype", [(False, torch.bfloat16), (True, torch.float32)])
