@@ -15,7 +15,8 @@
 // that shared memory (224 KB: Q' 64, dO' 64, states 16, dS 32, W' 16, two operand tiles 32) has no room for; for 128
 // channels dO' is streamed through two stages from a copy in the workspace instead.
 // The 16-bit gradients are scaled by powers of two, so that none leaves the fp16 range whatever the values: P by 2^kappa from
-// the share of the listed slots in the softmax, dO by 2^e from its largest value, dS per block from the largest P |dP - D| of
+// the share of the listed slots in the softmax, dO by a factor per row from the
+// row's largest value (rows of very different size stand in a tile: well predicted tokens beside others), dS per block from the largest P |dP - D| of
 // its items (|dP - D| has no bound of its own: it is of the size of dO times the values), the moments per block from a bound on
 // the sums in them; dW, summed in tensor memory, leaves it when its unit changes.
 #include "smooth.cuh"
@@ -39,8 +40,8 @@ struct Bars {
     uint64_t pre1_full[2], pre2_full[2], pre_empty[2], kv_full[2], kv_free[2], sdp_full, s_read, pds_full;
     uint64_t dkv_full[2], dkv_empty, kg_full[2], kg_free[2], dq_full[2], dq_empty, dpre_full[2], dp_free, blk_done, drain;
     uint32_t tmem_base;
-    int abort_flag, drain_flag;
-    unsigned spin_limit, dmax, pmax, qmax;
+    int abort_flag, drain_flag, emin, bad;      // emin: exponent of the row factor of the largest |dO|; bad: a row of dO is not finite
+    unsigned spin_limit, pmax, qmax;
     // of the block worked on, per warp: largest P |dP - D| of an item (a bound on it), |dP - D|, P; largest |E / 4|
     alignas(16) float red_b[SM_WARPS], red_x[SM_WARPS], red_p[SM_WARPS], red_e[GATE_WARPS];
     float fs[GATE_WARPS], fm[GATE_WARPS];      // its factors of dS and of the moments, a copy per gate warp
@@ -50,7 +51,7 @@ struct Bars {
 template <int NK> struct L {
     static constexpr int NDO = NK == 1 ? NCH : 2;
     static constexpr int Q = 0, DO = Q + NCH * ATOM, A = DO + NDO * ATOM, DS = A + NK * ATOM, W = DS + 2 * ATOM, B0 = W + 2 * WPIECE,
-                         B1 = B0 + ATOM, LSE = B1 + ATOM, DL = LSE + TM * 4, BAR = DL + TM * 4, SMEM = BAR + 640 + 1024;
+                         B1 = B0 + ATOM, LSE = B1 + ATOM, DL = LSE + TM * 4, GF = DL + TM * 4, RX = GF + TM * 2, BAR = RX + TM, SMEM = BAR + 640 + 1024;
     static_assert(sizeof(Bars) <= 640 && BAR % 16 == 0 && SMEM <= 227 * 1024, "shared memory");
 };
 
@@ -94,7 +95,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
     using M = L<NK>;
     Bars* bars = reinterpret_cast<Bars*>(sm + M::BAR);
     float* lse_sh = reinterpret_cast<float*>(sm + M::LSE);     // log2(e) LSE - kappa; +inf for rows that do not count
-    float* dl_sh = reinterpret_cast<float*>(sm + M::DL);       // 2^e D
+    float* dl_sh = reinterpret_cast<float*>(sm + M::DL);       // row factor times D
+    __half* gf_sh = reinterpret_cast<__half*>(sm + M::GF);     // smallest row factor over the row's
+    unsigned char* rx_sh = sm + M::RX;                         // its exponent, negated; 255: dO is not finite
     volatile int* abort_flag = &bars->abort_flag;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int tile = blockIdx.x, h = blockIdx.y, b = a.order ? a.order[blockIdx.z] : (int)blockIdx.z;
@@ -128,7 +131,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
         bars->abort_flag = *reinterpret_cast<volatile int*>(status);
         bars->drain_flag = 0;
         bars->spin_limit = a.test_withhold ? 64u : MBEMA_SPIN_LIMIT;
-        bars->dmax = 0u;
+        bars->emin = INT_MAX;
+        bars->bad = 0;
         bars->pmax = 0u;
         bars->qmax = 0u;
         fence_barrier_init();
@@ -140,15 +144,18 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
     __syncthreads();
     // Q' and dO' tiles (thread: step t, chunk c), D = dO . O, the scales
     const float rest = a.v_total - (float)a.kcount[b];
-    float e2 = 1.f, kappa = 15.f;
+    float kappa = 15.f;
+    int emin;
     {
         const int t = tid & (TM - 1), c = (tid >> 7) & 3;
         const bool ok = t0 + t < Lb;
         float beta[NJ], v[16];
         basis(t, level, beta);
-        float* scr = reinterpret_cast<float*>(sm + M::B0);     // [4][128] partial sums of dO . O
+        float* scr = reinterpret_cast<float*>(sm + M::B0);                    // [4][128] partial sums of dO . O
+        unsigned* scm = reinterpret_cast<unsigned*>(sm + M::B0) + NCH * TM;    // [4][128] largest |dO| (as bits: NaN above infinity)
         if (tid < TM * NCH) {
-            float dot = 0.f, mx = 0.f, qm = 0.f;
+            float dot = 0.f, qm = 0.f;
+            unsigned mx = 0u;
 #pragma unroll
             for (int i = 0; i < 16; i += 4) {
                 const float4 q = ok ? ld4_dyn_f32(a.Q, a.q_dt, (row0 + t) * HD + c * 16 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -164,11 +171,11 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
                 const float4 o = ok ? *reinterpret_cast<const float4*>(a.O + (row0 + t) * HD + c * 16 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
                 v[i] = g.x; v[i + 1] = g.y; v[i + 2] = g.z; v[i + 3] = g.w;
                 dot += g.x * o.x + g.y * o.y + g.z * o.z + g.w * o.w;
-                mx = fmaxf(mx, fmaxf(fmaxf(fabsf(g.x), fabsf(g.y)), fmaxf(fabsf(g.z), fabsf(g.w))));
+#pragma unroll
+                for (int e = 0; e < 4; ++e) mx = max(mx, __float_as_uint(fabsf(v[i + e])));
             }
             scr[c * TM + t] = dot;
-            for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-            if (lane == 0) atomicMax(&bars->dmax, __float_as_uint(mx));
+            scm[c * TM + t] = mx;
             if (c == 0) {
                 float share = 1.f;
                 if (!a.listed_only && rest > 0.f) share = ok ? 1.f - rest * __expf(-a.LSE[row0 + t]) : 0.f;
@@ -177,12 +184,18 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
             }
         }
         __syncthreads();
-        const float dm = __uint_as_float(bars->dmax);
-        if (dm > 0.f && dm < INFINITY) e2 = exp2f((float)max(min(-ilogbf(dm), 90), -100));      // largest |dO| in [1, 2)
         kappa = 15.f + floorf(-log2f(fminf(fmaxf(__uint_as_float(bars->pmax), 1.0f / 512.0f), 1.0f)));
+        int er = INT_MAX;          // exponent of the row's factor: largest |dO| of the row in [2^13, 2^14)
+        bool bad = false;
         if (tid < TM * NCH) {
+            const unsigned m = max(max(scm[t], scm[TM + t]), max(scm[2 * TM + t], scm[3 * TM + t]));
+            const float dl = scr[t] + scr[TM + t] + scr[2 * TM + t] + scr[3 * TM + t];
+            if (m != 0u) er = max(-114, min(80, 13 + 127 - (int)(m >> 23)));
+            const float rs = m != 0u ? exp2f((float)er) : 1.f;
+            bad = m >= 0x7f800000u || !(fabsf(dl * rs) < INFINITY);
+            // a row that is not finite is left out of the products; everything it reaches becomes NaN at the end
 #pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] *= e2;
+            for (int i = 0; i < 16; ++i) v[i] = bad ? 0.f : v[i] * rs;
             if (NK == 1) {
                 store_basis_rows(sm + M::DO + c * ATOM, t, v, beta, 1.0f);
             } else {
@@ -191,8 +204,21 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
             }
             if (c == 0) {
                 lse_sh[t] = ok ? a.LSE[row0 + t] * 1.4426950409f - kappa : INFINITY;
-                dl_sh[t] = (scr[t] + scr[TM + t] + scr[2 * TM + t] + scr[3 * TM + t]) * e2;
+                dl_sh[t] = bad ? 0.f : dl * rs;
+                const int e = __reduce_min_sync(0xffffffffu, bad ? INT_MAX : er);
+                const bool any = __any_sync(0xffffffffu, bad);
+                if (lane == 0) {
+                    atomicMin(&bars->emin, e);
+                    if (any) bars->bad = 1;
+                }
             }
+        }
+        __syncthreads();
+        emin = bars->emin == INT_MAX ? 0 : bars->emin;
+        if (tid < TM) {
+            const int k = bad || er == INT_MAX ? 0 : er - emin;
+            gf_sh[t] = __float2half_rn(exp2f((float)-k));
+            rx_sh[t] = bad ? 255 : k;
         }
     }
     asm volatile("fence.proxy.async;" ::: "memory");      // the operand tiles, in shared memory and (NK = 2) in the workspace
@@ -203,7 +229,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
     const int n_items = it.count[bt].x, n_blk = it.count[bt].y;          // the hot slots are the every-step kernel's
     const int n_it = bars->abort_flag ? 0 : n_blk << level;
     const unsigned* lim = &bars->spin_limit;
-    const float unit = exp2f(kappa) * e2;        // factor of P dO; dS, dK, dc and dpre carry it times the block's factor (dS ln 2 more)
+    const float unit = exp2f(kappa + (float)emin);      // factor of P dO; dS, dK, dc and dpre carry it times the block's factor (dS ln 2 more)
 
     if (warp < GATE_WARPS) {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
@@ -211,7 +237,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
         const int wg = warp >> 2, r = tid & 127, x7 = r & 7;
         const uint32_t t_lane = tmem + ((uint32_t)((warp & 3) * 32) << 16);
         const int2* meta = it.meta + (size_t)bt * it.IB * IBLK + r;
-        const float ov = 0.25f / unit;
+        const float ov = 0.25f / unit * (bars->bad ? NAN : 1.0f);
         float fw = 0.f;          // factor of dS times that of the moments, the unit of the dW sums
         // the dW sums in tensor memory: lane n, chunks 2 wg and 2 wg + 1
         auto flush = [&](int seg, bool first) {
@@ -220,7 +246,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
                 const float len = (float)(TM >> level), l2 = log2f(a.rhos[r]);
                 const float mid = (float)seg * len + 0.5f * (len - 1.0f), ha = 0.5f * len * 0.9238795325f, hb = 0.5f * len * 0.3826834324f;
                 const float pa = exp2f(l2 * (mid + ha)), pb = exp2f(l2 * (mid + hb)), pc = exp2f(l2 * (mid - hb)), pd = exp2f(l2 * (mid - ha));
-                const float sc = STATE_F16_UNSCALE / unit * inverse(fw);
+                const float sc = 4.0f * STATE_F16_UNSCALE * ov * inverse(fw);
                 const float r0 = 0.25f * (pa + pb + pc + pd) * sc, r1 = 0.5f * (0.9238795325f * (pa - pd) + 0.3826834324f * (pb - pc)) * sc;
 #pragma unroll 1
                 for (int q = 0; q < 4; ++q) {
@@ -339,10 +365,10 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
                 if (c == 0) {      // the block's factors: red_e of all gate warps, red_b, red_x and red_p of the step warps
                     if (!(alive = warp_wait(&bars->kv_full[1], 1u, abort_flag, 3, lim) && warp_wait(&bars->pds_full, (uint32_t)(i & 1), abort_flag, 8, lim))) break;
                     // what the moments are at most: 128 steps, basis of at most 1.85, four coefficients into each of four nodes, a
-                    // derivative below 1.1; dS, P, dO (below 2) and q (log2(e) / 8) at their largest
+                    // derivative below 1.1; dS, P, dO (below 2^14) and q (log2(e) / 8) at their largest
                     constexpr float SUM = 128.0f * 1.85f * 16.0f * 1.1f;
                     const float f = ds_scale(bars), qm = 0.125f * 1.4426950409f * __uint_as_float(bars->qmax);
-                    const float top = SUM * f * max8(bars->red_e) * (qm * max8(bars->red_b) + 2.0f * max8(bars->red_p));
+                    const float top = SUM * f * max8(bars->red_e) * (qm * max8(bars->red_b) + 16384.0f * max8(bars->red_p));
                     const float fits = f * scale_to_f16(top, 50, 30);
                     // The unit stays while the blocks fit (64 times smaller than the first one needs: rarely more than one unit a segment);
                     // a smaller one, or a new segment, and what has been summed leaves tensor memory (blk_done has been waited for).
@@ -496,15 +522,18 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
             if (!(alive = warp_wait(&bars->s_read, (uint32_t)(i & 1), abort_flag, 10, lim))) break;
             tc_fence_after_sync();
             const float fs = ds_scale(bars), cs = LN2 * fs;
-            // the scores have been read by both halves: P^T takes their first 64 columns, dS^T the other 64
+            // the scores have been read by both halves: P^T takes their first 64 columns, dS^T the other 64, both over the smallest row
+            // factor (they are summed over the steps); dS^T for dQ keeps the rows' own
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 const int tb = half * 64 + k * 16;
                 float dp[16];
-                uint32_t d2[8];
+                uint32_t g2[8], d2[8];
                 tmem_ld_32x32b_x16(t_lane + T_DP + tb, dp);
+                *reinterpret_cast<uint4*>(g2) = *reinterpret_cast<const uint4*>(gf_sh + tb);
+                *reinterpret_cast<uint4*>(g2 + 4) = *reinterpret_cast<const uint4*>(gf_sh + tb + 8);
 #pragma unroll
-                for (int e = 0; e < 8; ++e) d2[e] = p2[k * 8 + e];
+                for (int e = 0; e < 8; ++e) d2[e] = mul_f16x2(p2[k * 8 + e], g2[e]);
                 tmem_st_x8(t_lane + T_S + half * 32 + k * 8, d2);
                 tmem_wait_ld();
 #pragma unroll
@@ -513,10 +542,12 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
                     d2[e / 2] = mul_f16x2(p2[k * 8 + e / 2], pack_f16x2_sat((dp[e] - dl.x) * cs, (dp[e + 1] - dl.y) * cs));
                     d2[e / 2 + 1] = mul_f16x2(p2[k * 8 + e / 2 + 1], pack_f16x2_sat((dp[e + 2] - dl.z) * cs, (dp[e + 3] - dl.w) * cs));
                 }
-                tmem_st_x8(t_lane + T_S + 64 + half * 32 + k * 8, d2);
                 unsigned char* ds = sm + M::DS + half * ATOM + r * 128;
                 st_shared_v4(ds + (((2 * k) ^ x7) << 4), d2[0], d2[1], d2[2], d2[3]);
                 st_shared_v4(ds + (((2 * k + 1) ^ x7) << 4), d2[4], d2[5], d2[6], d2[7]);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) d2[e] = mul_f16x2(d2[e], g2[e]);
+                tmem_st_x8(t_lane + T_S + 64 + half * 32 + k * 8, d2);
             }
             tmem_wait_st();
             tc_fence_before_sync();
@@ -553,7 +584,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
             if (!alive) break;
         }
         if (alive && t0 + r < a.T) {
-            const float sc = t0 + r < Lb ? 0.125f / (unit * LN2) : 0.f;
+            const int k = rx_sh[r];
+            const float sc = k == 255 ? NAN : t0 + r < Lb ? 0.125f / LN2 * exp2f(-kappa - (float)(emin + k)) : 0.f;
 #pragma unroll
             for (int cc = 0; cc < 2; ++cc)
 #pragma unroll

@@ -143,6 +143,37 @@ def test_values_and_gradients_of_any_size_in_a_peaked_softmax(mb, N, ev):
     assert rel_err(out["dW"], ref["dW"]) < TOL_GRAD
 
 
+@pytest.mark.parametrize("N", [64, 128])
+def test_gradient_rows_of_very_different_size(mb, N):
+    """A row of dO smaller by a power of two gives the row of dQ smaller by it, whatever stands beside it in the tile."""
+    c, V = case(41, 300, 300, N, unlisted=0.0)
+    plain = attend(mb, c, V, "tc_bf16")
+    f = 2.0 ** -torch.randint(0, 60, c["dO"].shape[:3], generator=torch.Generator().manual_seed(4)).float().cuda()[..., None]
+    c["dO"] = c["dO"] * f
+    c["Q"] = c["Q"].float()                # dQ in fp32
+    out, ref = attend(mb, c, V, "tc_bf16"), attend(mb, c, V, "fp32")
+    compare(out, ref)
+    a, b = (out["dQ"] / f).double().flatten(0, -2), plain["dQ"].double().flatten(0, -2)
+    assert float(((a - b).norm(dim=1) / b.norm(dim=1)).max()) < 2.0 ** -7      # `plain` is rounded to bf16
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_gradients_that_are_not_finite_say_so(mb, bad):
+    c, V = case(43, 300, 300, 64, H=4, unlisted=0.0)
+    c["dO"][1, 2, 150, 7] = bad
+    out = attend(mb, c, V, "tc_bf16")
+    finite = {k: torch.isfinite(v) for k, v in out.items()}
+    rows = finite["dQ"].all(-1)
+    assert not bool(rows[1, 2, 150]) and int((~rows).sum()) == 1
+    listed = (c["unique"][1] >= 0)
+    for k in ("dEk", "dEv"):
+        heads = finite[k].view(*finite[k].shape[:2], 4, 64)
+        assert not bool(heads[1, listed, 2].all(-1).any())
+        heads[1, :, 2] = True
+        assert bool(heads.all())
+    assert not bool(finite["dW"].view(64, 4, 64)[:, 2].all()) and bool(finite["dW"].view(64, 4, 64)[:, [0, 1, 3]].all())
+
+
 @pytest.mark.parametrize("silu,dtype", [(False, torch.bfloat16), (True, torch.float32)])
 def test_linear_gate_and_fp32_inputs(mb, silu, dtype):
     c, V = case(5, 257, 333, 64, dtype=dtype)
