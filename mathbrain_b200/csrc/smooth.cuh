@@ -8,14 +8,16 @@
 // tensor-core products; one gate evaluation serves 32 steps.  An occurrence inside the tile starts a new item with the
 // state (state + 1) rho^-(step), extended backwards to the tile start and valid for the steps after it.
 //
-// Error: the remainder of the cubic interpolant is f''''(x) d^4 / 192 with d the change of the pre-activation over half
-// a tile.  k_levels takes d per tile (root mean square over the gate's columns of M . lambda . W * 64) and the decay over
-// half a tile, and picks the number of segments the tile is cut into (1, 2, 4 or 8, each with nodes of its own);
-// what eight segments do not resolve goes to the kernels that evaluate every step (level LEVEL_EXACT).  With
-// half-lives of 1024..4096, states to 600 and W_pe ~ N(0, 0.02^2) the outputs differ from the exact sum by 1e-6 and
-// dW_pe by 1e-4 (norm-wise), against about 1e-3 from the 16-bit operands.
+// Error: with d the change of a column's pre-activation over half a segment, the cubic interpolant of SiLU is off by at most
+// 1.8e-3 d^4 / (1 + 0.033 d^3) (root mean square over the segment; an upper fit of the measured error for d in 0.1 .. 12), and only
+// where the column passes through the bend of SiLU, |x| < d + 3.5.  k_levels evaluates this for every item and head with the actual
+// pre-activations, and picks the number of segments the tile is cut into (1, 2, 4 or 8, each with nodes of its own) so that the
+// interpolation moves no item's gate by more than TOL_GATE of its norm over a head's columns; what eight segments do not resolve goes to
+// the kernels that evaluate every step (level LEVEL_EXACT).  Against 64 bits the outputs are then closer than the every-step kernels':
+// 5.2e-4 (2-norm) against 6.2e-4 for the 46M training chunks, W_pe ~ N(0, 0.02^2), states to 600.
 #pragma once
 #include "flash.cuh"
+#include <cuda_fp16.h>
 
 namespace mbema {
 namespace smooth {
@@ -30,10 +32,19 @@ static constexpr int WPIECE = 64 * 128;     // W' rows (node, 16 columns) x 64 c
 static constexpr int LEVELS = 4;            // level L cuts the tile into 2^L segments
 static constexpr int LEVEL_EXACT = LEVELS;
 static constexpr int SEG_IMAGES = (1 << LEVELS) - 1;   // W' images: segment s of level L at index 2^L - 1 + s
-// Half a segment's decay exponent and pre-activation change that a cubic still resolves: remainders below
-// 0.16^4 / 192 = 3.4e-6 (of the state sum) and, at 2.5, below 16-bit rounding of the gradients (measured dW_pe: 5e-4).
-// The backward's two-term node powers (smooth_bwd.cu) want the decay smaller: 0.045^2 / 4 = 5e-4.
-static constexpr float MAX_DECAY = 0.16f, MAX_SWING = 2.5f, MAX_DECAY_BWD = 0.045f;
+// Half a segment's decay exponent that a cubic still resolves: remainder below 0.16^4 / 192 = 3.4e-6 of the state sum.  The
+// backward's two-term node powers (smooth_bwd.cu) want it smaller: 0.045^2 / 4 = 5e-4.
+static constexpr float MAX_DECAY = 0.16f, MAX_DECAY_BWD = 0.045f;
+// Interpolation error of an item's gate over a head's columns, relative to their norm: half the unit roundoff of the fp16 that gates
+// are packed to (2^-11).  In the backward the same for SiLU' with the full unit.
+static constexpr float TOL_GATE = 1.0f / 4096.0f, TOL_SLOPE = 1.0f / 2048.0f;
+// Items whose pre-activations cannot change by more than this over half a tile meet TOL_GATE in every case (1.8e-3 d^4 against
+// a gate that itself moves by d / 3) and are not looked at.
+static constexpr float SMALL_SWING = 0.35f;
+// The coefficients are sums of up to four gates in fp16: items of larger ones (norm over a head's columns at mid-tile; up to
+// 3.6 times as much at the start of the fastest decays that eight segments resolve) go to the every-step kernels.
+static constexpr float MAX_GATE = 4096.0f;
+static constexpr float STATE_WEIGHT = 64.0f * 0.5f * MAX_GATE / SMALL_SWING;      // |state| that can reach half of it counts like a change of SMALL_SWING
 
 // Slots with the largest states, per tile.  They stand at the end of the item list, in blocks of their own: the forward walks
 // all blocks, the backward leaves these slots to the every-step kernel.  Their pre-activations move most inside a tile
@@ -46,7 +57,7 @@ struct Items {
     uint4* mask;            // [B * nT][IB][128] bit i of row t: item i of the block is valid at step t
     int2* meta;             // [B * nT][IB * 128] {slot, first valid step | last << 8}
     int* src;               // [B * nT][IB * 128] where the state comes from: slot k (snapshot) or -1 - step (occurrence); INT_MAX: padding
-    float* q;               // [B * nT][IB * 128] |lambda . state|^2
+    float* q;               // [B * nT][IB * 128] |lambda . state|^2 (or |state|^2 / STATE_WEIGHT^2 where that is larger)
     int4* count;            // [B * nT] {items and blocks before the hot ones, items and blocks in all}
     int* hot;               // [B * nT][HOT + 1] number of hot slots, the slots
     int IB;                 // blocks reserved per tile
@@ -54,7 +65,8 @@ struct Items {
 
 // Per-call workspace (after the status block).
 struct Ws {
-    float* gram;            // [N, N] W_pe W_pe^T / D
+    __half* probe;          // [3][D][N] W_pe scaled to pre-activations at mid-tile, and to their change over half a tile at the start and the end
+    float* wnorm;           // [D] |column of W_pe|^2
     unsigned char* w_img;   // [SEG_IMAGES][H][NCH][N / 64][WPIECE] node-scaled W_pe, fp16, swizzled operand pieces
     int* level;             // [B * nT] of the forward
     int* level_bwd;         // [B * nT] of the backward
@@ -84,7 +96,7 @@ inline Items carve_items(void* p0, int64_t B, int64_t T, int64_t N, int64_t K) {
 
 inline size_t ws_bytes(int64_t B, int64_t H, int64_t T, int64_t N, bool backward) {
     const size_t tiles = (size_t)B * ((T + TM - 1) / TM), NK = (size_t)N / 64;
-    return align_up((size_t)N * N * 4, 1024) + SEG_IMAGES * (size_t)H * NCH * NK * WPIECE + 2 * align_up(tiles * 4, 1024) +
+    return align_up((size_t)H * HD * (3 * N * 2 + 4), 1024) + SEG_IMAGES * (size_t)H * NCH * NK * WPIECE + 2 * align_up(tiles * 4, 1024) +
            (backward && NK == 2 ? tiles * H * NCH * ATOM : 0) + 1024;
 }
 
@@ -92,7 +104,8 @@ inline Ws carve(void* p0, int64_t B, int64_t H, int64_t T, int64_t N) {
     const size_t tiles = (size_t)B * ((T + TM - 1) / TM), NK = (size_t)N / 64;
     unsigned char* p = reinterpret_cast<unsigned char*>(align_up(reinterpret_cast<size_t>(p0), 1024));
     Ws w;
-    w.gram = reinterpret_cast<float*>(p); p += align_up((size_t)N * N * 4, 1024);
+    w.probe = reinterpret_cast<__half*>(p);
+    w.wnorm = reinterpret_cast<float*>(p + (size_t)H * HD * 3 * N * 2); p += align_up((size_t)H * HD * (3 * N * 2 + 4), 1024);
     w.w_img = p; p += SEG_IMAGES * (size_t)H * NCH * NK * WPIECE;
     w.level = reinterpret_cast<int*>(p); p += align_up(tiles * 4, 1024);
     w.level_bwd = reinterpret_cast<int*>(p); p += align_up(tiles * 4, 1024);

@@ -1,4 +1,4 @@
-// What the smooth attention kernels read: node-scaled W_pe images, the Gram matrix of W_pe, and per (sample, tile) the
+// What the smooth attention kernels read: node-scaled W_pe images, the segments a tile is cut into, and per (sample, tile) the
 // items (slots, and occurrences inside the tile) with their states as ready-made operand tiles.
 #include "smooth.cuh"
 #include "sm100_ptx.cuh"
@@ -14,19 +14,35 @@ __device__ __forceinline__ int sw_chunk(int r, int c8) { return r * 128 + ((c8 ^
 // ---------------------------------------------------------------------------------------------------------------
 // blocks [0, SEG_IMAGES * H * NCH): the W' image of (segment, head, column chunk): row i * 16 + dd holds
 // W[n, head * 64 + chunk * 16 + dd] rho_n^(node i of the segment), fp16, 64 x (the states carry 1/64) and, for SiLU,
-// 1/2 x (SiLU(x) = h + h tanh h, h = x / 2).  The remaining N N / 8 blocks: a warp per entry of the Gram matrix (a warp for
-// eight of them, one after the other: 11 us; one each: 6.6 us).
+// 1/2 x (SiLU(x) = h + h tanh h, h = x / 2).  The remaining D * N / 2048 blocks, a thread per column and eight channels: the probe
+// images (rows of N fp16, 64 x as well) that k_levels reads, and the columns' squared norms.
 // ---------------------------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) k_weights(FlashArgs a, Ws w) {
     const int N = a.N, D = a.H * HD, NK = N >> 6, tid = threadIdx.x;
     const int n_img = SEG_IMAGES * a.H * NCH;
     if ((int)blockIdx.x >= n_img) {
-        const int pair = ((int)blockIdx.x - n_img) * 8 + (tid >> 5), n = pair / N, m = pair % N, lane = tid & 31;
-        float s = 0.f;
-#pragma unroll 4
-        for (int d = lane; d < D; d += 32) s = fmaf(a.W[(size_t)n * D + d], a.W[(size_t)m * D + d], s);
-        s = warp_sum(s);
-        if (lane == 0) w.gram[n * N + m] = s / (float)D;
+        __shared__ float part[256];
+        const int cols = 2048 / N, dd = tid % cols, c8 = tid / cols, d = ((int)blockIdx.x - n_img) * cols + dd;      // D is a multiple of 64
+        float f[3][8], sq = 0.f;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const int n = c8 * 8 + e;
+            const float l2 = log2f(a.rhos[n]), lam = fabsf(l2) * 0.6931471806f, v = a.W[(size_t)n * D + d];
+            sq = fmaf(v, v, sq);
+            f[0][e] = v * STATE_F16_UNSCALE * exp2f(63.5f * l2);
+            f[1][e] = v * STATE_F16_UNSCALE * 64.0f * lam;
+            f[2][e] = f[1][e] * exp2f(127.0f * l2);
+        }
+#pragma unroll
+        for (int p = 0; p < 3; ++p)
+            *reinterpret_cast<uint4*>(w.probe + ((size_t)p * D + d) * N + c8 * 8) =
+                make_uint4(pack_f16x2(f[p][0], f[p][1]), pack_f16x2(f[p][2], f[p][3]), pack_f16x2(f[p][4], f[p][5]), pack_f16x2(f[p][6], f[p][7]));
+        part[tid] = sq;
+        __syncthreads();
+        if (c8 == 0) {
+            for (int i = 1; i < N / 8; ++i) sq += part[i * cols + dd];
+            w.wnorm[d] = sq;
+        }
         return;
     }
     const int c = blockIdx.x % NCH, h = (blockIdx.x / NCH) % a.H, img = blockIdx.x / (NCH * a.H);
@@ -206,7 +222,7 @@ __global__ void __launch_bounds__(IL_THREADS) k_items_list(FlashArgs a, Items it
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// one CTA per (block of items, tile, sample): operand tile, validity masks, |lambda . state|^2
+// one CTA per (block of items, tile, sample): operand tile, validity masks, |lambda . state|^2 (or the share of |state|^2)
 // ---------------------------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) k_items_fill(FlashArgs a, Items it) {
     __shared__ float rho_sh[128], lam_sh[128];
@@ -243,15 +259,20 @@ __global__ void __launch_bounds__(256) k_items_fill(FlashArgs a, Items it) {
         }
         *reinterpret_cast<uint4*>(img + (c8 >> 3) * ATOM + sw_chunk(r, c8 & 7)) = v;
         const uint32_t u[4] = {v.x, v.y, v.z, v.w};
-        float q = 0.f;
+        float q = 0.f, m2 = 0.f;
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const float2 f = unpack_f16x2(u[e]);
+            m2 = fmaf(f.x, f.x, fmaf(f.y, f.y, m2));
             const float x = f.x * lam_sh[c8 * 8 + 2 * e], y = f.y * lam_sh[c8 * 8 + 2 * e + 1];
             q = fmaf(x, x, fmaf(y, y, q));
         }
-        for (int o = CH / 2; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
-        if (c8 == 0) it.q[i0 + r] = q;
+        for (int o = CH / 2; o > 0; o >>= 1) {
+            q += __shfl_xor_sync(0xffffffffu, q, o);
+            m2 += __shfl_xor_sync(0xffffffffu, m2, o);
+        }
+        constexpr float WT = (STATE_F16_UNSCALE / STATE_WEIGHT) * (STATE_F16_UNSCALE / STATE_WEIGHT);
+        if (c8 == 0) it.q[i0 + r] = m2 * WT > q ? m2 * WT : q;        // (NaN stays)
     }
     const int row = tid & (TM - 1), half = tid >> 7;
     unsigned m0 = 0u, m1 = 0u;
@@ -265,102 +286,203 @@ __global__ void __launch_bounds__(256) k_items_fill(FlashArgs a, Items it) {
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// one CTA per (tile, sample): the levels.  v' G v <= |v|^2 times the largest absolute row sum of G (its largest eigenvalue is
-// no larger); items whose bound could matter are looked at closely, the others are not.  (The trace bounds it too, but
-// twenty times looser: with it a thousand items a tile were looked at, 84 us for 224 tiles.)
+// one CTA per (tile, sample): the levels (see smooth.cuh).  Items whose change over half a tile is below SMALL_SWING by Cauchy-Schwarz are
+// passed over.  The others (some eighty of the 46M training chunks' 2500) go through warp-level products with every column, for the
+// pre-activation at mid-tile and its change over half a tile at the tile's start and end: too few items and columns for a tensor-memory
+// pipeline to pay.  A warp keeps half a head's columns and walks the items, so that the images are read once.  Items that one segment does not
+// resolve, rare ones, go through another pass for two, and so on.  Bound by the issue of some 25
+// instructions a value: 62 us for 224 tiles of N = 64 and 8 heads, 35 us for 64; a root mean square over all columns, which one large column
+// escapes, took 31 and 17.
 // ---------------------------------------------------------------------------------------------------------------
-static constexpr int MAX_CHECKED = 1024;
-static constexpr int LV_THREADS = 1024, LV_ITEMS = 4;      // a warp looks at four items at once: one read of the Gram matrix for all
+static constexpr int LV_THREADS = 512, LV_WINDOW = 4096, LV_HEADS = LV_THREADS / 64;      // heads at a time: half a head a warp
 
+__device__ __forceinline__ void mma_16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// a lane's share of eight staged rows or columns: contiguous channels, since the contraction may take them in any order
+template <int NK> struct Frag {
+    uint32_t v[8 * NK];
+    __device__ __forceinline__ void load(const __half* p) {
+#pragma unroll
+        for (int i = 0; i < 2 * NK; ++i) *reinterpret_cast<uint4*>(v + 4 * i) = *(reinterpret_cast<const uint4*>(p) + i);
+    }
+};
+template <int NK>
+__device__ __forceinline__ void product(float (&c)[4], const Frag<NK>& lo, const Frag<NK>& hi, const Frag<NK>& col) {
+    c[0] = c[1] = c[2] = c[3] = 0.f;
+#pragma unroll
+    for (int k = 0; k < 4 * NK; ++k) {
+        const uint32_t a[4] = {lo.v[2 * k], hi.v[2 * k], lo.v[2 * k + 1], hi.v[2 * k + 1]};
+        mma_16816(c, a, col.v[2 * k], col.v[2 * k + 1]);
+    }
+}
+// interpolation error of SiLU, root mean square over a segment, for a change of d over half of it
+__device__ __forceinline__ float cubic_error(float d) {
+    const float d2 = d * d;
+    return __fdividef(1.8e-3f * d2 * d2, fmaf(0.033f * d, d2, 1.0f));
+}
+__device__ __forceinline__ float quad_sum(float v) {
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    return v + __shfl_xor_sync(0xffffffffu, v, 2);
+}
+
+// over a head's columns: squared interpolation error, gate, a quarter for every column with SiLU' >= 1/2
+struct Sums { float err, gate, slope; };
+template <bool SILU>
+__device__ __forceinline__ void add_column(Sums& s, float x, float d, float shrink) {
+    const float gate = SILU ? x * fmaf(0.5f, tanh_approx(0.5f * x), 0.5f) : fabsf(x);
+    const float er = SILU && fabsf(x) <= d + 3.5f ? cubic_error(d * shrink) : 0.f;
+    s.err = fmaf(er, er, s.err);
+    s.gate = fmaf(gate, gate, s.gate);
+    s.slope += !SILU || x >= 0.f ? 0.25f : 0.f;
+}
+
+template <bool SILU, int NK>
 __global__ void __launch_bounds__(LV_THREADS) k_levels(FlashArgs a, Items it, Ws w) {
-    __shared__ int chk[MAX_CHECKED], n_chk;
-    __shared__ unsigned swing_sh[2], decay_sh;          // [0] items before the hot ones, [1] hot items
-    __shared__ unsigned row_sh;
-    __shared__ float lam_sh[128];
-    const int bt = blockIdx.y * a.nT + blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int N = a.N, NK = N >> 6;
+    constexpr int N = NK * 64, LD = N + 8, SH = 16 * NK;          // halves a staged row, a lane's share of it
+    constexpr int CHUNK = 64, MT = CHUNK / 16;                    // items at a time
+    __shared__ __align__(16) __half rows[CHUNK * LD];
+    __shared__ Sums sums[2 * LV_HEADS][CHUNK];
+    __shared__ unsigned short chk[LV_WINDOW];             // items to look at, from the start of the window
+    __shared__ unsigned char open[2][CHUNK];              // rows that the level before did not resolve
+    __shared__ int n_chk, n_open[2];
+    __shared__ unsigned fail[2][CHUNK / 32], decay_sh, wmax_sh;      // rows whose gate, slope is not resolved at this level
+    __shared__ int need[2];                  // levels of the forward (all items) and of the backward (cold ones)
+    const int bt = blockIdx.y * a.nT + blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, jq = lane & 3;
+    const int D = a.H * HD;
     const int4 cnt = it.count[bt];
     if (cnt.w == 0) {
         if (tid == 0) w.level[bt] = w.level_bwd[bt] = 0;
         return;
     }
-    if (tid == 0) { n_chk = 0; row_sh = 0u; swing_sh[0] = swing_sh[1] = decay_sh = 0u; }
+    if (tid == 0) decay_sh = wmax_sh = 0u;
     __syncthreads();
     if (tid < N) {
         const float lam = fabsf(logf(a.rhos[tid]));               // rho = 0: infinite, every step
-        lam_sh[tid] = lam;
         atomicMax(&decay_sh, __float_as_uint(lam == lam ? lam : INFINITY));
     }
-    for (int n = warp; n < N; n += LV_THREADS / 32) {
-        float t = 0.f;
-        for (int m = lane; m < N; m += 32) t += fabsf(w.gram[n * N + m]);
-        t = warp_sum(t);
-        if (lane == 0) atomicMax(&row_sh, __float_as_uint(t));
+    float m = 0.f;
+    for (int d = tid; d < D; d += LV_THREADS) { const float v = w.wnorm[d]; m = v <= m ? m : (v == v ? v : INFINITY); }
+    m = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m)));
+    if (lane == 0) atomicMax(&wmax_sh, __float_as_uint(m));
+    __syncthreads();
+    const float decay = 64.0f * __uint_as_float(decay_sh), wmax = __uint_as_float(wmax_sh);
+    if (tid == 0) {
+        auto resolves = [&](float max_decay) {
+            int level = 0;
+            while (level < LEVEL_EXACT && !(decay <= max_decay * (float)(1 << level))) ++level;
+            return cnt.x < 0 ? LEVEL_EXACT : level;          // a token listed twice: every step in any case
+        };
+        need[0] = resolves(MAX_DECAY);
+        need[1] = resolves(MAX_DECAY_BWD);
     }
-    __syncthreads();
-    const float row_sum = __uint_as_float(row_sh);
-    const float look = (MAX_SWING / 64.0f) * (MAX_SWING / 64.0f) / fmaxf(row_sum, 1e-30f);
+    const float look = (SMALL_SWING / 64.0f) * (SMALL_SWING / 64.0f) / fmaxf(wmax, 1e-30f);
     const float* q = it.q + (size_t)bt * it.IB * IBLK;
-    for (int i = tid; i < cnt.w * IBLK; i += LV_THREADS)
-        if (!(q[i] <= look)) {
-            const int at = atomicAdd(&n_chk, 1);
-            if (at < MAX_CHECKED) chk[at] = i;
-            else atomicMax(&swing_sh[i >= cnt.y * IBLK], __float_as_uint(q[i] * row_sum));       // list full: the bound itself
-        }
-    __syncthreads();
     const unsigned char* img = it.a_img + (size_t)bt * it.IB * NK * ATOM;
-    const int n_look = min(n_chk, MAX_CHECKED);
-    for (int j0 = warp * LV_ITEMS; j0 < n_look; j0 += LV_THREADS / 32 * LV_ITEMS) {      // a lane per channel
-        float vl[LV_ITEMS][4], y[LV_ITEMS][4];
-#pragma unroll
-        for (int g = 0; g < LV_ITEMS; ++g) {
-            const int item = chk[min(j0 + g, n_look - 1)], r = item & (IBLK - 1);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int n = lane + 32 * e;
-                vl[g][e] = y[g][e] = 0.f;
-                if (n < N)
-                    vl[g][e] = __half2float(*reinterpret_cast<const __half*>(img + (size_t)(item / IBLK) * NK * ATOM + (n >> 6) * ATOM +
-                                                                             sw_chunk(r, (n >> 3) & 7) + (n & 7) * 2)) * (STATE_F16_UNSCALE * lam_sh[n]);
+    const int total = cnt.w * IBLK, n_cold = cnt.y * IBLK;
+    for (int i0 = 0; i0 < total; i0 += LV_WINDOW) {
+        __syncthreads();
+        if (tid == 0) n_chk = 0;
+        __syncthreads();
+        for (int i = i0 + tid; i < min(i0 + LV_WINDOW, total); i += LV_THREADS)
+            if (!(q[i] < look)) chk[atomicAdd(&n_chk, 1)] = (unsigned short)(i - i0);
+        __syncthreads();
+        const int n_look = n_chk;
+        for (int j0 = 0; j0 < n_look; j0 += CHUNK) {
+            const int n = min(CHUNK, n_look - j0);
+            if (need[0] >= LEVEL_EXACT && need[1] >= LEVEL_EXACT) break;          // uniform: written before the last barrier only
+            for (int i = tid; i < CHUNK * (N / 8); i += LV_THREADS) {
+                const int j = i / (N / 8), c8 = i % (N / 8), item = i0 + chk[j0 + min(j, n - 1)];
+                *reinterpret_cast<uint4*>(rows + j * LD + c8 * 8) =
+                    *reinterpret_cast<const uint4*>(img + ((size_t)(item / IBLK) * NK + (c8 >> 3)) * ATOM + sw_chunk(item & (IBLK - 1), c8 & 7));
             }
-        }
+            if (tid < CHUNK) open[0][tid] = (unsigned char)min(tid, n - 1);
+            if (tid == 0) n_open[0] = n;
+            // of row `tid`: gate, slope (cold items only) not resolved yet at the level; a level that the tile needs anyway is not looked at
+            const bool cold = tid < n && i0 + chk[j0 + tid] < n_cold;
+            bool open_g = true, open_s = cold;
+            const int first = min(need[0], need[1]);
+            for (int level = first; level < LEVEL_EXACT; ++level) {
+                const unsigned char* list = open[(level - first) & 1];
+                int* m_open = &n_open[(level - first) & 1];
+                if (tid < CHUNK / 32) fail[0][tid] = fail[1][tid] = 0u;
+                if (tid == 0) n_open[(level - first + 1) & 1] = 0;
+                __syncthreads();
+                const int m_rows = *m_open, mts = (m_rows + 15) / 16;
+                if (m_rows == 0) break;
+                const float shrink = 1.0f / (float)(1 << level);
+                for (int h0 = 0; h0 < a.H; h0 += LV_HEADS) {
+                    const int heads = min(LV_HEADS, a.H - h0);
+                    if (warp < 2 * heads) {
+                        Sums acc[MT][2];
 #pragma unroll
-        for (int e2 = 0; e2 < 4; ++e2) {
-            if (32 * e2 >= N) break;
-#pragma unroll 4
-            for (int l = 0; l < 32; ++l) {
-                const float* g = w.gram + (size_t)(32 * e2 + l) * N;
-                float gr[4];
+                        for (int m = 0; m < MT; ++m) acc[m][0] = acc[m][1] = Sums{0.f, 0.f, 0.f};
+                        const __half* col = w.probe + ((size_t)h0 * HD + warp * 32 + g) * N + jq * SH;
+                        Frag<NK> B[3];
 #pragma unroll
-                for (int e = 0; e < 4; ++e) gr[e] = 32 * e < N ? __ldg(g + lane + 32 * e) : 0.f;
+                        for (int p = 0; p < 3; ++p) B[p].load(col + (size_t)p * D * N);
+#pragma unroll 1
+                        for (int nt = 0; nt < 4; ++nt) {
+                            // the next columns are on their way while these are worked on
+                            const __half* next = col + (size_t)min(nt + 1, 3) * 8 * N;
 #pragma unroll
-                for (int i = 0; i < LV_ITEMS; ++i) {
-                    const float vm = __shfl_sync(0xffffffffu, vl[i][e2], l);
+                            for (int p = 0; p < 3; ++p) asm volatile("prefetch.global.L1 [%0];" ::"l"(next + (size_t)p * D * N));
 #pragma unroll
-                    for (int e = 0; e < 4; ++e)
-                        if (32 * e < N) y[i][e] = fmaf(vm, gr[e], y[i][e]);
+                            for (int m = 0; m < MT; m += 2) {          // two at a time: their chains run side by side
+                                if (m >= mts) break;
+                                float c[2][3][4];
+#pragma unroll
+                                for (int k = 0; k < 2; ++k) {
+                                    Frag<NK> lo, hi;
+                                    lo.load(rows + list[min((m + k) * 16 + g, m_rows - 1)] * LD + jq * SH);
+                                    hi.load(rows + list[min((m + k) * 16 + 8 + g, m_rows - 1)] * LD + jq * SH);
+#pragma unroll
+                                    for (int p = 0; p < 3; ++p) product<NK>(c[k][p], lo, hi, B[p]);
+                                }
+#pragma unroll
+                                for (int e = 0; e < 4; ++e)
+#pragma unroll
+                                    for (int k = 0; k < 2; ++k)
+                                        add_column<SILU>(acc[m + k][e >> 1], c[k][0][e], fmaxf(fabsf(c[k][1][e]), fabsf(c[k][2][e])), shrink);
+                            }
+#pragma unroll
+                            for (int p = 0; p < 3; ++p) B[p].load(next + (size_t)p * D * N);
+                        }
+#pragma unroll
+                        for (int m = 0; m < MT; ++m)
+#pragma unroll
+                            for (int s = 0; s < 2; ++s) {
+                                const Sums t{quad_sum(acc[m][s].err), quad_sum(acc[m][s].gate), quad_sum(acc[m][s].slope)};
+                                if (jq == 0) sums[warp][m * 16 + 8 * s + g] = t;
+                            }
+                    }
+                    __syncthreads();
+                    for (int i = tid; i < m_rows * heads; i += LV_THREADS) {
+                        const int j = i % m_rows, h = i / m_rows, r = list[j];
+                        const Sums u = sums[2 * h][j], v = sums[2 * h + 1][j];
+                        const float es = u.err + v.err, gs = u.gate + v.gate;
+                        if (!(gs < MAX_GATE * MAX_GATE && es <= TOL_GATE * TOL_GATE * gs)) atomicOr(&fail[0][r >> 5], 1u << (r & 31));
+                        if (!(gs < MAX_GATE * MAX_GATE && es <= TOL_SLOPE * TOL_SLOPE * (u.slope + v.slope))) atomicOr(&fail[1][r >> 5], 1u << (r & 31));
+                    }
+                    __syncthreads();
                 }
+                if (tid < n) {
+                    open_g = open_g && ((fail[0][tid >> 5] >> (tid & 31)) & 1u);
+                    open_s = open_s && ((fail[1][tid >> 5] >> (tid & 31)) & 1u);
+                    if (open_g) atomicMax(&need[0], level + 1);
+                    if (cold && (open_g || open_s)) atomicMax(&need[1], level + 1);
+                    if (open_g || open_s) open[(level - first + 1) & 1][atomicAdd(&n_open[(level - first + 1) & 1], 1)] = (unsigned char)tid;
+                }
+                __syncthreads();
             }
-        }
-#pragma unroll
-        for (int i = 0; i < LV_ITEMS; ++i) {
-            const float v = warp_sum(vl[i][0] * y[i][0] + vl[i][1] * y[i][1] + vl[i][2] * y[i][2] + vl[i][3] * y[i][3]);
-            const int item = chk[min(j0 + i, n_look - 1)];
-            if (lane == 0) atomicMax(&swing_sh[item >= cnt.y * IBLK], __float_as_uint(v >= 0.f ? v : (v < 0.f ? 0.f : INFINITY)));
+            __syncthreads();
         }
     }
     __syncthreads();
     if (tid == 0) {
-        const float decay = 64.0f * __uint_as_float(decay_sh);
-        auto pick = [&](float max_decay, float q2) {
-            const float swing = 64.0f * sqrtf(q2);
-            int level = 0;
-            while (level < LEVEL_EXACT && !(decay <= max_decay * (float)(1 << level) && swing <= MAX_SWING * (float)(1 << level))) ++level;
-            return cnt.x < 0 ? LEVEL_EXACT : level;
-        };
-        const float cold = __uint_as_float(swing_sh[0]), hot = __uint_as_float(swing_sh[1]);
-        w.level[bt] = pick(MAX_DECAY, fmaxf(cold, hot));
-        w.level_bwd[bt] = pick(MAX_DECAY_BWD, cold);
+        w.level[bt] = need[0];
+        w.level_bwd[bt] = need[1];
     }
 }
 
@@ -372,8 +494,15 @@ int build_items(const FlashArgs& a, const Items& it, cudaStream_t st) {
 }
 
 int prepare(const FlashArgs& a, const Items& it, const Ws& w, cudaStream_t st) {
-    k_weights<<<SEG_IMAGES * a.H * NCH + a.N * a.N / 8, 256, 0, st>>>(a, w);
-    k_levels<<<dim3(a.nT, a.B), LV_THREADS, 0, st>>>(a, it, w);
+    k_weights<<<SEG_IMAGES * a.H * NCH + a.H * HD * a.N / 2048, 256, 0, st>>>(a, w);
+    const dim3 grid(a.nT, a.B);
+    if (a.silu) {
+        if (a.N == 64) k_levels<true, 1><<<grid, LV_THREADS, 0, st>>>(a, it, w);
+        else k_levels<true, 2><<<grid, LV_THREADS, 0, st>>>(a, it, w);
+    } else {
+        if (a.N == 64) k_levels<false, 1><<<grid, LV_THREADS, 0, st>>>(a, it, w);
+        else k_levels<false, 2><<<grid, LV_THREADS, 0, st>>>(a, it, w);
+    }
     return check_launch();
 }
 
