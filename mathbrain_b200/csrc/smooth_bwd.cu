@@ -44,8 +44,9 @@ struct Bars {
     unsigned spin_limit, pmax, qmax;
     // of the block worked on, per warp: largest P |dP - D| of an item (a bound on it), |dP - D|, P; largest |E / 4|
     alignas(16) float red_b[SM_WARPS], red_x[SM_WARPS], red_p[SM_WARPS], red_e[GATE_WARPS];
-    float fs[GATE_WARPS], fm[GATE_WARPS];      // its factors of dS and of the moments, a copy per gate warp
-    int dw_fresh;                              // its dW products start the sums anew
+    float fs, fm;                              // its factors of dS and of the moments
+    float fw, fw_old;                          // their product, the unit of the dW sums: it stays while the blocks fit; the one before
+    int dw_fresh;                              // the block's dW products start the sums anew
 };
 
 template <int NK> struct L {
@@ -134,6 +135,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
         bars->emin = INT_MAX;
         bars->bad = 0;
         bars->pmax = 0u;
+        bars->fw = 0.f;
         bars->qmax = 0u;
         fence_barrier_init();
     }
@@ -221,6 +223,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
             rx_sh[t] = bad ? 255 : k;
         }
     }
+    for (int i = tid; i < N * (HD / 4); i += THREADS)
+        *reinterpret_cast<float4*>(part + (i / (HD / 4)) * 128 + (i % (HD / 4)) * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
     asm volatile("fence.proxy.async;" ::: "memory");      // the operand tiles, in shared memory and (NK = 2) in the workspace
     tc_fence_before_sync();
     __syncthreads();
@@ -238,9 +242,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
         const uint32_t t_lane = tmem + ((uint32_t)((warp & 3) * 32) << 16);
         const int2* meta = it.meta + (size_t)bt * it.IB * IBLK + r;
         const float ov = 0.25f / unit * (bars->bad ? NAN : 1.0f);
-        float fw = 0.f;          // factor of dS times that of the moments, the unit of the dW sums
-        // the dW sums in tensor memory: lane n, chunks 2 wg and 2 wg + 1
-        auto flush = [&](int seg, bool first) {
+        // the dW sums in tensor memory, in the unit `fw`: lane n, chunks 2 wg and 2 wg + 1
+        auto flush = [&](int seg, float fw) {
             tc_fence_after_sync();
             if (r < N) {         // whole warps
                 const float len = (float)(TM >> level), l2 = log2f(a.rhos[r]);
@@ -260,14 +263,12 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
                     for (int dd = 0; dd < 8; dd += 4) {
                         const float4 v = make_float4(r0 * d0[dd] + r1 * d1[dd], r0 * d0[dd + 1] + r1 * d1[dd + 1], r0 * d0[dd + 2] + r1 * d1[dd + 2],
                                                      r0 * d0[dd + 3] + r1 * d1[dd + 3]);
-                        if (first) *reinterpret_cast<float4*>(o + dd) = v;
-                        else red_v4(o + dd, v.x, v.y, v.z, v.w);
+                        red_v4(o + dd, v.x, v.y, v.z, v.w);
                     }
                 }
             }
             tc_fence_before_sync();
         };
-        bool first = true;
         size_t eo = 0;          // this item's E columns of chunk 0
         ERow<EF32> ek, ev;
         if (n_it > 0) {
@@ -362,30 +363,16 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
                 fence_proxy_async_smem();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&bars->kg_full[st]);
-                if (c == 0) {      // the block's factors: red_e of all gate warps, red_b, red_x and red_p of the step warps
-                    if (!(alive = warp_wait(&bars->kv_full[1], 1u, abort_flag, 3, lim) && warp_wait(&bars->pds_full, (uint32_t)(i & 1), abort_flag, 8, lim))) break;
-                    // what the moments are at most: 128 steps, basis of at most 1.85, four coefficients into each of four nodes, a
-                    // derivative below 1.1; dS, P, dO (below 2^14) and q (log2(e) / 8) at their largest
-                    constexpr float SUM = 128.0f * 1.85f * 16.0f * 1.1f;
-                    const float f = ds_scale(bars), qm = 0.125f * 1.4426950409f * __uint_as_float(bars->qmax);
-                    const float top = SUM * f * max8(bars->red_e) * (qm * max8(bars->red_b) + 16384.0f * max8(bars->red_p));
-                    const float fits = f * scale_to_f16(top, 50, 30);
-                    // The unit stays while the blocks fit (64 times smaller than the first one needs: rarely more than one unit a segment);
-                    // a smaller one, or a new segment, and what has been summed leaves tensor memory (blk_done has been waited for).
-                    const bool fresh = blk == 0 || fw > fits;
-                    if (fresh) {
-                        if (i > 0) { flush((i - 1) / n_blk, first); first = false; }
-                        fw = fits * 0.015625f;
-                    }
-                    if (lane == 0) { bars->fs[warp] = f; bars->fm[warp] = fw * inverse(f); bars->dw_fresh = fresh; }
-                    __syncwarp();
+                if (c == 0) {      // the block's factors, from the step warps
+                    if (!(alive = warp_wait(&bars->pds_full, (uint32_t)(i & 1), abort_flag, 8, lim))) break;
+                    if (i > 0 && bars->dw_fresh) flush((i - 1) / n_blk, bars->fw_old);       // (blk_done has been waited for)
                 }
                 if (!(alive = warp_wait(&bars->dkv_full[st], (uint32_t)(use & 1), abort_flag, 6, lim))) break;
                 tc_fence_after_sync();
                 float* gk = a.dEk + eo + c * 16;
                 float* gv = a.dEv + eo + c * 16;
                 const bool live = blk * IBLK + r < n_items;
-                const float fs = bars->fs[warp], fm = bars->fm[warp], oe = ov * inverse(fs);
+                const float fs = bars->fs, fm = bars->fm, oe = ov * inverse(fs);
                 uint32_t m0[4], m1[4];
 #pragma unroll
                 for (int q = 0; q < 2; ++q) {      // four columns at a time
@@ -452,10 +439,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
             }
             eo = eo_next;
         }
-        if (n_it > 0 && alive && warp_wait(&bars->blk_done, (uint32_t)((n_it - 1) & 1), abort_flag, 8, lim)) flush((n_it - 1) / n_blk, first);
-        if (n_blk == 0)
-            for (int i = tid; i < N * (HD / 4); i += GATE_WARPS * 32)
-                *reinterpret_cast<float4*>(part + (i / (HD / 4)) * 128 + (i % (HD / 4)) * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (n_it > 0 && alive && warp_wait(&bars->blk_done, (uint32_t)((n_it - 1) & 1), abort_flag, 8, lim)) flush((n_it - 1) / n_blk, bars->fw);
     } else if (warp < GATE_WARPS + SM_WARPS) {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
         // ======================================================== softmax (item r, steps 64 half ..), then dQ (step r)
@@ -552,6 +536,25 @@ __global__ void __launch_bounds__(THREADS, 1) k_smooth_bwd(FlashArgs a, Items it
             tmem_wait_st();
             tc_fence_before_sync();
             fence_proxy_async_smem();
+            if (warp == GATE_WARPS) {      // the factors for the gate warps (red_e is theirs)
+                if (!(alive = warp_wait(&bars->kv_full[1], 1u, abort_flag, 3, lim))) break;
+                // what the moments are at most: 128 steps, basis of at most 1.85, four coefficients into each of four nodes, a
+                // derivative below 1.1; dS, P, dO (below 2^14) and q (log2(e) / 8) at their largest
+                constexpr float SUM = 128.0f * 1.85f * 16.0f * 1.1f;
+                const float qm = 0.125f * 1.4426950409f * __uint_as_float(bars->qmax);
+                const float top = SUM * fs * max8(bars->red_e) * (qm * max8(bars->red_b) + 16384.0f * max8(bars->red_p));
+                if (lane == 0) {
+                    // The unit of the dW sums stays while the blocks fit (64 times smaller than the first one needs: rarely more than one
+                    // a segment); with a smaller one, or a new segment, what has been summed leaves tensor memory.
+                    const float fits = fs * scale_to_f16(top, 50, 30), fw = bars->fw;
+                    const bool fresh = i % n_blk == 0 || fw > fits;
+                    bars->dw_fresh = fresh;
+                    bars->fw_old = fw;
+                    if (fresh) bars->fw = fits * 0.015625f;
+                    bars->fs = fs;
+                    bars->fm = bars->fw * inverse(fs);
+                }
+            }
             __syncwarp();
             if (lane == 0) mbar_arrive(&bars->pds_full);
             int rr = r;
