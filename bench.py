@@ -27,11 +27,21 @@ if ROOT not in sys.path:
 
 CFG = dict(B=56, T=512, D=512, H=8, N=64, L=6, V=50257, min_hl=1024.0, max_hl=4096.0, max_prefix=8192, min_fill=64)
 METRIC = "flash_ema_fwd_bwd_tokens_per_s"
-# DRAM traffic of the attention backward, bytes per slot-step (one listed slot of one sample at one time step):
-# dram__bytes_read.sum + dram__bytes_write.sum of one profiler capture of the B=16 profile case divided by that
-# launch's slot-steps.  Traffic grows in proportion to the slot-steps, so a full launch is this figure times its own.
-BWD_DRAM_BYTES_PER_SLOT_STEP = 22.3
+HOT = 16                     # slots of a 128-step tile that the backward takes at every step
 DECODE = dict(B=64, K0=3000, capacity=4608, steps=2048, warmup=16)
+
+
+def attention_flops(c, kb, mode):
+    """Tensor operations of one layer's attention, forward and backward, over slot lists of `kb` entries (tensor [B]): what the products
+    over smooth slot states take per slot-step and column, and the largest slots of every tile at every step in the backward.
+    Smooth states, a tile of 128 steps, a head of 64 columns, four coefficients a column: forward gate 2 * 256 N, scores and P.V 2 * 128 * 256 each;
+    backward gate twice, S, dP, dK, dV and dQ 2 * 128 * 256 each, dW_pe 2 * 128 N.  At every step (and in the fp32 mode): 2 N D in the forward, 4 N D in the backward."""
+    N, D = c["N"], c["D"]
+    every = float((kb * c["T"]).sum())
+    if mode == "fp32":
+        return 2.0 * N * D * every, 4.0 * N * D * every
+    hot = float((kb.clamp_max(HOT) * c["T"]).sum())
+    return (N / 16.0 + 16.0) * D * every, (10.0 * N / 64.0 + 40.0) * D * (every - hot) + 4.0 * N * D * hot
 
 
 def peaks():
@@ -1051,8 +1061,7 @@ def main():
         c = CFG
         pk = peaks()
         tokens = hp.tokens * world
-        flops_bwd = 4.0 * c["N"] * c["D"] * hp.slot_steps      # per launch (one layer), tensor flops only
-        flops_fwd = 2.0 * c["N"] * c["D"] * hp.slot_steps
+        flops_fwd, flops_bwd = attention_flops(c, hp.host["pad_mask"].sum(1).double(), args.mode)      # per layer
         avg_bwd = sum(bwd_ms) / max(1, len(bwd_ms)) / 1000.0
         avg_fwd = sum(fwd_ms) / max(1, len(fwd_ms)) / 1000.0
         ach = flops_bwd / avg_bwd / 1e12
@@ -1079,8 +1088,7 @@ def main():
                     "d2h_bytes_per_step": 8},
             "roofline": {"bound": "tensor", "kernel": "flash-EMA backward (one layer)", "achieved": ach,
                          "peak": pk["tflops"], "unit": "TFLOP/s", "frac": ach / pk["tflops"],
-                         "traffic": BWD_DRAM_BYTES_PER_SLOT_STEP * hp.slot_steps,
-                         "traffic_unit": "bytes/launch (profiler capture of the B=16 profile case, scaled by slot-steps)",
+                         "flops": "products over smooth slot states, the sixteen largest slots of a tile at every step",
                          "peak_source": pk["src"], "flops_per_launch": flops_bwd, "ms_per_launch": avg_bwd * 1000.0,
                          "forward": {"achieved": flops_fwd / avg_fwd / 1e12, "ms_per_launch": avg_fwd * 1000.0},
                          "scan_ms": sum(scan_ms) / max(1, len(scan_ms)), "gate_ms_per_step": sum(gate_ms) / args.steps},
